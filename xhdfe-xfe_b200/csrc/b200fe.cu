@@ -304,17 +304,61 @@ int build_sparse_block(b200fe_context* ctx) {
         st.pc_nshort = cnt[0];
         st.pc_nlong = cnt[1];
         st.pc_nlchunks = cnt[2];
-        B_CHECK(get_buf(ctx, "pc_short_meta", std::max<int64_t>(st.pc_nshort, 1), &st.pc_short_meta));
-        B_CHECK(get_buf(ctx, "pc_long_rows", std::max<int64_t>(st.pc_nlong, 1), &st.pc_long_rows));
-        B_CHECK(get_buf(ctx, "pc_long_c0", std::max<int64_t>(st.pc_nlong, 1), &st.pc_long_c0));
-        B_CHECK(get_buf(ctx, "pc_long_c1", std::max<int64_t>(st.pc_nlong, 1), &st.pc_long_c1));
+        B_CHECK(get_buf(ctx, "pc_short_row", std::max<int64_t>(st.pc_nshort, 1), &st.pc_short_rows));
+        B_CHECK(get_buf(ctx, "pc_long_meta", std::max<int64_t>(st.pc_nlong, 1), &st.pc_long_meta));
         B_CHECK(get_buf(ctx, "pc_lchunk_meta", std::max<int64_t>(st.pc_nlchunks, 1), &st.pc_lchunk_meta));
         pcg_lists_fill_kernel<<<grid_for(ctx, L.G, T256), T256, 0, s>>>(
-            st.sp_row_off, L.G, is_short, short_idx, long_idx, chunk_off, st.pc_short_meta,
-            st.pc_long_rows, st.pc_long_c0, st.pc_long_c1, st.pc_lchunk_meta, huge_idx, st.pc_huge_li);
+            st.sp_row_off, L.G, is_short, short_idx, long_idx, chunk_off, st.pc_short_rows, st.pc_long_meta,
+            st.pc_lchunk_meta, huge_idx, st.pc_huge_li);
         B_LAUNCHED();
     }
     st.sparse = true;
+    return B200FE_OK;
+}
+
+// Tiles of the short rows for a column pitch of 4 cq (PcgTiles): without a
+// coupled small dim one order serves every pitch.
+int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
+    Structure& st = ctx->st;
+    const cudaStream_t s = ctx->stream;
+    const bool coupled = st.coupled && st.nS == 1;
+    const int slot = !coupled || cq == 1 ? 0 : cq == 2 ? 1 : 2;
+    PcgTiles& t = st.pc_tiles[slot];
+    *out = &t;
+    if (t.built) return B200FE_OK;
+    const std::string sfx = std::to_string(slot);
+    const int sr = coupled ? 32 / cq : kPcgRowsPerWarp;
+    const int lists = coupled ? kPcgListsPerSm * ctx->num_sms : 0;
+    const int64_t npad = (st.pc_nshort + sr - 1) / sr * sr;
+    t.n = npad / kPcgRowsPerWarp;
+    const size_t t1 = static_cast<size_t>(t.n) + 1;
+    const int64_t cap = st.sp_nnz + 4 * t.n + 4;  // every tile padded to a multiple of four entries
+    int32_t *key, *row, *key_s, *row_s, *len, *off;
+    B_CHECK(get_buf(ctx, "pc_key", std::max<int64_t>(npad, 1), &key));
+    B_CHECK(get_buf(ctx, "pc_row", std::max<int64_t>(npad, 1), &row));
+    B_CHECK(get_buf(ctx, "pc_key_s", std::max<int64_t>(npad, 1), &key_s));
+    B_CHECK(get_buf(ctx, "pc_row_s", std::max<int64_t>(npad, 1), &row_s));
+    B_CHECK(get_buf(ctx, "pc_tile_len", t1, &len));
+    B_CHECK(get_buf(ctx, "pc_tile_off", t1, &off));
+    B_CHECK(get_buf(ctx, "pc_tile_meta" + sfx, t1, &t.meta));
+    B_CHECK(get_buf(ctx, "pc_tile_rows" + sfx, t1 * kPcgRowsPerWarp, &t.rows));
+    B_CHECK(get_buf(ctx, "pc_tile_col" + sfx, cap, &t.col));
+    B_CHECK(get_buf(ctx, "pc_tile_val64" + sfx, cap, &t.val64));
+    B_CHECK(get_buf(ctx, "pc_tile_val32" + sfx, cap, &t.val32));
+    if (npad > 0) {
+        pcg_tile_key_kernel<<<grid_for(ctx, npad, 256), 256, 0, s>>>(st.sp_row_off, st.pc_short_rows, st.pc_nshort,
+                                                                     npad, sr, lists, key, row);
+        B_LAUNCHED();
+        B_CHECK(cub_sort_pairs(ctx, key, key_s, row, row_s, npad, std::max(lists, 1) * (kShortNnz + 2)));
+        pcg_tile_len_kernel<<<grid_for(ctx, static_cast<int64_t>(t1), 256), 256, 0, s>>>(st.sp_row_off, row_s, t.n,
+                                                                                        len);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, len, off, static_cast<int64_t>(t1)));
+        pcg_tile_fill_kernel<<<grid_for(ctx, t.n * 32, 256), 256, 0, s>>>(
+            st.sp_row_off, st.sp_col, st.sp_val64, row_s, t.n, off, t.meta, t.rows, t.col, t.val64, t.val32);
+        B_LAUNCHED();
+    }
+    t.built = true;
     return B200FE_OK;
 }
 
@@ -1558,12 +1602,17 @@ double pcg_iter_bytes(const Structure& st, int CP, size_t tsize) {
     return b;
 }
 
+// Bytes of the rows of p that one application of the explicit block gathers.
+double pcg_gather_bytes(const Structure& st, int CP, size_t tsize) {
+    return (static_cast<double>(st.sp_nnz) + static_cast<double>(st.GR)) * CP * static_cast<double>(tsize);
+}
+
 // Inner PCG as one cooperative launch (pcg_kernels.cuh).  Returns
 // B200FE_UNAVAILABLE (nothing run) when the launch cannot be made, so the
 // caller falls back to the multi-kernel PCG.
 template <typename T, int CQ>
-int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, T* r, T* z, T* p,
-                   T* q, const std::vector<double>& thr_host, int max_iter, int* iters_out) {
+int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, T* r, T* p, T* q,
+                   const std::vector<double>& thr_host, int max_iter, int* iters_out) {
     const Structure& st = ctx->st;
     constexpr int CP = 4 * CQ;
     const cudaStream_t s = ctx->stream;
@@ -1571,13 +1620,24 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     const int SG = coupled ? st.SG : 0;
     const int SGP = coupled ? st.SGP : 0;
     if (SG > kPcgMaxSG) return B200FE_UNAVAILABLE;
-    const size_t smem = pcg_smem_bytes<T>(CP, SGP);
-    auto kern = pcg_persistent_kernel<T, CQ>;
-    B_TRY(raise_smem_limit(reinterpret_cast<const void*>(kern), static_cast<int>(smem)));
-    int per_sm = 0;
-    B_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPcgThreads, smem));
-    if (per_sm < 1) return B200FE_UNAVAILABLE;
-    const int nb = ctx->num_sms * std::min(per_sm, 2);
+    // two staging buffers of the coupling where they fit beside the rest
+    const int cbuf = pcg_smem_bytes<T>(CP, SG, SGP, 2) <= 200 * 1024 ? 2 : 1;
+    const size_t smem = pcg_smem_bytes<T>(CP, SG, SGP, cbuf);
+    constexpr int NT = pcg_threads<T>();
+    // small systems: one thread-block cluster, whose CTAs meet at the hardware
+    // barrier (kPcgClusterBytes); the others, and all where a cluster of that
+    // size cannot be launched: a cooperative launch of one CTA per SM
+    const bool cluster = pcg_gather_bytes(st, CP, sizeof(T)) <= kPcgClusterBytes;
+    // levels per lane of the coupling: none, or SG over the 32 / CQ lanes of a column quad
+    constexpr int KF = 2 * CQ, KS = CQ == 4 ? 5 : KF;
+    using Kernel = void (*)(PcgArgs<T>);
+    const Kernel kern_cluster = SG == 0             ? pcg_persistent_kernel<T, CQ, 0, true>
+                                : SG * CQ <= 32 * KS ? pcg_persistent_kernel<T, CQ, KS, true>
+                                                     : pcg_persistent_kernel<T, CQ, KF, true>;
+    const Kernel kern_grid = SG == 0             ? pcg_persistent_kernel<T, CQ, 0, false>
+                             : SG * CQ <= 32 * KS ? pcg_persistent_kernel<T, CQ, KS, false>
+                                                  : pcg_persistent_kernel<T, CQ, KF, false>;
+    const int nb_max = std::max(kPcgMinCtas, ctx->num_sms);
     PcgArgs<T> a{};
     a.CP = CP;
     a.Gf = st.L[0].G;
@@ -1587,13 +1647,20 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     a.col = st.sp_col;
     a.val = pick_prec<T>(st.sp_val32, st.sp_val64);
     a.nshort = st.pc_nshort;
-    a.short_meta = st.pc_short_meta;
+    a.short_rows = st.pc_short_rows;
+    const PcgTiles* tiles;
+    B_CHECK(build_pcg_tiles(ctx, CQ, &tiles));
+    a.ntiles = tiles->n;
+    a.tile_meta = tiles->meta;
+    a.tile_rows = tiles->rows;
+    a.tile_col = tiles->col;
+    a.tile_val = pick_prec<T>(tiles->val32, tiles->val64);
+    a.lists = kPcgListsPerSm * ctx->num_sms;
+    a.cbuf = cbuf;
     a.nlchunks = st.pc_nlchunks;
     a.lchunk_meta = st.pc_lchunk_meta;
     a.nlong = st.pc_nlong;
-    a.long_rows = st.pc_long_rows;
-    a.long_c0 = st.pc_long_c0;
-    a.long_c1 = st.pc_long_c1;
+    a.long_meta = st.pc_long_meta;
     a.nhuge = st.pc_nhuge;
     a.huge_li = st.pc_huge_li;
     a.cfy = coupled ? pick_prec<T>(st.cfy32, st.cfy64) : nullptr;
@@ -1601,14 +1668,13 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     a.dinv = dinv;
     a.x = x;
     a.r = r;
-    a.z = z;
     a.p = p;
     a.q = q;
     a.part_stride = CP * (3 + SG);
     a.max_iter = max_iter;
     const std::string tag = std::is_same<T, float>::value ? "pc32_" : "pc64_";
     B_CHECK(get_buf(ctx, tag + "lpart", static_cast<size_t>(std::max<int64_t>(st.pc_nlchunks, 1)) * CP, &a.lpart));
-    B_CHECK(get_buf(ctx, tag + "cta_part", static_cast<size_t>(nb) * a.part_stride, &a.cta_part));
+    B_CHECK(get_buf(ctx, tag + "cta_part", static_cast<size_t>(nb_max) * a.part_stride, &a.cta_part));
     double* thr_d;
     B_CHECK(get_buf(ctx, tag + "thr", CP, &thr_d));
     B_CHECK(get_buf(ctx, tag + "rz", CP, &a.rz_out));
@@ -1625,8 +1691,36 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     void* args[] = {&a};
     {
         ProfScope ps(ctx, B200FE_PROF_PASS, 0.0);
-        const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(nb),
-                                                          dim3(kPcgThreads), args, smem, s);
+        auto launch = [&](bool as_cluster) -> cudaError_t {
+            const void* kern = reinterpret_cast<const void*>(as_cluster ? kern_cluster : kern_grid);
+            cudaError_t e = raise_smem_limit(kern, static_cast<int>(smem));
+            if (e != cudaSuccess) return e;
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = dim3(as_cluster ? kPcgMinCtas : ctx->num_sms);
+            lc.blockDim = dim3(NT);
+            lc.dynamicSmemBytes = smem;
+            lc.stream = s;
+            cudaLaunchAttribute at[1];
+            if (as_cluster) {
+                e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                if (e != cudaSuccess) return e;
+                at[0].id = cudaLaunchAttributeClusterDimension;
+                at[0].val.clusterDim.x = kPcgMinCtas;
+                at[0].val.clusterDim.y = 1;
+                at[0].val.clusterDim.z = 1;
+            } else {
+                at[0].id = cudaLaunchAttributeCooperative;
+                at[0].val.cooperative = 1;
+            }
+            lc.attrs = at;
+            lc.numAttrs = 1;
+            return cudaLaunchKernelExC(&lc, kern, args);
+        };
+        cudaError_t e = launch(cluster);
+        if (e != cudaSuccess && cluster) {
+            cudaGetLastError();
+            e = launch(false);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             B_TRY(cudaStreamSynchronize(s));  // thr_host copy done before the caller's fallback
@@ -1889,7 +1983,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                 B_LAUNCHED();
                 int prc = B200FE_UNAVAILABLE;
                 if (st.sparse && ctx->persistent)
-                    prc = pcg_persistent<float, CQ>(ctx, w32, dinv32_use, x32, r32, z32, p32, q32, thr,
+                    prc = pcg_persistent<float, CQ>(ctx, w32, dinv32_use, x32, r32, p32, q32, thr,
                                                     round_cap, &its);
                 if (prc == B200FE_UNAVAILABLE)
                     B_CHECK((pcg<float, CQ>(ctx, w32, st.wp32, st.run_w32, st.block_w32, dinv32_use, x32, r32, z32, p32, q32, thr,
@@ -1904,7 +1998,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                 B_LAUNCHED();
                 int prc = B200FE_UNAVAILABLE;
                 if (st.sparse && ctx->persistent)
-                    prc = pcg_persistent<double, CQ>(ctx, w64, dinv64_use, x64, rin64, z64, p64, q64, thr,
+                    prc = pcg_persistent<double, CQ>(ctx, w64, dinv64_use, x64, rin64, p64, q64, thr,
                                                      round_cap, &its);
                 if (prc == B200FE_UNAVAILABLE)
                     B_CHECK((pcg<double, CQ>(ctx, w64, st.wp64, st.run_w64, st.block_w64, dinv64_use, x64, rin64, z64, p64, q64, thr,

@@ -56,6 +56,17 @@ struct LargeDim {
     int32_t *sup_c0 = nullptr, *sup_c1 = nullptr;      // [nsup] chunk range of each super-chunk
 };
 
+// Tiles of short rows of the explicit Schur block (pcg_kernels.cuh), built on
+// first use: with a coupled small dim they depend on the column pitch.
+struct PcgTiles {
+    bool built = false;
+    int64_t n = 0;
+    int2 *meta = nullptr, *rows = nullptr;
+    int32_t* col = nullptr;
+    double* val64 = nullptr;
+    float* val32 = nullptr;
+};
+
 struct Structure {
     bool valid = false;
     int64_t n = 0;
@@ -121,8 +132,9 @@ struct Structure {
     LargeDim sp;                       // chunk lists over the CSR rows (chunk fields only)
     // work lists of the persistent PCG over the same rows (pcg_kernels.cuh)
     int64_t pc_nshort = 0, pc_nlong = 0, pc_nlchunks = 0;
-    int4* pc_short_meta = nullptr;     // {row, begin, end, 0} of the short rows
-    int32_t *pc_long_rows = nullptr, *pc_long_c0 = nullptr, *pc_long_c1 = nullptr;
+    int32_t* pc_short_rows = nullptr;  // short rows, ascending
+    PcgTiles pc_tiles[3];              // tiles of short rows for 4, 8, 16 columns
+    int4* pc_long_meta = nullptr;      // {row, first chunk, last chunk + 1, 0} of the long rows
     int4* pc_lchunk_meta = nullptr;    // {row, begin, end, first} of the long-row chunks
     int64_t pc_nhuge = 0;
     int32_t* pc_huge_li = nullptr;

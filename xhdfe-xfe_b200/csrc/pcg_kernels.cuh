@@ -7,32 +7,43 @@
 // Jacobi (dinv).  Every column runs its own CG with its own mask; a column
 // stops when r'r <= thr[c] (or r'z stops being positive) and then keeps its x.
 //
-// One cooperative launch of NB CTAs (all resident) runs every iteration:
+// One launch of NB CTAs (all resident) runs every iteration:
 //
-//   A  q = S p for the large rows: "short" rows (<= kShortNnz nonzeros,
-//      including empty ones) by one lane group each, "long" rows in chunks of
-//      kLongChunk nonzeros by one warp each (partials).  The same warps form
-//      C_fy' p_f: each stages its rows' p and C_fy rows in shared memory and
-//      adds their outer product into registers (lane l keeps column l % CP of
-//      levels l / CP, l / CP + 32 / CP, ...), so C_fy is read once per
-//      iteration.  The dot p'q per CTA (by linearity also for long-row chunks
-//      and the small rows).
+//   A  q = S p for the large rows.  "Long" rows are cut into chunks of
+//      kLongChunk nonzeros, one warp each (partials).  "Short" rows
+//      (<= kShortNnz nonzeros, including empty ones) are taken twice by the
+//      same warp: in row order for the products with C_fy (C_fy p_small, and
+//      C_fy' p_f in registers, so C_fy is read once per iteration; the next
+//      rows are copied to shared memory meanwhile), and in tiles of eight
+//      rows of about equal length (PcgTiles) for the gathers of p, the next
+//      tile's nonzeros copied meanwhile.  The dot p'q per CTA (by linearity
+//      also for long-row chunks and small rows).
 //   -- grid barrier --
 //   B  alpha = r'z / p'q (every CTA reduces the NB partials in the same order,
-//      so all hold the same alpha); long rows and small rows are finished
-//      round-robin over CTAs and updated; then every CTA updates its
-//      contiguous range of short rows: x += alpha p, r -= alpha q, z = dinv r,
-//      with per-CTA partials of r'z and r'r.
+//      so all hold the same alpha); long and small rows are finished, a warp
+//      or a CTA each; r -= alpha q over the CTA's contiguous range of short
+//      rows; per-CTA partials of r'z and r'r with z = dinv r.
 //   -- grid barrier --
-//   C  new r'z, r'r, beta, masks (again the same in every CTA); p = z + beta p
-//      over the CTA's contiguous range of all rows.
+//   C  new r'z, r'r, beta, masks (again the same in every CTA); x += alpha p
+//      and p = z + beta p over the CTA's contiguous range of all rows.
 //   -- grid barrier --
 //
 // Data written by other CTAs during the launch is read with ld.global.cg (L2;
 // L1 is not coherent across CTAs).  Every sum has a fixed order, so results
 // are bitwise reproducible.  The barrier's wait is bounded (kBarrierCycles):
 // on timeout it sets *status and every CTA leaves at its next barrier.
-
+//
+// What bounds it: small systems by latency (three barriers and some ten
+// dependent L2 reads an iteration), large ones by the gathers of p from L2,
+// the shared-memory reads of the C_fy products and the vector passes.  Hence
+// one CTA per SM, sums by shuffles with one CTA-wide barrier each, no z array,
+// x updated where p is read anyway, lanes of a quad on one shared-memory
+// address (an LDS.128 then takes 2 cycles instead of 4), rows in tiles of
+// equal length (no lane of a warp waits for another row's nonzeros), and FP32
+// -> FP64 by shifts in the gathers.  Per iteration (B200, FP32): 10k rows
+// 2-way, 4 columns 28.0 -> 9.4 us; 300k rows 3-way, 4 columns 47 -> 19; 5M rows
+// 3-way, 16 columns 72 -> 44; 50M rows 366 -> 251; FP64, 1M rows 3-way, 16
+// columns 46 -> 32.
 #pragma once
 
 #include <cstdint>
@@ -42,12 +53,30 @@
 
 namespace b200fe {
 
-constexpr int kPcgThreads = 256;
 constexpr int kShortNnz = 32;        // rows with at most this many nonzeros: one lane group
 constexpr int kLongChunk = 256;      // nonzeros per warp chunk of a long row
 constexpr int kPcgMaxSG = 64;        // small-dim rows the kernel handles (coupled levels)
-constexpr int kHugeChunks = 32;      // long rows with more chunks: summed by a whole CTA
+constexpr int kHugeChunks = 16;      // long rows with more chunks: summed by a whole CTA
+constexpr int kPcgRowsPerWarp = 8;   // short rows per warp step
+constexpr int kPcgListsPerSm = 16;   // summation lists of C_fy' p_f per SM: the warps of the FP32 grid's CTA
+constexpr int kPcgMinCtas = 16;      // CTAs of the smallest launch
+constexpr int kPcgOwnRows = (kPcgMaxSG + kPcgMinCtas - 1) / kPcgMinCtas;  // small rows a CTA finishes, at most
+// Rows of p gathered per iteration, in bytes, up to which the launch is one
+// cluster of kPcgMinCtas CTAs: there an iteration is a chain of L2 latencies
+// and barriers, and the hardware barrier of 16 CTAs with 16 partials to add is
+// shorter than the grid's; above it 16 SMs are too few.  Per iteration on B200
+// (FP32, 4 columns), cluster against grid: 10k rows 2-way 9.5 / 12.6 us, 100k
+// rows 2-way 10.0 / 12.9, 300k rows 3-way (about 1 MB) 16.6 / 16.6, 1M rows
+// 2-way 19.6 / 13.7.
+constexpr double kPcgClusterBytes = 1e6;
 constexpr long long kBarrierCycles = 4000000000LL;  // ~2 s at 1.9 GHz
+
+// One CTA per SM (16 warps in FP32, kPcgListsPerSm): half as many arrivals and partials per grid barrier as with
+// two, and the registers a thread needs (128 in FP32, more in FP64).
+template <typename T>
+__host__ __device__ constexpr int pcg_threads() {
+    return sizeof(T) == 4 ? 512 : 256;
+}
 
 template <typename T>
 struct PcgArgs {
@@ -58,21 +87,25 @@ struct PcgArgs {
     const int32_t* col;
     const T* val;
     int64_t nshort;
-    const int4* short_meta;     // rows with <= kShortNnz nonzeros, ascending: {row, begin, end, 0}
+    const int32_t* short_rows;  // rows of at most kShortNnz nonzeros, ascending
+    int64_t ntiles;             // tiles of short rows (PcgTiles)
+    const int2* tile_meta;      // {first entry / 4, entries}
+    const int2* tile_rows;      // [ntiles][8] {row or -1, first entry in the tile | nonzeros << 16}
+    const int32_t* tile_col;
+    const T* tile_val;
+    int lists;                  // summation lists of C_fy' p_f (see the kernel)
+    int cbuf;                   // staging buffers of the coupling step (1 or 2)
     int64_t nlchunks;           // chunks of long rows (kLongChunk nonzeros each)
     const int4* lchunk_meta;    // {row, begin, end, 1 for the row's first chunk}
     int64_t nlong;
-    const int32_t* long_rows;   // [nlong] row of each long row
-    const int32_t* long_c0;     // [nlong] its chunk range in lchunk_*
-    const int32_t* long_c1;
+    const int4* long_meta;      // [nlong] {row, first chunk, last chunk + 1, 0}
     int64_t nhuge;              // long rows of more than kHugeChunks chunks
-    const int32_t* huge_li;     // [nhuge] their index in long_rows
+    const int32_t* huge_li;     // [nhuge] their index in long_meta
     const T* cfy;               // [Gf][SGP] or null
     const double* cyy;          // [SG][SG] or null
     const T* dinv;              // [GR]
     T* x;
     T* r;
-    T* z;
     T* p;
     T* q;
     double* lpart;              // [nlchunks][CP]
@@ -84,7 +117,7 @@ struct PcgArgs {
     double* rz_out;             // [CP]
     int* iters_out;             // [CP] iterations while active
     int* loops_out;             // [1] iterations run
-    unsigned int* bar;          // [2] grid barrier: arrivals, generation (zero at launch)
+    unsigned int* bar;          // [1] grid barrier: arrivals since the launch (zero at launch)
     int* status;                // [1] 0 ok; 2 barrier timeout
 };
 
@@ -105,84 +138,29 @@ __device__ __forceinline__ void v4_store(double* p, const V4<double>& a) {
     reinterpret_cast<double2*>(p)[1] = make_double2(a.v[2], a.v[3]);
 }
 
-// Dynamic shared memory of pcg_persistent_kernel: small rows of p [64][CP],
-// per-warp staging of GPW rows of p and C_fy, the CTA's C_fy' p_f partial.
+// A warp's slab in shared memory (byte offsets): two buffers of a tile's
+// {columns, values}; with a coupled small dim cbuf buffers of a coupling
+// step's rows of {p, C_fy} and one such row; the warp's C_fy' p_f in FP64
+// [SG][CP] takes the front of the slab at the end of phase A.
 template <typename T>
-__host__ __device__ constexpr size_t pcg_smem_bytes(int CP, int SGP) {
+struct PcgSlab {
+    int val, buf, step, step_bytes, row, bytes;
+    __host__ __device__ constexpr PcgSlab(int CP, int SG, int SGP, int cbuf)
+        : val(kPcgRowsPerWarp * kShortNnz * 4),
+          buf(val + kPcgRowsPerWarp * kShortNnz * static_cast<int>(sizeof(T))),
+          step(2 * buf),
+          step_bytes(SG > 0 ? 128 / CP * (CP + SGP) * static_cast<int>(sizeof(T)) : 0),
+          row(step + cbuf * step_bytes),
+          bytes(row + (SG > 0 ? (CP + SGP) * static_cast<int>(sizeof(T)) : 0)) {
+        if (bytes < SG * CP * 8) bytes = SG * CP * 8;
+    }
+};
+// Dynamic shared memory of pcg_persistent_kernel: small rows of p [64][CP] and
+// the warps' slabs.
+template <typename T>
+__host__ __device__ constexpr size_t pcg_smem_bytes(int CP, int SG, int SGP, int cbuf) {
     return align16(static_cast<size_t>(kPcgMaxSG) * CP * sizeof(T)) +
-           align16(static_cast<size_t>(kPcgThreads / 32) * (32 / (CP / 4)) * (CP + SGP) * sizeof(T)) +
-           static_cast<size_t>(kPcgMaxSG) * CP * sizeof(double);
-}
-
-// Grid-wide barrier for a cooperative launch, bounded: returns false (and
-// sets *status) when the wait exceeds kBarrierCycles or another CTA gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, int* status) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* gen = bar + 1;
-        const unsigned int g = *gen;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(bar, 1u);
-        int ok = 1;
-        if (arrived == gridDim.x - 1) {
-            bar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            const long long t0 = clock64();
-            while (*gen == g) {
-                if (*reinterpret_cast<volatile int*>(status) != 0 || clock64() - t0 > kBarrierCycles) {
-                    atomicOr(status, 2);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        if (*reinterpret_cast<volatile int*>(status) != 0) ok = 0;
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s != 0;
-}
-
-// sum over CTAs b of part[b * stride + off + c] for c < CP, in CTA order
-// within each thread's slice and a fixed tree across slices; the result is
-// valid in threads c < CP.
-__device__ __forceinline__ double cta_column_sum(const double* part, int nb, int stride, int off,
-                                                 int CP, double* red) {
-    const int t = threadIdx.x;
-    const int J = kPcgThreads / CP;
-    const int c = t % CP, j = t / CP;
-    double s = 0.0;
-    for (int b = j; b < nb; b += J) s += __ldcg(part + static_cast<int64_t>(b) * stride + off + c);
-    red[t] = s;
-    __syncthreads();
-    for (int h = J / 2; h > 0; h >>= 1) {
-        if (j < h) red[t] += red[t + h * CP];
-        __syncthreads();
-    }
-    const double v = red[c];
-    __syncthreads();
-    return v;
-}
-
-// per-column sum of one value per thread (thread t holds column t % CP)
-__device__ __forceinline__ double cta_reduce_by_column(double v, int CP, double* red) {
-    const int t = threadIdx.x;
-    const int J = kPcgThreads / CP;
-    const int j = t / CP;
-    red[t] = v;
-    __syncthreads();
-    for (int h = J / 2; h > 0; h >>= 1) {
-        if (j < h) red[t] += red[t + h * CP];
-        __syncthreads();
-    }
-    const double s = red[t % CP];
-    __syncthreads();
-    return s;
+           static_cast<size_t>(pcg_threads<T>() / 32) * PcgSlab<T>(CP, SG, SGP, cbuf).bytes;
 }
 
 // 16-byte asynchronous copy global -> shared (cached in L2 only); the
@@ -194,23 +172,23 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// Per-column CTA sums of four values per thread: thread t holds columns
-// 4 (t % CQ) .. 4 (t % CQ) + 3; fixed tree over the threads of one column
-// quad.  out[c] (shared, CP entries) is valid after the call.
-__device__ __forceinline__ void cta_reduce_quads(const double (&v)[4], int CQ, double* red, double* out) {
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        red[t] = v[i];
-        __syncthreads();
-        for (int h = kPcgThreads / 2; h >= CQ; h >>= 1) {
-            if (t < h) red[t] += red[t + h];
-            __syncthreads();
-        }
-        if (t < CQ) out[4 * t + i] = red[t];
-        __syncthreads();
-    }
+// 2^-896 times a finite value as FP64, exactly (zeros and subnormals too), and
+// the factor that undoes it: an FP32 -> FP64 conversion per gathered element
+// is what the gathers wait for (2-way 50M rows, 16 columns: 189 us an iteration
+// with conversions, 151 with shifts), and the factor goes into the other operand
+// of the product, once for the four columns of a lane.
+__device__ __forceinline__ double scaled64(float x) {
+    const int u = __float_as_int(x);
+    return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
 }
+__device__ __forceinline__ double scaled64(double x) { return x; }
+template <typename T>
+__device__ __forceinline__ double unscale64() {
+    return sizeof(T) == 4 ? 0x1p896 : 1.0;
+}
+// z = M^-1 r: the FP32 product rounded once, as the exact FP64 product would be
+__device__ __forceinline__ float precond(float d, float r) { return __fmul_rn(d, r); }
+__device__ __forceinline__ double precond(double d, double r) { return __dmul_rn(d, r); }
 
 // q += sum over nonzeros j of val[j] p[col[j]] (4 columns of this lane) for
 // j = j0, j0 + step, ... < je, U nonzeros per batch; the next batch's column
@@ -234,9 +212,9 @@ __device__ __forceinline__ void gather_rows(const int32_t* __restrict__ col, con
             if (cj[u] >= 0) v4_load_cg(p + static_cast<int64_t>(cj[u]) * CP + 4 * q4, xv[u]);
             else v4_zero(xv[u]);
         }
-        T vc[U];
+        double vc[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) vc[u] = vj[u];
+        for (int u = 0; u < U; ++u) vc[u] = static_cast<double>(vj[u]) * unscale64<T>();
         const int32_t jn = jb + U * step;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -248,14 +226,10 @@ __device__ __forceinline__ void gather_rows(const int32_t* __restrict__ col, con
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                acc.v[i] = fma(static_cast<double>(vc[u]), static_cast<double>(xv[u].v[i]), acc.v[i]);
+                acc.v[i] = fma(vc[u], scaled64(xv[u].v[i]), acc.v[i]);
     }
 }
 
-// Per-warp outer-product accumulation of C_fy' p_f over the rows the warp
-// staged (slab: nrows rows of [p (CP) | C_fy (SGP)]).  The [SGP/4][CP/4]
-// blocks of 4 levels x 4 columns are dealt to the lanes (block l and l + 32),
-// so a row costs a lane two 128-bit shared loads and 16 FMAs per block.
 template <typename T>
 __device__ __forceinline__ void lds4(const T* p, T (&v)[4]);
 template <>
@@ -270,521 +244,718 @@ __device__ __forceinline__ void lds4<double>(const double* p, double (&v)[4]) {
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
-template <typename T, int CQ>
-__device__ __forceinline__ void couple_rows(const T* slab, int nrows, int SGP, int lane,
-                                            T (&cacc)[2][16]) {
-    constexpr int CP = 4 * CQ;
-    const int nblk = (SGP / 4) * CQ;
-    for (int r = 0; r < nrows; ++r) {
-        const T* row = slab + r * (CP + SGP);
+// C_fy' p_f in registers: lane (hs, q4) keeps levels hs, hs + HS, ... (KH of
+// them) of column quad q4, row after row.
+template <typename T, int CQ, int KH>
+struct PcgCouple {
+    static constexpr int CP = 4 * CQ;
+    static constexpr int HS = 32 / CQ;
+    T acc[KH][4];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int bk = lane + 32 * k;
-            if (bk < nblk) {
-                const int lq = bk / CQ, cq = bk % CQ;
-                T pv[4], cv[4];
-                lds4<T>(row + 4 * cq, pv);
-                lds4<T>(row + CP + 4 * lq, cv);
+        for (int k = 0; k < KH; ++k)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 4; ++i) acc[k][i] = T(0);
+    }
+    __device__ __forceinline__ void row(const T* crow, const T* prow, int SG, int hs, int q4) {
+        T pv[4];
+        lds4<T>(prow + 4 * q4, pv);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) cacc[k][4 * i + j] = fma(cv[i], pv[j], cacc[k][4 * i + j]);
-            }
+        for (int k = 0; k < KH; ++k) {
+            const int h = hs + HS * k;
+            const T c = h < SG ? crow[h] : T(0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[k][i] = fma(c, pv[i], acc[k][i]);
+        }
+    }
+};
+// C_fy[row] p_small for a column quad of xs (rows of CP), level after level
+template <typename T, int CP>
+__device__ __forceinline__ void couple_dot(const T* crow, const T* xs, int SGP, T (&cs)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cs[i] = T(0);
+#pragma unroll 2
+    for (int h = 0; h < SGP; h += 4) {
+        T c4[4];
+        lds4<T>(crow + h, c4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            T xr[4];
+            lds4<T>(xs + (h + u) * CP, xr);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cs[i] = fma(c4[u], xr[i], cs[i]);
         }
     }
 }
 
-template <typename T, int CQ>
-__global__ void __launch_bounds__(kPcgThreads, sizeof(T) == 4 ? 2 : 1)
-pcg_persistent_kernel(const PcgArgs<T> a) {
+// CLUSTER: the whole grid is one thread-block cluster and meets at the
+// hardware cluster barrier; otherwise a cooperative launch of one CTA per SM.
+// KH: levels of the small dim per lane (PcgCouple); 0 without coupling.
+//
+// C_fy' p_f is summed in the solve precision over a.lists lists (list v: the
+// first chunks of long rows among chunks v, v + lists, ..., then steps
+// v, v + lists, ... of 32 / CQ short rows in row order), the lists' sums in
+// FP64; a warp takes whole lists.  C_fy's rows cancel (a balanced row sums to
+// zero over the levels), so the rounding of these FP32 sums shows in badly
+// identified rows of the answer: neither the lists nor the level order of
+// C_fy p_small depend on the launch, and the answer depends on it only through
+// FP64 rounding.
+template <typename T, int CQ, int KH, bool CLUSTER>
+__global__ void __launch_bounds__(pcg_threads<T>(), 1) pcg_persistent_kernel(const PcgArgs<T> a) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr bool coupled = KH > 0;
+    constexpr bool LISTS = coupled && CLUSTER && sizeof(T) == 4;  // a warp takes several lists
+    constexpr int NT = pcg_threads<T>();
+    constexpr int NW = NT / 32;
     constexpr int CP = 4 * CQ;
-    constexpr int GPW = 32 / CQ;  // lane groups per warp
-    constexpr int U = 8;          // gathers in flight per lane group
-    __shared__ double red[kPcgThreads];
-    __shared__ double s_alpha[CP], s_beta[CP], s_rz[CP], s_pq[CP], s_q1[CP], s_q2[CP];
+    static_assert(sizeof(T) != 4 || NW == kPcgListsPerSm, "one list per warp of the FP32 grid");
+    constexpr int RW = kPcgRowsPerWarp;
+    constexpr int LPR = 32 / RW;  // lanes per short row
+    constexpr int SR = 32 / CQ;   // short rows per coupling step
+    constexpr int J = LPR / CQ;   // of which this many share a column quad
+    constexpr int U = sizeof(T) == 4 ? 8 : 4;  // gathers in flight per lane
+    __shared__ double red_q[2][NW][CP], red_c[2][NW][CP], red_s[2][NW][CP];
+    __shared__ double s_alpha[CP], s_beta[CP], s_rz[CP];
     __shared__ int s_active[CP], s_iters[CP];
-    __shared__ int s_any;
+    __shared__ int s_any, s_ok;
+    __shared__ double s_cyy[coupled ? kPcgOwnRows : 1][kPcgMaxSG], s_yq[kPcgOwnRows][CP];  // this CTA's small rows
     extern __shared__ __align__(16) unsigned char pcg_smem_raw[];
     T* s_xs = reinterpret_cast<T*>(pcg_smem_raw);  // [kPcgMaxSG][CP] small rows of p
-    T* s_stage = reinterpret_cast<T*>(pcg_smem_raw + align16(static_cast<size_t>(kPcgMaxSG) * CP * sizeof(T)));
-    double* s_cpart = reinterpret_cast<double*>(
-        pcg_smem_raw + align16(static_cast<size_t>(kPcgMaxSG) * CP * sizeof(T)) +
-        align16(static_cast<size_t>(kPcgThreads / 32) * GPW * (CP + a.SGP) * sizeof(T)));
-
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int gw = lane / CQ;
-    const int q4 = lane % CQ;
     const int NB = gridDim.x;
     const int b = blockIdx.x;
     const int64_t GR = a.Gf + a.SG;
     const int PS = a.part_stride;
-    const bool coupled = a.SG > 0;
+    const int SG = a.SG, SGP = a.SGP;
     double* mypart = a.cta_part + static_cast<int64_t>(b) * PS;
-    T* slab = s_stage + static_cast<size_t>(warp) * GPW * (CP + a.SGP);  // this warp's staging
+    const PcgSlab<T> sl(CP, SG, SGP, a.cbuf);
+    unsigned char* s_slabs = pcg_smem_raw + align16(static_cast<size_t>(kPcgMaxSG) * CP * sizeof(T));
+    unsigned char* slab = s_slabs + static_cast<size_t>(warp) * sl.bytes;  // this warp's staging
     // contiguous row range owned by this CTA (updates, directions)
     const int64_t r0 = GR * b / NB, r1 = GR * (b + 1) / NB;
-    const int c_of_t = tid % CP;  // column of this thread in flat row loops (256 % CP == 0)
-    const int npairs = a.SG * CP;
+    const int c_of_t = tid % CP;  // column of this thread where a thread owns one column
+    const int tq = tid % CQ;      // column quad of this thread where it owns four
+    // lane (gw, jl, q4): row gw of a tile, every J-th of its nonzeros from jl on,
+    // column quad q4; once the J shares have met, the lane owns columns
+    // oc .. oc + CQ of the row.  With the row in the low bits, lanes of one
+    // quad share the address of a row of p_small or p in shared memory.
+    const int gw = lane & (RW - 1);
+    const int q4 = (lane / RW) % CQ;
+    const int jl = lane / (RW * CQ);
+    const int oc = 4 * q4 + jl * CQ;
+    const int hs = gw + RW * jl;
+    const int npairs = SG * CP;
+    unsigned int epoch = 0;
 
-    // ---- init: x = 0, z = dinv r, p = z; partials of r'z, r'r ----
+    // CTA sums of K values: v[k][i] of column 4 (lane % CQ) + i, and w[k] of
+    // column lane % CP; thread c < CP stores the sum of column c at
+    // mypart[off[k] + c], then the grid meets.  Everything the CTA wrote
+    // before is visible to the CTAs that have passed the barrier.
+    auto publish = [&](auto& v, auto& w, const int (&off)[2], int K) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k >= K) break;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                double t = v[k][i];
+#pragma unroll
+                for (int o = 16; o >= CQ; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+                if (lane < CQ) red_q[k][warp][4 * lane + i] = t;
+            }
+            double t = w[k];
+#pragma unroll
+            for (int o = 16; o >= CP; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+            if (lane < CP) red_c[k][warp][lane] = t;
+        }
+        __syncthreads();
+        if (tid < CP) {
+            for (int k = 0; k < K; ++k) {
+                double s = 0.0;
+#pragma unroll
+                for (int j = 0; j < NW; ++j) s += red_q[k][j][tid] + red_c[k][j][tid];
+                mypart[off[k] + tid] = s;
+            }
+        }
+    };
+    // the same for p'q: dot of columns oc .. in the lanes gw = 0, w of column lane % CP
+    auto publish_own = [&](const double (&dot)[CQ], const double (&w)[2]) {
+        if (gw == 0) {
+#pragma unroll
+            for (int i = 0; i < CQ; ++i) red_q[0][warp][oc + i] = dot[i];
+        }
+        double t = w[0];
+#pragma unroll
+        for (int o = 16; o >= CP; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+        if (lane < CP) red_c[0][warp][lane] = t;
+        __syncthreads();
+        if (tid < CP) {
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < NW; ++j) s += red_q[0][j][tid] + red_c[0][j][tid];
+            mypart[tid] = s;
+        }
+    };
+    auto meet = [&]() -> bool {
+        if (CLUSTER) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            return true;
+        }
+        ++epoch;
+        if (warp == 0) {
+            __syncwarp();
+            if (lane == 0) {
+                int ok = 1;
+                const unsigned int target = epoch * static_cast<unsigned int>(NB);
+                __threadfence();
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+                unsigned int seen;
+                long long t0 = 0;
+                for (unsigned int spin = 1;; ++spin) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+                    if (seen >= target) break;
+                    if ((spin & 255u) == 0) {  // now and then: has the wait run out, here or elsewhere
+                        const long long t = clock64();
+                        if (t0 == 0) t0 = t;
+                        if (*reinterpret_cast<volatile int*>(a.status) != 0 || t - t0 > kBarrierCycles) {
+                            atomicOr(a.status, 2);
+                            ok = 0;
+                            break;
+                        }
+                    }
+                }
+                s_ok = ok;
+            }
+        }
+        __syncthreads();
+        return s_ok != 0;
+    };
+    // sum over CTAs of part[cta * stride + off[k] + c]: returned to threads
+    // c < CP (fixed order: a thread's slice, a shuffle tree, the warps in order)
+    auto col_sums = [&](const double* part, int nparts, int stride, int off0, int off1, int K, double (&out)[2]) {
+        double s[2] = {0.0, 0.0};
+        for (int i = tid / CP; i < nparts; i += NT / CP) {
+            const double* src = part + static_cast<int64_t>(i) * stride + c_of_t;
+            s[0] += __ldcg(src + off0);
+            if (K > 1) s[1] += __ldcg(src + off1);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k >= K) break;
+#pragma unroll
+            for (int o = 16; o >= CP; o >>= 1) s[k] += __shfl_xor_sync(kFull, s[k], o);
+            if (lane < CP) red_s[k][warp][lane] = s[k];
+        }
+        __syncthreads();
+        out[0] = out[1] = 0.0;
+        if (tid < CP) {
+            for (int k = 0; k < K; ++k) {
+                double t = 0.0;
+#pragma unroll
+                for (int j = 0; j < NW; ++j) t += red_s[k][j][tid];
+                out[k] = t;
+            }
+        }
+    };
+    const int off_rr[2] = {CP * (1 + SG), CP * (2 + SG)};
+
+    if (coupled)
+        for (int i = tid; i < kPcgOwnRows * SG; i += NT) {
+            const int k = i / SG, h = b + k * NB;
+            if (h < SG) s_cyy[k][i - k * SG] = __ldg(a.cyy + h * SG + i - k * SG);
+        }
+
+    // ---- init: x = 0, p = z = dinv r; partials of r'z, r'r ----
     // (streaming loops: a thread owns column quad tq of rows in its CTA's
     // range, two quads in flight, every load issued before the stores)
-    const int tq = tid % CQ;
     {
-        double rz4[4] = {0.0, 0.0, 0.0, 0.0}, rr4[4] = {0.0, 0.0, 0.0, 0.0};
+        double v[2][4] = {}, w[2] = {0.0, 0.0};
         const int64_t e1 = r1 * CQ;
-        for (int64_t e = r0 * CQ + tid; e < e1; e += 2 * kPcgThreads) {
-            const int64_t eb = e + kPcgThreads;
-            const bool vb = eb < e1;
-            V4<T> rv[2];
-            T dv[2];
-            v4_load_cg(a.r + 4 * e, rv[0]);
-            dv[0] = __ldg(a.dinv + e / CQ);
-            if (vb) {
-                v4_load_cg(a.r + 4 * eb, rv[1]);
-                dv[1] = __ldg(a.dinv + eb / CQ);
-            }
+        for (int64_t e = r0 * CQ + tid; e < e1; e += NT) {
+            V4<T> rv, zv, xz;
+            v4_load_cg(a.r + 4 * e, rv);
+            const T dv = __ldg(a.dinv + e / CQ);
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (k == 1 && !vb) break;
-                const int64_t ee = k ? eb : e;
-                V4<T> zv, xz;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const double ri = static_cast<double>(rv[k].v[i]);
-                    zv.v[i] = static_cast<T>(static_cast<double>(dv[k]) * ri);
-                    xz.v[i] = T(0);
-                    rz4[i] = fma(ri, static_cast<double>(zv.v[i]), rz4[i]);
-                    rr4[i] = fma(ri, ri, rr4[i]);
-                }
-                v4_store(a.x + 4 * ee, xz);
-                v4_store(a.z + 4 * ee, zv);
-                v4_store(a.p + 4 * ee, zv);
+            for (int i = 0; i < 4; ++i) {
+                const double ri = static_cast<double>(rv.v[i]);
+                zv.v[i] = precond(dv, rv.v[i]);
+                xz.v[i] = T(0);
+                v[0][i] = fma(ri, static_cast<double>(zv.v[i]), v[0][i]);
+                v[1][i] = fma(ri, ri, v[1][i]);
             }
+            v4_store(a.x + 4 * e, xz);
+            v4_store(a.p + 4 * e, zv);
         }
-        cta_reduce_quads(rz4, CQ, red, s_q1);
-        cta_reduce_quads(rr4, CQ, red, s_q2);
-        if (tid < CP) {
-            mypart[CP * (1 + a.SG) + tid] = s_q1[tid];
-            mypart[CP * (2 + a.SG) + tid] = s_q2[tid];
-        }
+        publish(v, w, off_rr, 2);
     }
-    if (!grid_barrier(a.bar, a.status)) return;
+    if (!meet()) return;
     {
-        const double rz = cta_column_sum(a.cta_part, NB, PS, CP * (1 + a.SG), CP, red);
-        const double rr = cta_column_sum(a.cta_part, NB, PS, CP * (2 + a.SG), CP, red);
-        if (tid < CP) {
-            s_rz[tid] = rz;
-            s_iters[tid] = 0;
-            s_active[tid] = (a.thr[tid] > 0.0 && rr > a.thr[tid] && rz > 0.0) ? 1 : 0;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            int any = 0;
-            for (int c = 0; c < CP; ++c) any |= s_active[c];
-            s_any = any;
+        double s[2];
+        col_sums(a.cta_part, NB, PS, off_rr[0], off_rr[1], 2, s);
+        if (warp == 0) {
+            int act = 0;
+            if (lane < CP) {
+                s_rz[lane] = s[0];
+                s_iters[lane] = 0;
+                act = (a.thr[lane] > 0.0 && s[1] > a.thr[lane] && s[0] > 0.0) ? 1 : 0;
+                s_active[lane] = act;
+            }
+            const int any = __any_sync(kFull, act);
+            if (lane == 0) s_any = any;
         }
         __syncthreads();
     }
 
+    const int64_t nwarps = static_cast<int64_t>(NB) * NW;
+    // warps of different CTAs get neighbouring work items, so that few items
+    // spread over many SMs
+    const int64_t wid = static_cast<int64_t>(warp) * NB + b;
     int it = 0;
     while (s_any && it < a.max_iter) {
         // ================= A: q = S p, C_fy' p_f, dots =================
         if (coupled) {
-            for (int i = tid; i < a.SGP * CP; i += kPcgThreads)
-                s_xs[i] = i < a.SG * CP ? __ldcg(a.p + a.Gf * CP + i) : T(0);
+            for (int i = tid; i < SGP * CP; i += NT) s_xs[i] = i < npairs ? __ldcg(a.p + a.Gf * CP + i) : T(0);
             __syncthreads();
         }
-        T cacc[2][16];  // this lane's 4x4 blocks of C_fy' p_f (see couple_rows)
+        double w[2] = {0.0, 0.0}, dot[CQ] = {};  // dot: the lane's own columns
+        // C_fy' p_f of the warp's current list, and of its lists before (an FP32
+        // grid has one list per warp, an FP64 sum needs no lists)
+        PcgCouple<T, CQ, coupled ? KH : 1> cpl;
+        cpl.zero();
+        double cdot[LISTS ? KH : 1][4] = {};
+        // own columns of a quad's sums
+        auto own = [&](const Acc4& acc, double (&o)[CQ]) {
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+            for (int i = 0; i < CQ; ++i) {
+                o[i] = acc.v[i];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) cacc[k][i] = T(0);
-        double dot[4] = {0.0, 0.0, 0.0, 0.0};
-        const int64_t nwarps = static_cast<int64_t>(NB) * (kPcgThreads / 32);
-        const int64_t wid = static_cast<int64_t>(b) * (kPcgThreads / 32) + warp;
-        // long-row chunks: a warp each, lane groups interleave the nonzeros;
-        // the next chunk's record is loaded one chunk ahead
-        int4 lm = wid < a.nlchunks ? __ldg(a.lchunk_meta + wid) : make_int4(0, 0, 0, 0);
-        for (int64_t ch = wid; ch < a.nlchunks; ch += nwarps) {
-            const int32_t g = lm.x, jb = lm.y, je = lm.z;
-            const bool first = lm.w != 0;
-            if (ch + nwarps < a.nlchunks) lm = __ldg(a.lchunk_meta + ch + nwarps);
-            Acc4 acc;
-            acc_zero(acc);
-            gather_rows<T, CP, U>(a.col, a.val, a.p, jb + gw, je, GPW, q4, acc);
-            // lane groups of the warp combined by a butterfly (every lane gets
-            // the same sum)
+                for (int j = 1; j < J; ++j)
+                    if (jl == j) o[i] = acc.v[j * CQ + i];
+            }
+        };
+        // rows of a coupling step: lane (sr, sq) stages and owns quad sq of row sr
+        const int sr = lane % SR, sq = lane / SR;
+        const int64_t nsteps = coupled ? (a.nshort + SR - 1) / SR : 0;
+        const int64_t lists = coupled ? a.lists : nwarps;
+        for (int64_t v = wid; v < lists; v += nwarps) {
+            if (coupled && v >= a.nlchunks && v >= nsteps) break;  // this list and the later ones are empty
+            T* srow = reinterpret_cast<T*>(slab + sl.row);
+            // ---- long-row chunks: a warp each, lane groups interleave the
+            // nonzeros; the next chunk's record is loaded one chunk ahead
+            int4 lm = v < a.nlchunks ? __ldg(a.lchunk_meta + v) : make_int4(0, 0, 0, 0);
+            // the first rows of the coupling do not depend on the chunks
+            int64_t st = v;
+            auto short_row = [&](int64_t step) {
+                const int64_t i = step * SR + sr;
+                return step < nsteps && i < a.nshort ? __ldg(a.short_rows + i) : -1;
+            };
+            int32_t g = coupled ? short_row(st) : -1;
+            auto stage_step = [&](int k) {
+                T* d = reinterpret_cast<T*>(slab + sl.step + k * sl.step_bytes);
+                constexpr int VT = 16 / sizeof(T);  // elements per 16-byte copy
+                if (g >= 0) {
 #pragma unroll
-            for (int o = 16; o >= CQ; o >>= 1)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc.v[i] += __shfl_xor_sync(0xffffffffu, acc.v[i], o);
-            V4<T> pv;
-            v4_load_cg(a.p + static_cast<int64_t>(g) * CP + 4 * q4, pv);
-            if (coupled && first) {
-                // the row's first chunk carries C_fy[g] p_small, and adds the
-                // row to the warp's C_fy' p_f
-                const T* crow = a.cfy + static_cast<int64_t>(g) * a.SGP;
-                if (gw == 0) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) slab[4 * q4 + i] = pv.v[i];
+                    for (int i = 0; i < 4 / VT; ++i)
+                        cp_async16(d + sr * CP + 4 * sq + i * VT, a.p + static_cast<int64_t>(g) * CP + 4 * sq + i * VT);
+                    T* c = d + SR * CP + sr * SGP;
+                    const T* src = a.cfy + static_cast<int64_t>(g) * SGP;
+                    for (int i = sq; i < SGP / VT; i += CQ) cp_async16(c + i * VT, src + i * VT);
                 }
-                for (int h = lane; h < a.SGP; h += 32) slab[CP + h] = __ldg(crow + h);
-                __syncwarp();
-                T cs[4] = {T(0), T(0), T(0), T(0)};
-                for (int h0 = 0; h0 < a.SGP; h0 += 4) {
-                    T c4[4];
-                    lds4<T>(slab + CP + h0, c4);
+                cp_async_commit();
+            };
+            if (coupled) stage_step(0);
+            for (int64_t ch = v; ch < a.nlchunks; ch += lists) {
+                const int32_t row = lm.x, jb = lm.y, je = lm.z;
+                const bool first = lm.w != 0;
+                if (ch + lists < a.nlchunks) lm = __ldg(a.lchunk_meta + ch + lists);
+                T pv[CQ], cs[4] = {};
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        T xr[4];
-                        lds4<T>(s_xs + (h0 + u) * CP + 4 * q4, xr);
+                for (int i = 0; i < CQ; ++i) pv[i] = __ldcg(a.p + static_cast<int64_t>(row) * CP + oc + i);
+                if (coupled && first) {  // the row's first chunk carries its products with C_fy
+                    for (int h = lane; h < SGP; h += 32)
+                        srow[CP + h] = __ldg(a.cfy + static_cast<int64_t>(row) * SGP + h);
+                    if (gw == 0) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cs[i] = fma(c4[u], xr[i], cs[i]);
+                        for (int i = 0; i < CQ; ++i) srow[oc + i] = pv[i];
                     }
+                    __syncwarp();
+                    couple_dot<T, CP>(srow + CP, s_xs + 4 * q4, SGP, cs);
+                    cpl.row(srow + CP, srow, SG, sr, sq);
+                    __syncwarp();
+                }
+                Acc4 acc;
+                acc_zero(acc);
+                gather_rows<T, CP, U>(a.col, a.val, a.p, jb + hs, je, 32 / CQ, q4, acc);
+                // lane groups of the warp combined by a butterfly
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    if (o >= RW && o < RW * CQ) continue;  // the lane bits of the column quad
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc.v[i] += __shfl_xor_sync(kFull, acc.v[i], o);
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc.v[i] += static_cast<double>(cs[i]);
-                couple_rows<T, CQ>(slab, 1, a.SGP, lane, cacc);
-                __syncwarp();
-            }
-            if (gw == 0) {
-                double* dst = a.lpart + ch * CP + 4 * q4;
+                double qo[CQ];
+                own(acc, qo);
+                if (gw == 0) {
+                    double* dst = a.lpart + ch * CP + oc;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    dst[i] = acc.v[i];
-                    dot[i] = fma(static_cast<double>(pv.v[i]), acc.v[i], dot[i]);
-                }
-            }
-        }
-        // short rows: GPW rows per warp, one lane group each.  With a coupled
-        // small dim the row's C_fy row is copied into the warp's slab
-        // (cp.async) while the gather runs.
-        int4 sm = wid * GPW + gw < a.nshort ? __ldg(a.short_meta + wid * GPW + gw) : make_int4(0, 0, 0, 0);
-        for (int64_t base = wid * GPW; base < a.nshort; base += nwarps * GPW) {
-            const int64_t si = base + gw;
-            const bool valid = si < a.nshort;
-            const int32_t g = sm.x, jb = sm.y, je = sm.z;
-            {  // the next step's record, one step ahead
-                const int64_t sn = si + nwarps * GPW;
-                sm = sn < a.nshort ? __ldg(a.short_meta + sn) : make_int4(0, 0, 0, 0);
-            }
-            T* srow = slab + gw * (CP + a.SGP);
-            if (coupled) {
-                constexpr int VT = 16 / sizeof(T);  // elements per 16-byte copy
-                const T* crow = a.cfy + static_cast<int64_t>(g) * a.SGP;
-                for (int v = q4; v < a.SGP / VT; v += CQ) {
-                    if (valid) {
-                        cp_async16(srow + CP + v * VT, crow + v * VT);
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < VT; ++u) srow[CP + v * VT + u] = T(0);
+                    for (int i = 0; i < CQ; ++i) {
+                        dst[i] = qo[i];
+                        dot[i] = fma(static_cast<double>(pv[i]), qo[i], dot[i]);
                     }
                 }
-                cp_async_commit();
             }
-            Acc4 acc;
-            acc_zero(acc);
-            gather_rows<T, CP, U>(a.col, a.val, a.p, jb, je, 1, q4, acc);
-            V4<T> pv;
-            if (valid) v4_load_cg(a.p + static_cast<int64_t>(g) * CP + 4 * q4, pv);
-            else v4_zero(pv);
+            // ---- the list's short rows in order, SR per step: C_fy p_small into
+            // q (completed below by this warp) and C_fy' p_f
             if (coupled) {
+                for (int k = 0; st < nsteps; st += lists) {
+                    const int32_t gc = g;
+                    const unsigned rows = __ballot_sync(kFull, sq == 0 && gc >= 0);
+                    g = short_row(st + lists);
+                    cp_async_wait_all();
+                    __syncwarp();
+                    const T* d = reinterpret_cast<const T*>(slab + sl.step + k * sl.step_bytes);
+                    if (a.cbuf == 2) stage_step(k ^= 1);
+                    if (gc >= 0) {
+                        T cs[4];
+                        couple_dot<T, CP>(d + SR * CP + sr * SGP, s_xs + 4 * sq, SGP, cs);
+                        V4<T> o;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o.v[i] = cs[i];
+                        v4_store(a.q + static_cast<int64_t>(gc) * CP + 4 * sq, o);
+                    }
+                    // rows of a step are a prefix of it
+                    const int nr = __popc(rows);
+#pragma unroll 8
+                    for (int r = 0; r < nr; ++r) cpl.row(d + SR * CP + r * SGP, d + r * CP, SG, sr, sq);
+                    __syncwarp();
+                    if (a.cbuf == 1) stage_step(0);
+                }
+                cp_async_wait_all();
+                if constexpr (LISTS) {
+#pragma unroll
+                    for (int k = 0; k < KH; ++k)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) cdot[k][i] += static_cast<double>(cpl.acc[k][i]);
+                    cpl.zero();
+                }
+                __syncwarp();
+            }
+            // ---- the same rows (without coupling: any) in tiles of about equal length
+            int64_t t = v, te = a.ntiles;
+            const int64_t ts = coupled ? 1 : nwarps;
+            if (coupled) {
+                const int64_t full = nsteps / lists, rest = nsteps - full * lists;
+                t = (v * full + min(v, rest)) * (SR / RW);
+                te = ((v + 1) * full + min(v + 1, rest)) * (SR / RW);
+            }
+            int2 tm = t < te ? __ldg(a.tile_meta + t) : make_int2(0, 0);
+            int2 row = t < te ? __ldg(a.tile_rows + t * RW + gw) : make_int2(-1, 0);
+            auto stage_tile = [&](int k) {
+                unsigned char* d = slab + k * sl.buf;
+                const unsigned char* c = reinterpret_cast<const unsigned char*>(a.tile_col + 4 * static_cast<int64_t>(tm.x));
+                const unsigned char* x = reinterpret_cast<const unsigned char*>(a.tile_val + 4 * static_cast<int64_t>(tm.x));
+                const int n16 = (tm.y + 3) >> 2;  // 16-byte pieces of the columns
+                for (int i = lane; i < n16; i += 32) cp_async16(d + 16 * i, c + 16 * i);
+                for (int i = lane; i < n16 * static_cast<int>(sizeof(T) / 4); i += 32)
+                    cp_async16(d + sl.val + 16 * i, x + 16 * i);
+                cp_async_commit();
+            };
+            stage_tile(0);
+            for (int k = 0; t < te; t += ts, k ^= 1) {
+                const int32_t gr = row.x;
+                const int e0 = row.y & 0xffff, len = row.y >> 16;
+                const int longest = __reduce_max_sync(kFull, len);
+                T pv[CQ], cs[CQ] = {};
+                if (gr >= 0) {
+#pragma unroll
+                    for (int i = 0; i < CQ; ++i) {
+                        pv[i] = __ldcg(a.p + static_cast<int64_t>(gr) * CP + oc + i);
+                        if (coupled) cs[i] = __ldcg(a.q + static_cast<int64_t>(gr) * CP + oc + i);
+                    }
+                }
+                tm = t + ts < te ? __ldg(a.tile_meta + t + ts) : make_int2(0, 0);
+                row = t + ts < te ? __ldg(a.tile_rows + (t + ts) * RW + gw) : make_int2(-1, 0);
                 cp_async_wait_all();
                 __syncwarp();
-                // C_fy[g] p_small (terms summed in the solve precision)
-                T cs[4] = {T(0), T(0), T(0), T(0)};
-                for (int h0 = 0; h0 < a.SGP; h0 += 4) {
-                    T c4[4];
-                    lds4<T>(srow + CP + h0, c4);
+                const unsigned char* d = slab + k * sl.buf;
+                const int32_t* tc = reinterpret_cast<const int32_t*>(d) + e0;
+                const T* tv = reinterpret_cast<const T*>(d + sl.val) + e0;
+                Acc4 acc;
+                acc_zero(acc);
+                bool staged = false;
+                for (int jb = jl; jb < longest || !staged; jb += J * U) {
+                    V4<T> xv[U];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        T xr[4];
-                        lds4<T>(s_xs + (h0 + u) * CP + 4 * q4, xr);
+                    for (int u = 0; u < U; ++u) {
+                        const int j = jb + u * J;
+                        if (j < len) v4_load_cg(a.p + static_cast<int64_t>(tc[j]) * CP + 4 * q4, xv[u]);
+                        else v4_zero(xv[u]);
+                    }
+                    if (!staged) {  // behind the first gathers: the next tile's copies
+                        stage_tile(k ^ 1);
+                        staged = true;
+                    }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) cs[i] = fma(c4[u], xr[i], cs[i]);
+                    for (int u = 0; u < U; ++u) {
+                        const int j = jb + u * J;
+                        const double vj = j < len ? static_cast<double>(tv[j]) * unscale64<T>() : 0.0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc.v[i] = fma(vj, scaled64(xv[u].v[i]), acc.v[i]);
                     }
                 }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    acc.v[i] += static_cast<double>(cs[i]);
-                    srow[4 * q4 + i] = pv.v[i];
-                }
                 __syncwarp();
-                couple_rows<T, CQ>(slab, GPW, a.SGP, lane, cacc);
-                __syncwarp();
-            }
-            if (valid) {
-                V4<T> qs;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) qs.v[i] = static_cast<T>(acc.v[i]);
-                v4_store(a.q + static_cast<int64_t>(g) * CP + 4 * q4, qs);
+                for (int o = RW * CQ; o < 32; o <<= 1)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)  // dot with the stored (rounded) value
-                    dot[i] = fma(static_cast<double>(pv.v[i]), static_cast<double>(qs.v[i]), dot[i]);
-            }
-        }
-        // this CTA's C_fy' p_f: warps added in warp order
-        if (coupled) {
-            for (int i = tid; i < npairs; i += kPcgThreads) s_cpart[i] = 0.0;
-            __syncthreads();
-            for (int w = 0; w < kPcgThreads / 32; ++w) {
-                if (warp == w) {
-                    const int nblk = (a.SGP / 4) * CQ;
+                    for (int i = 0; i < 4; ++i) acc.v[i] += __shfl_xor_sync(kFull, acc.v[i], o);
+                double qo[CQ];
+                own(acc, qo);
+                if (gr >= 0) {
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const int bk = lane + 32 * k;
-                        if (bk < nblk) {
-                            const int lq = bk / CQ, cq = bk % CQ;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int h = 4 * lq + i;
-                                if (h < a.SG) {
-#pragma unroll
-                                    for (int j = 0; j < 4; ++j)
-                                        s_cpart[h * CP + 4 * cq + j] += static_cast<double>(cacc[k][4 * i + j]);
-                                }
-                            }
-                        }
+                    for (int i = 0; i < CQ; ++i) {
+                        const T qs = static_cast<T>(qo[i] + static_cast<double>(cs[i]));
+                        a.q[static_cast<int64_t>(gr) * CP + oc + i] = qs;
+                        // dot with the stored (rounded) value
+                        dot[i] = fma(static_cast<double>(pv[i]), static_cast<double>(qs), dot[i]);
                     }
                 }
-                __syncthreads();
             }
+            cp_async_wait_all();
+            __syncwarp();
         }
-        // this CTA's pq partial: row dots (lane (gw, q4) holds columns 4 q4 + i,
-        // summed over threads in thread order), plus p_small . (C_fy' p_f
-        // partial), plus (CTA 0) p_small' C_yy p_small
-        for (int i = 0; i < 4; ++i) {
-            red[tid] = dot[i];
-            __syncthreads();
-            if (tid < CQ) {
-                double sacc = 0.0;
-                for (int t = tid; t < kPcgThreads; t += CQ) sacc += red[t];
-                s_pq[4 * tid + i] = sacc;
-            }
-            __syncthreads();
-        }
-        double cdot = 0.0;  // column c_of_t
+        // this CTA's C_fy' p_f, and its share of p'q: the row dots above plus
+        // p_small . (C_fy' p_f partial), plus p_small' C_yy p_small dealt over
+        // the CTAs by level
         if (coupled) {
-            for (int pr = tid; pr < npairs; pr += kPcgThreads) {
-                const int h = pr / CP;  // pr % CP == c_of_t
-                mypart[CP + pr] = s_cpart[pr];
-                cdot = fma(static_cast<double>(s_xs[pr]), s_cpart[pr], cdot);
-                if (b == 0) {
-                    double yq = 0.0;
-                    for (int h2 = 0; h2 < a.SG; ++h2)
-                        yq = fma(a.cyy[h * a.SG + h2], static_cast<double>(s_xs[h2 * CP + c_of_t]), yq);
-                    cdot = fma(static_cast<double>(s_xs[pr]), yq, cdot);
+            double* dump = reinterpret_cast<double*>(slab);  // [SG][CP]
+#pragma unroll
+            for (int k = 0; k < KH; ++k) {
+                const int h = sr + SR * k;
+                if (h < SG) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if constexpr (LISTS) dump[h * CP + 4 * sq + i] = cdot[k][i];
+                        else dump[h * CP + 4 * sq + i] = static_cast<double>(cpl.acc[k][i]);
+                    }
                 }
             }
+            __syncthreads();
+            for (int pr = tid; pr < npairs; pr += NT) {
+                double cp = 0.0;  // pr % CP == c_of_t
+#pragma unroll
+                for (int k = 0; k < NW; ++k) cp += reinterpret_cast<const double*>(s_slabs + k * sl.bytes)[pr];
+                mypart[CP + pr] = cp;
+                w[0] = fma(static_cast<double>(s_xs[pr]), cp, w[0]);
+            }
+            // rows b, b + NB, ... of C_yy p_small, by CP threads each from the last warp down
+            const int k = (NT - 1 - tid) / CP, h = b + k * NB;
+            if (k < kPcgOwnRows && h < SG) {
+                double yq = 0.0;
+                for (int h2 = 0; h2 < SG; ++h2)
+                    yq = fma(s_cyy[k][h2], static_cast<double>(s_xs[h2 * CP + c_of_t]), yq);
+                s_yq[k][c_of_t] = yq;
+                w[0] = fma(static_cast<double>(s_xs[h * CP + c_of_t]), yq, w[0]);
+            }
         }
-        {
-            const double cs = cta_reduce_by_column(cdot, CP, red);
-            if (tid < CP) mypart[tid] = s_pq[tid] + cs;
+        // own columns into the quads' order: lane (0, jl, q4) holds columns oc ..
+#pragma unroll
+        for (int i = 0; i < CQ; ++i) {
+#pragma unroll
+            for (int o = RW / 2; o > 0; o >>= 1) dot[i] += __shfl_xor_sync(kFull, dot[i], o);
         }
-        if (!grid_barrier(a.bar, a.status)) return;
+        publish_own(dot, w);
+        if (!meet()) return;
 
-        // ================= B: alpha, finish special rows, update =================
+        // ================= B: alpha, finish long and small rows, r -= alpha q =================
         {
-            const double pq = cta_column_sum(a.cta_part, NB, PS, 0, CP, red);
-            if (tid < CP) {
-                const int act = s_active[tid];
-                s_alpha[tid] = (act && pq > 0.0) ? s_rz[tid] / pq : 0.0;
-            }
+            double s[2];
+            col_sums(a.cta_part, NB, PS, 0, 0, 1, s);
+            if (tid < CP) s_alpha[tid] = (s_active[tid] && s[0] > 0.0) ? s_rz[tid] / s[0] : 0.0;
             __syncthreads();
         }
-        double rzp = 0.0, rrp = 0.0;  // thread's column c_of_t
-        // long rows of at most kHugeChunks chunks: a group of CP threads each
-        // (thread c sums column c of the row's chunk partials in chunk order)
+        // entry (row, c) of r = ri, whose q is finished here; its share of r'z and r'r
+        double rzp = 0.0, rrp = 0.0;  // column c_of_t
+        auto finish = [&](int64_t row, int c, T ri, T dv, double qv) {
+            const double al = s_alpha[c];
+            if (al != 0.0) {
+                ri = static_cast<T>(static_cast<double>(ri) - al * static_cast<double>(static_cast<T>(qv)));
+                a.r[row * CP + c] = ri;
+            }
+            const double rd = static_cast<double>(ri);
+            rzp = fma(rd, static_cast<double>(precond(dv, ri)), rzp);
+            rrp = fma(rd, rd, rrp);
+        };
+        // long rows of at most kHugeChunks chunks: CP lanes each, lane c sums
+        // column c of the row's chunk partials in chunk order
         {
-            const int64_t ngrp = static_cast<int64_t>(NB) * (kPcgThreads / CP);
-            const double al = s_alpha[c_of_t];
-            for (int64_t li = static_cast<int64_t>(b) * (kPcgThreads / CP) + tid / CP; li < a.nlong;
-                 li += ngrp) {
-                const int32_t c0 = __ldg(a.long_c0 + li), c1 = __ldg(a.long_c1 + li);
-                if (c1 - c0 > kHugeChunks) continue;
-                const int64_t row = __ldg(a.long_rows + li);
+            constexpr int RPW = 32 / CP;  // rows per warp
+            const int64_t step = nwarps * RPW;
+            int64_t li = wid * RPW + lane / CP;
+            int4 m = li < a.nlong ? __ldg(a.long_meta + li) : make_int4(0, 0, 0, 0);
+            for (; li < a.nlong; li += step) {
+                const int4 cur = m;
+                if (li + step < a.nlong) m = __ldg(a.long_meta + li + step);
+                if (cur.z - cur.y > kHugeChunks) continue;
+                const T ri = __ldcg(a.r + static_cast<int64_t>(cur.x) * CP + c_of_t);
+                const T dv = __ldg(a.dinv + cur.x);
                 double qv = 0.0;
-                for (int32_t k = c0; k < c1; ++k) qv += __ldcg(a.lpart + static_cast<int64_t>(k) * CP + c_of_t);
-                const int64_t i = row * CP + c_of_t;
-                double ri = static_cast<double>(__ldcg(a.r + i));
-                if (al != 0.0) {
-                    a.x[i] = static_cast<T>(static_cast<double>(__ldcg(a.x + i)) +
-                                            al * static_cast<double>(__ldcg(a.p + i)));
-                    ri -= al * static_cast<double>(static_cast<T>(qv));
-                    const T rs = static_cast<T>(ri);
-                    a.r[i] = rs;
-                    ri = static_cast<double>(rs);
+                for (int32_t k = cur.y; k < cur.z; k += 8) {
+                    double u[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        u[j] = k + j < cur.z ? __ldcg(a.lpart + static_cast<int64_t>(k + j) * CP + c_of_t) : 0.0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) qv += u[j];
                 }
-                const T zi = static_cast<T>(static_cast<double>(__ldg(a.dinv + row)) * ri);
-                a.z[i] = zi;
-                rzp = fma(ri, static_cast<double>(zi), rzp);
-                rrp = fma(ri, ri, rrp);
+                finish(cur.x, c_of_t, ri, dv, qv);
             }
         }
-        // huge long rows and small rows, round-robin over CTAs; the CTA sums the
-        // row's partials in a fixed order, thread c < CP updates column c
-        const int64_t nspecial = a.nhuge + a.SG;
-        for (int64_t sI = b; sI < nspecial; sI += NB) {
-            int64_t row;
-            double qv;
-            if (sI < a.nhuge) {
-                const int32_t li = __ldg(a.huge_li + sI);
-                row = __ldg(a.long_rows + li);
-                const int32_t c0 = __ldg(a.long_c0 + li), c1 = __ldg(a.long_c1 + li);
-                qv = cta_column_sum(a.lpart + static_cast<int64_t>(c0) * CP, c1 - c0, CP, 0, CP, red);
-            } else {
-                const int h = static_cast<int>(sI - a.nhuge);
-                row = a.Gf + h;
-                qv = cta_column_sum(a.cta_part, NB, PS, CP + h * CP, CP, red);
-                for (int h2 = 0; h2 < a.SG; ++h2)
-                    qv = fma(a.cyy[h * a.SG + h2], static_cast<double>(s_xs[h2 * CP + c_of_t]), qv);
+        // small rows b, b + NB, ... and huge long rows (dealt from the last CTA
+        // down): the CTA sums the row's partials in a fixed order, thread
+        // c < CP updates column c
+        if (coupled) {
+            for (int h = b, k = 0; h < SG; h += NB, ++k) {
+                const int64_t row = a.Gf + h;
+                const T ri = tid < CP ? __ldcg(a.r + row * CP + tid) : T(0);
+                double s[2];
+                col_sums(a.cta_part, NB, PS, CP + h * CP, 0, 1, s);
+                if (tid < CP) finish(row, tid, ri, __ldg(a.dinv + row), s[0] + s_yq[k][tid]);
+                __syncthreads();  // red_s is free again
             }
-            if (tid < CP) {
-                const int64_t i = row * CP + tid;
-                const T qs = static_cast<T>(qv);
-                const double al = s_alpha[tid];
-                double ri = static_cast<double>(__ldcg(a.r + i));
-                if (al != 0.0) {
-                    a.x[i] = static_cast<T>(static_cast<double>(__ldcg(a.x + i)) +
-                                            al * static_cast<double>(__ldcg(a.p + i)));
-                    ri -= al * static_cast<double>(qs);
-                    const T rs = static_cast<T>(ri);
-                    a.r[i] = rs;
-                    ri = static_cast<double>(rs);
-                }
-                const T zi = static_cast<T>(static_cast<double>(__ldg(a.dinv + row)) * ri);
-                a.z[i] = zi;
-                rzp = fma(ri, static_cast<double>(zi), rzp);
-                rrp = fma(ri, ri, rrp);
-            }
+        }
+        for (int64_t sI = NB - 1 - b; sI < a.nhuge; sI += NB) {
+            const int4 m = __ldg(a.long_meta + __ldg(a.huge_li + sI));
+            double s[2];
+            col_sums(a.lpart + static_cast<int64_t>(m.y) * CP, m.z - m.y, CP, 0, 0, 1, s);
+            if (tid < CP)
+                finish(m.x, tid, __ldcg(a.r + static_cast<int64_t>(m.x) * CP + tid), __ldg(a.dinv + m.x), s[0]);
+            __syncthreads();
         }
         // this CTA's short rows (contiguous range; long and small rows skipped)
-        double rz4[4] = {0.0, 0.0, 0.0, 0.0}, rr4[4] = {0.0, 0.0, 0.0, 0.0};
         {
+            double vb[2][4] = {}, wb[2];
             double al4[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) al4[i] = s_alpha[4 * tq + i];
             const bool any_al = al4[0] != 0.0 || al4[1] != 0.0 || al4[2] != 0.0 || al4[3] != 0.0;
             const int64_t e1 = min(r1, a.Gf) * CQ;
-            for (int64_t e = r0 * CQ + tid; e < e1; e += 2 * kPcgThreads) {
-                const int64_t ev[2] = {e, e + kPcgThreads};
+            for (int64_t e = r0 * CQ + tid; e < e1; e += 2 * NT) {
+                const int64_t ev[2] = {e, e + NT};
                 bool use[2];
-                V4<T> rv[2], xv[2], pv[2], qv[2];
+                V4<T> rv[2], qv[2];
                 T dv[2];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     use[k] = ev[k] < e1;
                     if (use[k]) {
                         const int64_t row = ev[k] / CQ;
-                        use[k] = __ldg(a.row_off + row + 1) - __ldg(a.row_off + row) <= kShortNnz;
-                    }
-                    if (use[k]) {
                         v4_load_cg(a.r + 4 * ev[k], rv[k]);
-                        dv[k] = __ldg(a.dinv + ev[k] / CQ);
-                        if (any_al) {
-                            v4_load_cg(a.x + 4 * ev[k], xv[k]);
-                            v4_load_cg(a.p + 4 * ev[k], pv[k]);
-                            v4_load_cg(a.q + 4 * ev[k], qv[k]);
-                        }
+                        dv[k] = __ldg(a.dinv + row);
+                        if (any_al) v4_load_cg(a.q + 4 * ev[k], qv[k]);
+                        use[k] = __ldg(a.row_off + row + 1) - __ldg(a.row_off + row) <= kShortNnz;
                     }
                 }
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     if (!use[k]) continue;
-                    V4<T> zv;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         double ri = static_cast<double>(rv[k].v[i]);
                         if (al4[i] != 0.0) {
-                            xv[k].v[i] = static_cast<T>(static_cast<double>(xv[k].v[i]) +
-                                                        al4[i] * static_cast<double>(pv[k].v[i]));
                             ri -= al4[i] * static_cast<double>(qv[k].v[i]);
                             rv[k].v[i] = static_cast<T>(ri);
                             ri = static_cast<double>(rv[k].v[i]);
                         }
-                        zv.v[i] = static_cast<T>(static_cast<double>(dv[k]) * ri);
-                        rz4[i] = fma(ri, static_cast<double>(zv.v[i]), rz4[i]);
-                        rr4[i] = fma(ri, ri, rr4[i]);
+                        const T zi = precond(dv[k], rv[k].v[i]);
+                        vb[0][i] = fma(ri, static_cast<double>(zi), vb[0][i]);
+                        vb[1][i] = fma(ri, ri, vb[1][i]);
                     }
-                    if (any_al) {
-                        v4_store(a.x + 4 * ev[k], xv[k]);
-                        v4_store(a.r + 4 * ev[k], rv[k]);
-                    }
-                    v4_store(a.z + 4 * ev[k], zv);
+                    if (any_al) v4_store(a.r + 4 * ev[k], rv[k]);
                 }
             }
+            wb[0] = rzp;
+            wb[1] = rrp;
+            publish(vb, wb, off_rr, 2);
         }
-        rzp = cta_reduce_by_column(rzp, CP, red);
-        rrp = cta_reduce_by_column(rrp, CP, red);
-        cta_reduce_quads(rz4, CQ, red, s_q1);
-        cta_reduce_quads(rr4, CQ, red, s_q2);
-        if (tid < CP) {
-            mypart[CP * (1 + a.SG) + tid] = rzp + s_q1[tid];
-            mypart[CP * (2 + a.SG) + tid] = rrp + s_q2[tid];
-        }
-        if (!grid_barrier(a.bar, a.status)) return;
+        if (!meet()) return;
 
-        // ================= C: beta, masks, directions =================
+        // ================= C: beta, masks; x += alpha p, p = z + beta p =================
         {
-            const double rz = cta_column_sum(a.cta_part, NB, PS, CP * (1 + a.SG), CP, red);
-            const double rr = cta_column_sum(a.cta_part, NB, PS, CP * (2 + a.SG), CP, red);
-            if (tid < CP) {
-                s_beta[tid] = 0.0;
-                if (s_active[tid]) {
-                    const double old = s_rz[tid];
-                    s_beta[tid] = old > 0.0 ? rz / old : 0.0;
-                    s_rz[tid] = rz;
-                    s_iters[tid] += 1;
-                    if (!(rr > a.thr[tid]) || !(rz > 0.0)) s_active[tid] = 0;
+            double s[2];
+            col_sums(a.cta_part, NB, PS, off_rr[0], off_rr[1], 2, s);
+            if (warp == 0) {
+                int act = 0;
+                if (lane < CP) {
+                    s_beta[lane] = 0.0;
+                    if (s_active[lane]) {
+                        const double old = s_rz[lane];
+                        s_beta[lane] = old > 0.0 ? s[0] / old : 0.0;
+                        s_rz[lane] = s[0];
+                        s_iters[lane] += 1;
+                        act = ((s[1] > a.thr[lane]) && (s[0] > 0.0)) ? 1 : 0;
+                        s_active[lane] = act;
+                    }
                 }
-            }
-            __syncthreads();
-            if (tid == 0) {
-                int any = 0;
-                for (int c = 0; c < CP; ++c) any |= s_active[c];
-                s_any = any;
+                const int any = __any_sync(kFull, act);
+                if (lane == 0) s_any = any;
             }
             __syncthreads();
         }
         {
             // a column that just stopped keeps p (its x and r no longer move)
             bool act4[4];
-            double be4[4];
+            double be4[4], al4[4];
+            bool work = false;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 act4[i] = s_active[4 * tq + i] != 0;
                 be4[i] = s_beta[4 * tq + i];
+                al4[i] = s_alpha[4 * tq + i];
+                work = work || act4[i] || al4[i] != 0.0;
             }
-            if (act4[0] || act4[1] || act4[2] || act4[3]) {
+            if (work) {
                 const int64_t e1 = r1 * CQ;
-                for (int64_t e = r0 * CQ + tid; e < e1; e += 2 * kPcgThreads) {
-                    const int64_t eb = e + kPcgThreads;
+                for (int64_t e = r0 * CQ + tid; e < e1; e += 2 * NT) {
+                    const int64_t eb = e + NT;
                     const bool vb = eb < e1;
-                    V4<T> zv[2], pv[2];
-                    v4_load_cg(a.z + 4 * e, zv[0]);
+                    V4<T> rv[2], pv[2], xv[2];
+                    T dv[2];
+                    v4_load_cg(a.r + 4 * e, rv[0]);
                     v4_load_cg(a.p + 4 * e, pv[0]);
+                    v4_load_cg(a.x + 4 * e, xv[0]);
+                    dv[0] = __ldg(a.dinv + e / CQ);
                     if (vb) {
-                        v4_load_cg(a.z + 4 * eb, zv[1]);
+                        v4_load_cg(a.r + 4 * eb, rv[1]);
                         v4_load_cg(a.p + 4 * eb, pv[1]);
+                        v4_load_cg(a.x + 4 * eb, xv[1]);
+                        dv[1] = __ldg(a.dinv + eb / CQ);
                     }
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
                         if (k == 1 && !vb) break;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (act4[i])
-                                pv[k].v[i] = static_cast<T>(static_cast<double>(zv[k].v[i]) +
-                                                            be4[i] * static_cast<double>(pv[k].v[i]));
+                        for (int i = 0; i < 4; ++i) {
+                            const double pi = static_cast<double>(pv[k].v[i]);
+                            if (al4[i] != 0.0)
+                                xv[k].v[i] = static_cast<T>(static_cast<double>(xv[k].v[i]) + al4[i] * pi);
+                            if (act4[i]) {
+                                const T zi = precond(dv[k], rv[k].v[i]);
+                                pv[k].v[i] = static_cast<T>(static_cast<double>(zi) + be4[i] * pi);
+                            }
+                        }
+                        v4_store(a.x + 4 * (k ? eb : e), xv[k]);
                         v4_store(a.p + 4 * (k ? eb : e), pv[k]);
                     }
                 }
             }
         }
         ++it;
-        if (!grid_barrier(a.bar, a.status)) return;
+        if (!CLUSTER) __syncthreads();  // every store of the CTA precedes the arrival
+        if (!meet()) return;
     }
     if (b == 0 && tid < CP) {
         a.rz_out[tid] = s_rz[tid];
@@ -797,9 +968,9 @@ pcg_persistent_kernel(const PcgArgs<T> a) {
 
 namespace b200fe {
 
-// Work lists of pcg_persistent_kernel over the CSR rows of S_ff: per row g,
-// is_short[g] (<= kShortNnz nonzeros), is_long[g] and its number of
-// kLongChunk chunks.
+// Work lists of pcg_persistent_kernel over the CSR rows of S_ff.  Per row g:
+// is_short[g] (<= kShortNnz nonzeros), is_long[g], its number of kLongChunk
+// chunks, is_huge[g].
 __global__ void pcg_lists_count_kernel(const int32_t* __restrict__ row_off, int32_t G,
                                        int32_t* __restrict__ is_short, int32_t* __restrict__ is_long,
                                        int32_t* __restrict__ nchunks, int32_t* __restrict__ is_huge) {
@@ -815,32 +986,90 @@ __global__ void pcg_lists_count_kernel(const int32_t* __restrict__ row_off, int3
     }
 }
 
-// Fills the lists from the exclusive scans of the three counts.
+// Fills the lists from the exclusive scans of the counts (short rows ascending).
 __global__ void pcg_lists_fill_kernel(const int32_t* __restrict__ row_off, int32_t G,
                                       const int32_t* __restrict__ is_short,
                                       const int32_t* __restrict__ short_idx,
                                       const int32_t* __restrict__ long_idx,
-                                      const int32_t* __restrict__ chunk_off,
-                                      int4* __restrict__ short_meta, int32_t* __restrict__ long_rows,
-                                      int32_t* __restrict__ long_c0, int32_t* __restrict__ long_c1,
-                                      int4* __restrict__ lchunk_meta,
+                                      const int32_t* __restrict__ chunk_off, int32_t* __restrict__ short_row,
+                                      int4* __restrict__ long_meta, int4* __restrict__ lchunk_meta,
                                       const int32_t* __restrict__ huge_idx, int32_t* __restrict__ huge_li) {
     for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < G;
          g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         if (is_short[g]) {
-            short_meta[short_idx[g]] = make_int4(static_cast<int32_t>(g), row_off[g], row_off[g + 1], 0);
+            short_row[short_idx[g]] = static_cast<int32_t>(g);
             continue;
         }
         const int32_t li = long_idx[g];
         const int32_t c0 = chunk_off[g], c1 = chunk_off[g + 1];
-        long_rows[li] = static_cast<int32_t>(g);
-        long_c0[li] = c0;
-        long_c1[li] = c1;
+        long_meta[li] = make_int4(static_cast<int32_t>(g), c0, c1, 0);
         if (c1 - c0 > kHugeChunks) huge_li[huge_idx[g]] = li;
         const int32_t b = row_off[g], e = row_off[g + 1];
         for (int32_t c = c0; c < c1; ++c) {
             const int32_t cb = b + (c - c0) * kLongChunk;
             lchunk_meta[c] = make_int4(static_cast<int32_t>(g), cb, min(e, cb + kLongChunk), c == c0 ? 1 : 0);
+        }
+    }
+}
+
+// PcgTiles: tiles of kPcgRowsPerWarp short rows of about equal length, their
+// nonzeros one row after the other, each tile from a multiple of four entries
+// on (16-byte copies).  Rows are sorted by falling length within their
+// summation list (lists > 0: steps of sr rows dealt to the lists) or all
+// together; padded with row -1 to npad = a multiple of sr.
+__global__ void pcg_tile_key_kernel(const int32_t* __restrict__ row_off, const int32_t* __restrict__ srow,
+                                    int64_t nshort, int64_t npad, int sr, int lists, int32_t* __restrict__ key,
+                                    int32_t* __restrict__ row) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < npad;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int32_t g = i < nshort ? srow[i] : -1;
+        const int32_t len = g >= 0 ? row_off[g + 1] - row_off[g] : 0;
+        const int32_t list = lists > 0 ? static_cast<int32_t>((i / sr) % lists) : 0;
+        key[i] = list * (kShortNnz + 2) + (g >= 0 ? kShortNnz - len : kShortNnz + 1);
+        row[i] = g;
+    }
+}
+// len[t]: entries / 4 of tile t, rounded up
+__global__ void pcg_tile_len_kernel(const int32_t* __restrict__ row_off, const int32_t* __restrict__ srow,
+                                    int64_t ntiles, int32_t* __restrict__ len) {
+    for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t <= ntiles;
+         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        int32_t n = 0;
+        for (int64_t k = t * kPcgRowsPerWarp; t < ntiles && k < (t + 1) * kPcgRowsPerWarp; ++k)
+            if (srow[k] >= 0) n += row_off[srow[k] + 1] - row_off[srow[k]];
+        len[t] = (n + 3) / 4;
+    }
+}
+// One warp per tile: lanes take (row, every fourth nonzero).
+__global__ void pcg_tile_fill_kernel(const int32_t* __restrict__ row_off, const int32_t* __restrict__ col,
+                                     const double* __restrict__ val, const int32_t* __restrict__ srow,
+                                     int64_t ntiles, const int32_t* __restrict__ off,
+                                     int2* __restrict__ meta, int2* __restrict__ rows,
+                                     int32_t* __restrict__ tcol, double* __restrict__ tval64,
+                                     float* __restrict__ tval32) {
+    constexpr int RW = kPcgRowsPerWarp;
+    const int lane = threadIdx.x & 31, r = lane % RW;
+    const int64_t nw = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+    for (int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; t < ntiles; t += nw) {
+        const int64_t k = t * RW + r;
+        const int32_t g = srow[k];
+        const int32_t b = g >= 0 ? row_off[g] : 0;
+        const int32_t n = g >= 0 ? row_off[g + 1] - b : 0;
+        int32_t e0 = 0, total = 0;
+        for (int i = 0; i < RW; ++i) {
+            const int32_t ni = __shfl_sync(0xffffffffu, n, i);
+            if (i < r) e0 += ni;
+            total += ni;
+        }
+        const int32_t o = off[t];
+        if (lane < RW) rows[k] = make_int2(g, e0 | (n << 16));
+        if (lane == 0) meta[t] = make_int2(o, total);
+        const int64_t d = 4 * static_cast<int64_t>(o) + e0;
+        for (int j = lane / RW; j < n; j += 32 / RW) {
+            const double x = val[b + j];
+            tcol[d + j] = col[b + j];
+            tval64[d + j] = x;
+            tval32[d + j] = static_cast<float>(x);
         }
     }
 }
