@@ -96,6 +96,36 @@ __device__ __forceinline__ void row_store(double* p, const double (&v)[VL]) {
     }
 }
 
+// acc += sum over a in [a0, a1) of c[a] row idx[a] of x, in order; the ids and
+// rows of a batch are loaded before its sums, so that a group has U rows in
+// flight (one row at a time a firm chunk is a chain of 64 dependent reads: 198
+// against 158 us with 1M matches and 64 lanes)
+template <int LW, int U>
+__device__ __forceinline__ void row_sums(const int32_t* __restrict__ idx, const double* __restrict__ c,
+                                         const double* __restrict__ x, int64_t a0, int64_t a1, int tg,
+                                         double (&acc)[LaneGeom<LW>::VL]) {
+    constexpr int VL = LaneGeom<LW>::VL;
+    for (int64_t a = a0; a < a1; a += U) {
+        int64_t r[U];
+        double ca[U], v[U][VL];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = a + u < a1;
+            r[u] = in ? __ldg(idx + a + u) : -1;
+            ca[u] = in ? __ldg(c + a + u) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (r[u] >= 0) row_load<VL>(x + r[u] * LW + tg * VL, v[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (r[u] < 0) break;
+#pragma unroll
+            for (int k = 0; k < VL; ++k) acc[k] = fma(ca[u], v[u][k], acc[k]);
+        }
+    }
+}
+
 // t[w] = Dw^{-1} sum_{matches a of w} c_a p[f_a]   (matches in worker order)
 template <int LW>
 __global__ void __launch_bounds__(kKssThreads)
@@ -112,15 +142,7 @@ kss_worker_kernel(int N, const int64_t* __restrict__ w_ptr, const int32_t* __res
         double acc[VL];
 #pragma unroll
         for (int v = 0; v < VL; ++v) acc[v] = 0.0;
-        const int64_t a1 = __ldg(w_ptr + w + 1);
-        for (int64_t a = __ldg(w_ptr + w); a < a1; ++a) {
-            const int64_t f = __ldg(m_f + a);
-            const double c = __ldg(m_c + a);
-            double pv[VL];
-            row_load<VL>(p + f * LW + tg * VL, pv);
-#pragma unroll
-            for (int v = 0; v < VL; ++v) acc[v] = fma(c, pv[v], acc[v]);
-        }
+        row_sums<LW, 1>(m_f, m_c, p, __ldg(w_ptr + w), __ldg(w_ptr + w + 1), tg, acc);  // 2-3 matches: batches only cost
         const double iw = __ldg(inv_dw + w);
 #pragma unroll
         for (int v = 0; v < VL; ++v) acc[v] *= iw;
@@ -148,15 +170,7 @@ kss_firm_kernel(int64_t nchunks, const int64_t* __restrict__ cbeg, const int32_t
         double acc[VL];
 #pragma unroll
         for (int v = 0; v < VL; ++v) acc[v] = 0.0;
-        const int64_t a1 = __ldg(cbeg + k + 1);
-        for (int64_t a = __ldg(cbeg + k); a < a1; ++a) {
-            const int64_t w = __ldg(mw_f + a);
-            const double c = __ldg(mc_f + a);
-            double tv[VL];
-            row_load<VL>(t + w * LW + tg * VL, tv);
-#pragma unroll
-            for (int v = 0; v < VL; ++v) acc[v] = fma(c, tv[v], acc[v]);
-        }
+        row_sums<LW, 8>(mw_f, mc_f, t, __ldg(cbeg + k), __ldg(cbeg + k + 1), tg, acc);
         const int32_t slot = __ldg(cslot + k);
         if (slot >= 0) {
             row_store<VL>(part + static_cast<int64_t>(slot) * LW + tg * VL, acc);
@@ -172,6 +186,10 @@ kss_firm_kernel(int64_t nchunks, const int64_t* __restrict__ cbeg, const int32_t
     }
 }
 
+// One CTA per firm of several chunks: its thread groups take every NG-th chunk
+// partial, the groups meet in a fixed tree (a Zipf giant owns thousands of
+// partials: one group adding them one L2 read at a time took 285 us of a 720 us
+// step with 1M matches and 64 lanes, a CTA takes 39).
 template <int LW>
 __global__ void __launch_bounds__(kKssThreads)
 kss_firm_combine_kernel(int64_t nmulti, const int32_t* __restrict__ mfirm,
@@ -180,29 +198,48 @@ kss_firm_combine_kernel(int64_t nmulti, const int32_t* __restrict__ mfirm,
                         const double* __restrict__ p, double* __restrict__ Ap, int ground,
                         const KssScalars* __restrict__ sc) {
     if (sc->nactive == 0) return;
-    constexpr int TG = LaneGeom<LW>::TG, VL = LaneGeom<LW>::VL;
-    const int64_t g0 = (static_cast<int64_t>(blockIdx.x) * kKssThreads + threadIdx.x) / TG;
-    const int tg = threadIdx.x % TG;
-    const int64_t ng = static_cast<int64_t>(gridDim.x) * (kKssThreads / TG);
-    for (int64_t i = g0; i < nmulti; i += ng) {
+    constexpr int TG = LaneGeom<LW>::TG, VL = LaneGeom<LW>::VL, NG = kKssThreads / TG, U = 4;
+    __shared__ double red[kKssThreads * VL];
+    const int tg = threadIdx.x % TG, grp = threadIdx.x / TG;
+    for (int64_t i = blockIdx.x; i < nmulti; i += gridDim.x) {
         const int64_t f = __ldg(mfirm + i);
         const int64_t s0 = __ldg(mslot0 + i);
         const int ns = __ldg(mnslot + i);
         double acc[VL];
 #pragma unroll
         for (int v = 0; v < VL; ++v) acc[v] = 0.0;
-        for (int s = 0; s < ns; ++s) {
-            double pv[VL];
-            row_load<VL>(part + (s0 + s) * LW + tg * VL, pv);
+        for (int s = grp; s < ns; s += U * NG) {
+            double pv[U][VL];
 #pragma unroll
-            for (int v = 0; v < VL; ++v) acc[v] += pv[v];
+            for (int u = 0; u < U; ++u)
+                if (s + u * NG < ns) row_load<VL>(part + (s0 + s + u * NG) * LW + tg * VL, pv[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VL; ++v)
+                    if (s + u * NG < ns) acc[v] += pv[u][v];
         }
-        double pv[VL], out[VL];
-        row_load<VL>(p + f * LW + tg * VL, pv);
-        const double df = __ldg(Df + f);
 #pragma unroll
-        for (int v = 0; v < VL; ++v) out[v] = (f == ground) ? 0.0 : df * pv[v] - acc[v];
-        row_store<VL>(Ap + f * LW + tg * VL, out);
+        for (int v = 0; v < VL; ++v) red[v * kKssThreads + threadIdx.x] = acc[v];
+        __syncthreads();
+        for (int h = NG / 2; h > 0; h >>= 1) {
+            if (grp < h) {
+#pragma unroll
+                for (int v = 0; v < VL; ++v)
+                    red[v * kKssThreads + threadIdx.x] += red[v * kKssThreads + threadIdx.x + h * TG];
+            }
+            __syncthreads();
+        }
+        if (grp == 0) {
+            double pv[VL], out[VL];
+            row_load<VL>(p + f * LW + tg * VL, pv);
+            const double df = __ldg(Df + f);
+#pragma unroll
+            for (int v = 0; v < VL; ++v)
+                out[v] = (f == ground) ? 0.0 : df * pv[v] - red[v * kKssThreads + threadIdx.x];
+            row_store<VL>(Ap + f * LW + tg * VL, out);
+        }
+        __syncthreads();
     }
 }
 
@@ -281,11 +318,23 @@ __device__ __forceinline__ void kss_reduce_tail(double s0, double s1, double* __
     __syncthreads();
     if (!last) return;
     __threadfence();
+    // the whole CTA adds the partials: slice j of the CTAs per group of LW threads
+    {
+        const int l = tid % LW, j = tid / LW;
+        double d[2] = {0.0, 0.0};
+#pragma unroll 4
+        for (unsigned b = j; b < gridDim.x; b += kKssThreads / LW)
+#pragma unroll
+            for (int k = 0; k < NDOT; ++k) d[k] += __ldcg(part + (static_cast<int64_t>(b) * NDOT + k) * LW + l);
+#pragma unroll
+        for (int k = 0; k < NDOT; ++k) red[k][tid] = d[k];
+    }
+    __syncthreads();
     if (tid < LW) {
         double d[2] = {0.0, 0.0};
-        for (unsigned b = 0; b < gridDim.x; ++b)
 #pragma unroll
-            for (int k = 0; k < NDOT; ++k) d[k] += __ldcg(part + (static_cast<int64_t>(b) * NDOT + k) * LW + tid);
+        for (int k = 0; k < NDOT; ++k)
+            for (int j = tid; j < kKssThreads; j += LW) d[k] += red[k][j];
         kss_action(sc, action, tid, d[0], d[1]);
     }
     __syncthreads();
@@ -802,7 +851,7 @@ int run_solve(b200fe_kss* kss, int nb) {
     const int flat_grid = grid_for(kss, J * LW, 4);
     const int worker_grid = grid_for(kss, static_cast<int64_t>(kss->N) * TG, 8);
     const int firm_grid = grid_for(kss, kss->nchunks * TG, 8);
-    const int multi_grid = grid_for(kss, kss->nmulti * TG, 8);
+    const int multi_grid = grid_for(kss, kss->nmulti * kKssThreads, 8);
     // r = grounded rhs, x = 0; ||r||^2 -> tol2, active lanes
     kss_pack_in_kernel<<<flat_grid, kKssThreads, 0, s>>>(J, LW, nb, kss->ground, kss->stage, kss->r);
     K_TRY(cudaMemsetAsync(kss->x, 0, sizeof(double) * J * LW, s));
@@ -952,7 +1001,7 @@ int jla_block(b200fe_kss* kss, JlaState& js, int d0, int B) {
         kss->nchunks, kss->cbeg, kss->cfirm, kss->cslot, kss->mw_f, kss->mc_f, js.xw, kss->Df, kss->z, kss->Ap,
         kss->slot_part, kss->ground, kss->sc_one);
     if (kss->nmulti > 0)
-        kss_firm_combine_kernel<LW><<<grid_for(kss, kss->nmulti * TG, 8), kKssThreads, 0, s>>>(
+        kss_firm_combine_kernel<LW><<<grid_for(kss, kss->nmulti * kKssThreads, 8), kKssThreads, 0, s>>>(
             kss->nmulti, kss->mfirm, kss->mslot0, kss->mnslot, kss->slot_part, kss->Df, kss->z, kss->Ap,
             kss->ground, kss->sc_one);
     jla_rhs_kernel<<<grid(J * nl), T, 0, s>>>(J, LW, nl, kss->ground, js.tf, kss->Ap, kss->stage);
@@ -1070,7 +1119,7 @@ int b200fe_kss_create(int n_workers, int n_firms, const int32_t* m_w, const int3
     kss->nchunks = static_cast<int64_t>(cfirm.size());
     kss->nmulti = static_cast<int64_t>(mfirm.size());
     kss->nslots = slots;
-    kss->dot_grid = kss->sms * 2;
+    kss->dot_grid = kss->sms * 4;
     int rc = B200FE_OK;
     if ((rc = upload(kss, &kss->w_ptr, w_ptr, static_cast<size_t>(n_workers) + 1)) ||
         (rc = upload(kss, &kss->m_f, m_f, M)) || (rc = upload(kss, &kss->m_c, m_c, M)) ||
