@@ -130,6 +130,38 @@ slope_moments_kernel(const SlopeDim d, const double* __restrict__ w, double* __r
     }
 }
 
+// The five moments of group g from its chunks' moments.  Groups of up to 8
+// chunks: the calling thread alone, in chunk order.  The larger ones of the
+// warp's groups are taken one after the other by all its lanes (a Zipf giant
+// has thousands of chunks).  Every lane of the warp calls this together.
+__device__ __forceinline__ void group_moments(const SlopeDim& d, const double* __restrict__ cm, int64_t g, bool valid,
+                                              double (&m)[5]) {
+    const int lane = threadIdx.x & 31;
+    const int32_t b = valid ? d.grp_ch[g] : 0, e = valid ? d.grp_ch[g + 1] : 0;
+#pragma unroll
+    for (int u = 0; u < 5; ++u) m[u] = 0.0;
+    if (e - b <= 8)
+        for (int32_t j = b; j < e; ++j)
+#pragma unroll
+            for (int u = 0; u < 5; ++u) m[u] += cm[static_cast<int64_t>(j) * 5 + u];
+    unsigned big = __ballot_sync(0xffffffffu, e - b > 8);
+    while (big) {
+        const int src = __ffs(big) - 1;
+        big &= big - 1;
+        const int32_t gb = __shfl_sync(0xffffffffu, b, src), ge = __shfl_sync(0xffffffffu, e, src);
+        double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int32_t j = gb + lane; j < ge; j += 32)
+#pragma unroll
+            for (int u = 0; u < 5; ++u) t[u] += cm[static_cast<int64_t>(j) * 5 + u];
+#pragma unroll
+        for (int u = 0; u < 5; ++u) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t[u] += __shfl_xor_sync(0xffffffffu, t[u], o);
+            if (lane == src) m[u] = t[u];
+        }
+    }
+}
+
 // Per group: combine the chunk moments in chunk order, form the block inverse
 // and the group's share of ||D'W||_F^2 (sum of the squared multipliers w and
 // w z of its basis columns); CTA partials of the latter in part_op[block].
@@ -138,12 +170,12 @@ slope_block_inverse_kernel(const SlopeDim d, const double* __restrict__ cm,
                            double* __restrict__ minv, double* __restrict__ part_op) {
     __shared__ double red[kSlopeThreads];
     double op = 0.0;
-    for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < d.G;
-         g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int32_t j = d.grp_ch[g]; j < d.grp_ch[g + 1]; ++j)
-#pragma unroll
-            for (int u = 0; u < 5; ++u) m[u] += cm[static_cast<int64_t>(j) * 5 + u];
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < d.G;
+         base += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t g = base + threadIdx.x;
+        double m[5];
+        group_moments(d, cm, g, g < d.G, m);
+        if (g >= d.G) continue;
         const double W = m[0], Z = m[1], ZZ = m[2];
         double m00 = 0.0, m01 = 0.0, m11 = 0.0;
         if (d.has_a && d.has_b) {
@@ -307,17 +339,33 @@ slope_gather_kernel(const SlopeGatherArgs a) {
     column_reduce(red, acc, C, a.RB, a.part + static_cast<int64_t>(blockIdx.x) * C);
 }
 
+// Sum over b of part[b * C + c] by one warp: lanes take every 32nd partial,
+// four loads in flight, then a fixed shuffle tree (a thread per column adding
+// 1,184 partials one read at a time took 140 us).
+__device__ __forceinline__ double warp_column_sum(const double* __restrict__ part, int nparts, int C, int c) {
+    const int lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int b = lane; b < nparts; b += 128) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = b + 32 * u < nparts ? part[static_cast<int64_t>(b + 32 * u) * C + c] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s += v[u];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+constexpr int kSlopeScalarThreads = 1024;  // one CTA, a warp per column
+
 // alpha_c = gamma_c / (q' W q)_c for the columns still iterating; the dots
-// come as CTA partials of one or two kernels, summed in order
-__global__ void slope_alpha_kernel(const double* __restrict__ part, int nparts,
-                                   const double* __restrict__ part2, int nparts2, int C,
-                                   const double* __restrict__ gamma, const int* __restrict__ active,
-                                   double* __restrict__ alpha) {
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        double dl = 0.0;
-        for (int b = 0; b < nparts; ++b) dl += part[static_cast<int64_t>(b) * C + c];
-        for (int b = 0; b < nparts2; ++b) dl += part2[static_cast<int64_t>(b) * C + c];
-        alpha[c] = (active[c] && dl > 0.0) ? gamma[c] / dl : 0.0;
+// come as CTA partials of one or two kernels, summed in a fixed order
+__global__ void __launch_bounds__(kSlopeScalarThreads)
+slope_alpha_kernel(const double* __restrict__ part, int nparts, const double* __restrict__ part2, int nparts2, int C,
+                   const double* __restrict__ gamma, const int* __restrict__ active, double* __restrict__ alpha) {
+    for (int c = threadIdx.x >> 5; c < C; c += kSlopeScalarThreads / 32) {
+        const double dl = warp_column_sum(part, nparts, C, c) + warp_column_sum(part2, nparts2, C, c);
+        if ((threadIdx.x & 31) == 0) alpha[c] = (active[c] && dl > 0.0) ? gamma[c] / dl : 0.0;
     }
 }
 
@@ -472,29 +520,29 @@ struct SlopeBetaArgs {
 };
 
 // One CTA: gamma_new = sum over dims and CTAs (fixed order), beta, stop test.
-__global__ void slope_beta_kernel(const SlopeBetaArgs a) {
+__global__ void __launch_bounds__(kSlopeScalarThreads) slope_beta_kernel(const SlopeBetaArgs a) {
     int any = 0;
-    for (int c = threadIdx.x; c < a.C; c += blockDim.x) {
+    for (int c = threadIdx.x >> 5; c < a.C; c += kSlopeScalarThreads / 32) {
         double g = 0.0, nu = 0.0;
-        for (int d = 0; d < a.nd; ++d)
-            for (int b = 0; b < a.grid[d]; ++b) {
-                const int64_t o = (d * a.stride + b) * a.C + c;
-                g += a.part_g[o];
-                nu += a.part_n[o];
-            }
-        a.nu[c] = nu;
-        if (a.init) {
-            a.gamma[c] = g;
-            a.beta[c] = 0.0;
-            a.active[c] = g > a.thr[c] ? 1 : 0;
-        } else if (a.active[c]) {
-            a.beta[c] = a.gamma[c] > 0.0 ? g / a.gamma[c] : 0.0;
-            a.gamma[c] = g;
-            if (!(g > a.thr[c])) a.active[c] = 0;
-        } else {
-            a.beta[c] = 0.0;
+        for (int d = 0; d < a.nd; ++d) {
+            g += warp_column_sum(a.part_g + d * a.stride * a.C, a.grid[d], a.C, c);
+            nu += warp_column_sum(a.part_n + d * a.stride * a.C, a.grid[d], a.C, c);
         }
-        any |= a.active[c];
+        if ((threadIdx.x & 31) == 0) {
+            a.nu[c] = nu;
+            if (a.init) {
+                a.gamma[c] = g;
+                a.beta[c] = 0.0;
+                a.active[c] = g > a.thr[c] ? 1 : 0;
+            } else if (a.active[c]) {
+                a.beta[c] = a.gamma[c] > 0.0 ? g / a.gamma[c] : 0.0;
+                a.gamma[c] = g;
+                if (!(g > a.thr[c])) a.active[c] = 0;
+            } else {
+                a.beta[c] = 0.0;
+            }
+            any |= a.active[c];
+        }
     }
     any = __syncthreads_or(any);
     if (threadIdx.x == 0) *a.done = any ? 0 : 1;
@@ -692,12 +740,12 @@ schur_block_inverse_kernel(const SlopeDim d, const double* __restrict__ cm,
                            double* __restrict__ part_op) {
     __shared__ double red[kSlopeThreads];
     double op = 0.0;
-    for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < d.G;
-         g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int32_t j = d.grp_ch[g]; j < d.grp_ch[g + 1]; ++j)
-#pragma unroll
-            for (int u = 0; u < 5; ++u) m[u] += cm[static_cast<int64_t>(j) * 5 + u];
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < d.G;
+         base += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t g = base + threadIdx.x;
+        double m[5];
+        group_moments(d, cm, g, g < d.G, m);
+        if (g >= d.G) continue;
         const double W = m[0], Z = m[1], ZZ = m[2];
         // csum: per group the sums of the three pair planes (segmented reduce)
         const double s11 = W - csum[g], s12 = Z - csum[d.G + g], s22 = ZZ - csum[2 * static_cast<int64_t>(d.G) + g];

@@ -509,7 +509,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         double vb = 0.0;
         for (int d = 0; d < ndt; ++d) vb += 24.0 * dims[d].G * dims[d].nb * C;
         ProfScope ps(ctx, B200FE_PROF_VECTOR, vb);
-        slope_beta_kernel<<<1, T, 0, s>>>(b);
+        slope_beta_kernel<<<1, kSlopeScalarThreads, 0, s>>>(b);
         B_LAUNCHED();
         for (int d = 0; d < ndt; ++d) {
             if (schur && d == p) continue;
@@ -629,7 +629,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             }
             {
                 ProfScope ps(ctx, B200FE_PROF_VECTOR, 0.0);
-                slope_alpha_kernel<<<1, T, 0, s>>>(pq, schur ? gS : gG, pq2, schur ? gF : 0, C,
+                slope_alpha_kernel<<<1, kSlopeScalarThreads, 0, s>>>(pq, schur ? gS : gG, pq2, schur ? gF : 0, C,
                                                    gamma, active, alpha);
                 B_LAUNCHED();
             }
