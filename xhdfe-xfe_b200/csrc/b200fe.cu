@@ -3232,24 +3232,30 @@ int drop_singletons_impl(b200fe_context* ctx, int nd, const int32_t* const* d_id
         a.ids[d] = d_ids[d];
         B_CHECK(get_buf(ctx, "prep_cnt" + std::to_string(d), G[d], &a.counts[d]));
     }
-    unsigned long long* dcount;
+    int32_t *dcount, *list;
     B_CHECK(get_buf(ctx, "prep_dropped", 1, &dcount));
+    B_CHECK(get_buf(ctx, "prep_list", n, &list));
     B_TRY(cudaMemsetAsync(d_keep, 1, n, s));
+    for (int d = 0; d < nd; ++d) {
+        B_TRY(cudaMemsetAsync(a.counts[d], 0, sizeof(int32_t) * G[d], s));
+        if (G[d] <= kSingletonSharedGroups)
+            singleton_count_kernel<true><<<grid_for(ctx, n, 256), 256, 0, s>>>(a.ids[d], n, G[d], a.counts[d]);
+        else
+            singleton_count_kernel<false><<<grid_for(ctx, n, 256), 256, 0, s>>>(a.ids[d], n, G[d], a.counts[d]);
+        B_LAUNCHED();
+    }
     int64_t total = 0;
     int r = 0;
     for (; r < std::max(1, max_iter); ++r) {
-        for (int d = 0; d < nd; ++d)
-            B_TRY(cudaMemsetAsync(a.counts[d], 0, sizeof(int32_t) * G[d], s));
-        B_TRY(cudaMemsetAsync(dcount, 0, sizeof(unsigned long long), s));
-        singleton_count_kernel<<<grid_for(ctx, n, 256), 256, 0, s>>>(a, n, d_keep);
+        B_TRY(cudaMemsetAsync(dcount, 0, sizeof(int32_t), s));
+        singleton_drop_kernel<<<grid_for(ctx, n, 256), 256, 0, s>>>(a, n, d_keep, list, dcount);
         B_LAUNCHED();
-        singleton_drop_kernel<<<grid_for(ctx, n, 256), 256, 0, s>>>(a, n, d_keep, dcount);
-        B_LAUNCHED();
-        unsigned long long h = 0;
-        B_TRY(cudaMemcpyAsync(&h, dcount, sizeof(h), cudaMemcpyDeviceToHost, s));
-        B_TRY(cudaStreamSynchronize(s));
+        int h = 0;
+        B_CHECK(sync_read_int(ctx, dcount, 1, &h));
         if (h == 0) break;
-        total += static_cast<int64_t>(h);
+        total += h;
+        singleton_uncount_kernel<<<grid_for(ctx, h, 256), 256, 0, s>>>(a, list, dcount);
+        B_LAUNCHED();
     }
     if (dropped) *dropped = total;
     if (rounds) *rounds = r;
@@ -3335,7 +3341,7 @@ int component_stats_impl(b200fe_context* ctx, const int32_t* d_fe1, const int32_
         }
         ++ctx->lib_calls;
     }
-    segment_offsets_kernel<<<grid_for(ctx, n + 1, 256), 256, 0, s>>>(slabel, n, static_cast<int32_t>(N), off);
+    cc_offsets_kernel<<<grid_for(ctx, N + 1, 256), 256, 0, s>>>(slabel, n, static_cast<int32_t>(N), off);
     B_LAUNCHED();
     B_TRY(cudaMemsetAsync(flags + 2, 0, 2 * sizeof(int), s));
     cc_count_kernel<<<grid_for(ctx, N, 256), 256, 0, s>>>(off, static_cast<int32_t>(N), flags + 2, flags + 3);
