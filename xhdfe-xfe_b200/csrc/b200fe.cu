@@ -686,7 +686,13 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                 B_CHECK(get_buf(ctx, "fy_rec_cf", L.nruns, &frec_cf));
                 B_CHECK(get_buf(ctx, "run_seg", L.nruns, &run_seg));
                 B_CHECK(get_buf(ctx, "grp_off0", static_cast<size_t>(L.G) + 1, &grp_off));
-                const int64_t nranges = (L.nruns + kFyRangeRuns - 1) / kFyRangeRuns;
+                // ranges of 512 runs where that gives every resident warp one,
+                // shorter ones on small panels (300k rows: 111 warps of 512 runs
+                // took 210 us)
+                const int64_t per_warp = L.nruns / (static_cast<int64_t>(ctx->num_sms) * 2 * kCoupleWarps);
+                const int range = static_cast<int>(
+                    std::min<int64_t>(kFyRangeRuns, std::max<int64_t>(kFyRangeRunsMin, per_warp / 32 * 32)));
+                const int64_t nranges = (L.nruns + range - 1) / range;
                 double* cpart;
                 B_CHECK(get_buf(ctx, "cfy64", static_cast<size_t>(L.G) * SGP, &st.cfy64));
                 B_CHECK(get_buf(ctx, "cfy32", static_cast<size_t>(L.G) * SGP, &st.cfy32));
@@ -707,13 +713,13 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                         frec_cf);
                     B_LAUNCHED();
                     coupling_fy_range_kernel<<<fgrid, kCoupleWarps * 32, fsmem, s>>>(
-                        L.nruns, nranges, L.G, frec, frec_cf, sorted_grp, grp_off, st.block_meta,
+                        L.nruns, nranges, range, L.G, frec, frec_cf, sorted_grp, grp_off, st.block_meta,
                         st.block_w64, st.SG, st.SGP, st.cfy64, cpart);
                     B_LAUNCHED();
                     if (nranges > 1) {
                         coupling_fy_join_kernel<<<static_cast<int>(std::min<int64_t>(
                                                       nranges, static_cast<int64_t>(ctx->num_sms) * 8)),
-                                                  256, 0, s>>>(L.nruns, nranges, sorted_grp, grp_off, cpart,
+                                                  256, 0, s>>>(L.nruns, nranges, range, sorted_grp, grp_off, cpart,
                                                                st.SGP, st.cfy64);
                         B_LAUNCHED();
                     }
@@ -754,7 +760,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                 B_CHECK(launch_yy(&coupling_yy_kernel, kCoupleYyWarps,
                                   static_cast<size_t>(kCoupleYyWarps) * couple_yy_warp_words(static_cast<int>(SG)) *
                                       sizeof(double)));
-            coupling_yy_reduce_kernel<<<grid_for(ctx, SG * SG, T256), T256, 0, s>>>(
+            coupling_yy_reduce_kernel<<<static_cast<int>((SG * SG + 31) / 32), 32 * kYySlices, 0, s>>>(
                 ypart, ny, st.SG, st.cyy, Wall + st.sbase[0], Eall + st.sbase[0]);
             B_LAUNCHED();
         }

@@ -395,25 +395,31 @@ row_dot_kernel(int64_t GR, int CP, const A* __restrict__ a, const B* __restrict_
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowThreads + threadIdx.x; i < total;
          i += stride)
         s = fma(static_cast<double>(a[i]), static_cast<double>(b[i]), s);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x < CP) {
-        double t = 0.0;
-        for (int k = threadIdx.x; k < kRowThreads; k += CP) t += red[k];
-        partial[static_cast<int64_t>(blockIdx.x) * CP + threadIdx.x] = t;
-    }
+    // CTA sums by a tree, the CTAs' partials by the whole last CTA (a thread per
+    // column adding them one read at a time took 25-100 us)
+    const int j = threadIdx.x / CP, c = threadIdx.x - j * CP;  // CP is a power of two or 1
+    auto tree = [&](double v) {
+        red[threadIdx.x] = v;
+        __syncthreads();
+        for (int h = kRowThreads / CP / 2; h > 0; h >>= 1) {
+            if (j < h) red[threadIdx.x] += red[threadIdx.x + h * CP];
+            __syncthreads();
+        }
+    };
+    tree(s);
+    if (threadIdx.x < CP) partial[static_cast<int64_t>(blockIdx.x) * CP + threadIdx.x] = red[threadIdx.x];
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x < CP) {
-        double t = 0.0;
-        for (int bb = 0; bb < static_cast<int>(gridDim.x); ++bb)
-            t += __ldcg(partial + static_cast<int64_t>(bb) * CP + threadIdx.x);
-        out[threadIdx.x] = t;
-    }
+    double t = 0.0;
+#pragma unroll 4
+    for (int bb = j; bb < static_cast<int>(gridDim.x); bb += kRowThreads / CP)
+        t += __ldcg(partial + static_cast<int64_t>(bb) * CP + c);
+    tree(t);
+    if (threadIdx.x < CP) out[threadIdx.x] = red[threadIdx.x];
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
@@ -521,7 +527,8 @@ __host__ __device__ __forceinline__ int couple_pitch(int SG) { return SG | 1; }
 // ids with no runs (between two consecutive firms of the order, or before the
 // first or after the last) get zero rows from the warp that passes them.
 constexpr int kCoupleWarps = 8;
-constexpr int kFyRangeRuns = 512;
+constexpr int kFyRangeRuns = 512;     // runs per range at most, and at least:
+constexpr int kFyRangeRunsMin = 32;
 constexpr int kFyPrefetch = 4;
 
 __device__ __forceinline__ void couple_put_row(double* dst, double a0, double a1, int lane, int SG, int SGP) {
@@ -557,7 +564,7 @@ __global__ void fy_run_record_kernel(int64_t nruns, const int32_t* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kCoupleWarps * 32)
-coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int32_t G, const int4* __restrict__ rec,
+coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int range, int32_t G, const int4* __restrict__ rec,
                          const double* __restrict__ rec_cf, const int32_t* __restrict__ sorted_grp,
                          const int32_t* __restrict__ grp_off, const int2* __restrict__ block_meta,
                          const double* __restrict__ block_w, int SG, int SGP, double* __restrict__ out_fy,
@@ -571,7 +578,7 @@ coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int32_t G, const int4* 
     __syncwarp();
     const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kCoupleWarps;
     for (int64_t rg = static_cast<int64_t>(blockIdx.x) * kCoupleWarps + warp; rg < nranges; rg += nwarps) {
-        const int64_t rb = rg * kFyRangeRuns, re = min(rb + kFyRangeRuns, nruns);
+        const int64_t rb = rg * range, re = min(rb + range, nruns);
         int32_t cur = sorted_grp[rb];
         const int32_t prev = rb > 0 ? sorted_grp[rb - 1] : -1;
         if (cur != prev) couple_zero_rows(out_fy, prev + 1, cur, lane, SGP);
@@ -659,17 +666,17 @@ coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int32_t G, const int4* 
 // range order (warp w sums ranges r + 1 + w, r + 9 + w, ...; the eight warp sums
 // are then added to slot 1 in warp order).  One CTA per range.
 __global__ void __launch_bounds__(256)
-coupling_fy_join_kernel(int64_t nruns, int64_t nranges, const int32_t* __restrict__ sorted_grp,
+coupling_fy_join_kernel(int64_t nruns, int64_t nranges, int range, const int32_t* __restrict__ sorted_grp,
                         const int32_t* __restrict__ grp_off, const double* __restrict__ part, int SGP,
                         double* __restrict__ out_fy) {
     __shared__ double ws[8][kCoupleMaxSG];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t r = blockIdx.x; r < nranges; r += gridDim.x) {
-        const int64_t rb = r * kFyRangeRuns, re = min(rb + kFyRangeRuns, nruns);
+        const int64_t rb = r * range, re = min(rb + range, nruns);
         const int32_t f = sorted_grp[re - 1];
         const int64_t fb = grp_off[f], fe = grp_off[f + 1];
         if (fb < rb || fe <= re) continue;  // uniform over the CTA
-        const int64_t r1 = (fe - 1) / kFyRangeRuns;
+        const int64_t r1 = (fe - 1) / range;
         double acc[2] = {0.0, 0.0};
         for (int64_t q = r + 1 + warp; q <= r1; q += 8) {
 #pragma unroll
@@ -867,26 +874,45 @@ coupling_yy_tile_kernel(int32_t Gp, const int2* __restrict__ seg_meta, const int
         partial[static_cast<int64_t>(blockIdx.x) * (SS + SG) + i] = red[i];
 }
 
-// C_yy = diag(W) - sum_s Y_s Y_s' / W_s, CTA partials summed in CTA order; the
-// level weights W_h and E_h = sum_s Y_s[h]^2 / W_s also go to the diagonal
-// arrays of the Jacobi preconditioner (diag C_yy = W_h - E_h, exact).
-__global__ void coupling_yy_reduce_kernel(const double* __restrict__ partial, int nparts, int SG,
-                                          double* __restrict__ out_yy, double* __restrict__ W_out,
-                                          double* __restrict__ E_out) {
+// C_yy = diag(W) - sum_s Y_s Y_s' / W_s from the CTA partials; the level
+// weights W_h and E_h = sum_s Y_s[h]^2 / W_s also go to the diagonal arrays of
+// the Jacobi preconditioner (diag C_yy = W_h - E_h, exact).  A CTA takes 32
+// entries, its warps every kYySlices-th partial, added in warp order (one
+// thread per entry: 47-90 us of dependent reads for 300-444 partials).
+constexpr int kYySlices = 16;
+__global__ void __launch_bounds__(32 * kYySlices)
+coupling_yy_reduce_kernel(const double* __restrict__ partial, int nparts, int SG, double* __restrict__ out_yy,
+                          double* __restrict__ W_out, double* __restrict__ E_out) {
+    __shared__ double red[2][kYySlices][32];
     const int SS = SG * SG;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < SS; i += gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int b = 0; b < nparts; ++b) acc += partial[static_cast<int64_t>(b) * (SS + SG) + i];
-        const int h = i / SG, h2 = i - h * SG;
-        if (h == h2) {
-            double W = 0.0;
-            for (int b = 0; b < nparts; ++b) W += partial[static_cast<int64_t>(b) * (SS + SG) + SS + h];
-            W_out[h] = W;
-            E_out[h] = acc;
-            out_yy[i] = W - acc;
-        } else {
-            out_yy[i] = -acc;
-        }
+    const int e = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + e;
+    const int h = i / SG, h2 = i - h * SG;
+    const bool diag = i < SS && h == h2;
+    double acc = 0.0, W = 0.0;
+    if (i < SS) {
+#pragma unroll 4
+        for (int b = sl; b < nparts; b += kYySlices) acc += partial[static_cast<int64_t>(b) * (SS + SG) + i];
+    }
+    if (diag) {
+#pragma unroll 4
+        for (int b = sl; b < nparts; b += kYySlices) W += partial[static_cast<int64_t>(b) * (SS + SG) + SS + h];
+    }
+    red[0][sl][e] = acc;
+    red[1][sl][e] = W;
+    __syncthreads();
+    if (sl != 0 || i >= SS) return;
+    acc = W = 0.0;
+    for (int k = 0; k < kYySlices; ++k) {
+        acc += red[0][k][e];
+        W += red[1][k][e];
+    }
+    if (diag) {
+        W_out[h] = W;
+        E_out[h] = acc;
+        out_yy[i] = W - acc;
+    } else {
+        out_yy[i] = -acc;
     }
 }
 
