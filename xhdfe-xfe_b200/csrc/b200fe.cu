@@ -2857,33 +2857,52 @@ void ldlt_solve(const Ldlt& f, std::vector<long double>& b) {
 }
 
 // sum_i f_i a_i b_i over the column pairs, summed over CTAs; out [npairs]
-int run_moments(b200fe_context* ctx, MomentArgs m, std::vector<double>& out, double* rss) {
+// 16-byte aligned columns at base + j * ld
+bool vector_columns(const double* base, int64_t ld, int cols) {
+    return (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (cols <= 1 || (ld & 1) == 0);
+}
+
+template <int NB>
+void launch_gram(bool vec, int grid, cudaStream_t s, const GramArgs& m) {
+    if (vec) gram_kernel<NB, true><<<grid, kOlsThreads, 0, s>>>(m);
+    else gram_kernel<NB, false><<<grid, kOlsThreads, 0, s>>>(m);
+}
+
+// Pair sums of the columns (GramArgs) to the host, upper triangle row by row.
+int run_gram(b200fe_context* ctx, GramArgs m, std::vector<double>& out) {
     const cudaStream_t s = ctx->stream;
     const int npairs = m.P * (m.P + 1) / 2;
-    const int grid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>((m.n + kOlsTile - 1) / kOlsTile, static_cast<int64_t>(ctx->num_sms) * 4)));
-    double *part, *sum, *rpart = nullptr, *rsum = nullptr;
-    B_CHECK(get_buf(ctx, "ols_part", static_cast<size_t>(grid) * npairs, &part));
+    const int NB = (m.P + 7) / 8;
+    const int grid = grid_for(ctx, (m.n + kGramRows - 1) / kGramRows * 32, kOlsThreads, 6);
+    double* sum;
+    B_CHECK(get_buf(ctx, "ols_part", static_cast<size_t>(grid) * gram_tiles(NB) * 64, &m.partial));
     B_CHECK(get_buf(ctx, "ols_sum", static_cast<size_t>(npairs) + 1, &sum));
-    if (rss) {
-        B_CHECK(get_buf(ctx, "ols_rpart", grid, &rpart));
-        B_CHECK(get_buf(ctx, "ols_rsum", 1, &rsum));
-    }
-    m.partial = part;
-    m.rss_partial = rpart;
-    moments_kernel<<<grid, kOlsThreads, 0, s>>>(m);
+    const bool vec = vector_columns(m.X, m.ld, m.p) && (m.P == m.p || vector_columns(m.y, 0, 1));
+    if (NB <= 1) launch_gram<1>(vec, grid, s, m);
+    else if (NB == 2) launch_gram<2>(vec, grid, s, m);
+    else if (NB == 3) launch_gram<3>(vec, grid, s, m);
+    else if (NB == 4) launch_gram<4>(vec, grid, s, m);
+    else launch_gram<5>(vec, grid, s, m);
     B_LAUNCHED();
-    partial_sum_kernel<<<grid_for(ctx, npairs, 256, 1), 256, 0, s>>>(part, grid, npairs, sum);
+    gram_pairs_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(m.partial, grid, NB, m.P, sum);
     B_LAUNCHED();
-    if (rss) {
-        partial_sum_kernel<<<1, 32, 0, s>>>(rpart, grid, 1, rsum);
-        B_LAUNCHED();
-    }
     out.assign(npairs, 0.0);
-    B_TRY(cudaMemcpyAsync(out.data(), sum, sizeof(double) * npairs, cudaMemcpyDeviceToHost, s));
-    if (rss) B_TRY(cudaMemcpyAsync(rss, rsum, sizeof(double), cudaMemcpyDeviceToHost, s));
-    B_TRY(cudaStreamSynchronize(s));
-    return B200FE_OK;
+    return sync_read_double(ctx, sum, npairs, out.data());
+}
+
+// RSS to the host and the per-row output of ResidualArgs
+int run_residuals(b200fe_context* ctx, ResidualArgs m, double* rss) {
+    const cudaStream_t s = ctx->stream;
+    const int grid = grid_for(ctx, (m.n + 1) / 2, kOlsThreads, 6);
+    double* rsum;
+    B_CHECK(get_buf(ctx, "ols_rpart", grid, &m.rss_partial));
+    B_CHECK(get_buf(ctx, "ols_rsum", 1, &rsum));
+    if (vector_columns(m.X, m.n, m.p)) residual_kernel<true><<<grid, kOlsThreads, 0, s>>>(m);
+    else residual_kernel<false><<<grid, kOlsThreads, 0, s>>>(m);
+    B_LAUNCHED();
+    rss_sum_kernel<<<1, 32, 0, s>>>(m.rss_partial, grid, rsum);
+    B_LAUNCHED();
+    return sync_read_double(ctx, rsum, 1, rss);
 }
 
 // upper-triangle pair list -> symmetric P x P (column-major)
@@ -2899,24 +2918,22 @@ std::vector<double> unpack_pairs(const std::vector<double>& v, int P) {
 }
 
 int ols_impl(b200fe_context* ctx, const double* d_y, const double* d_X, int64_t n, int p,
-             const double* d_w, const int32_t* d_cl, int32_t G, int se_type, double n_effective,
-             int wfreq, b200fe_ols_result* out) {
+             const double* d_w, const int32_t* d_cl, int32_t G, bool cl_sorted, int se_type,
+             double n_effective, int wfreq, b200fe_ols_result* out) {
     const cudaStream_t s = ctx->stream;
     std::memset(out, 0, sizeof(*out));
     out->p = p;
     // 1. Gram [X y]' W [X y]
-    MomentArgs m{};
+    GramArgs m{};
     m.n = n;
     m.P = p + 1;
     m.p = p;
     m.X = d_X;
-    m.cs = n;
-    m.rs = 1;
+    m.ld = n;
     m.y = d_y;
-    m.w = d_w;
-    m.mode = kMomGram;
+    m.f = d_w;
     std::vector<double> g;
-    B_CHECK(run_moments(ctx, m, g, nullptr));
+    B_CHECK(run_gram(ctx, m, g));
     const std::vector<double> GM = unpack_pairs(g, p + 1);
     std::vector<double> xtx(static_cast<size_t>(p) * p);
     std::vector<long double> xty(p);
@@ -2940,14 +2957,18 @@ int ols_impl(b200fe_context* ctx, const double* d_y, const double* d_X, int64_t 
         for (int i = 0; i < p; ++i) inv[static_cast<size_t>(j) * p + i] = static_cast<double>(e[i]);
     }
     for (int i = 0; i < p * p; ++i) out->xtx_inv[i] = inv[i];
-    // 2. residual pass: RSS, and the meat for robust inference
-    m.P = p;
-    m.mode = se_type == 1 ? kMomRobust : kMomRss;
-    m.wfreq = wfreq;
-    for (int j = 0; j < p; ++j) m.beta[j] = out->coef[j];
-    std::vector<double> rm;
+    // 2. residual pass: RSS, and per row what the meat needs
+    ResidualArgs ra{};
+    ra.n = n;
+    ra.p = p;
+    ra.X = d_X;
+    ra.y = d_y;
+    ra.w = d_w;
+    for (int j = 0; j < p; ++j) ra.beta[j] = out->coef[j];
+    ra.output = se_type == 2 ? kRowScore : se_type == 1 ? (wfreq ? kRowRobustFreq : kRowRobust) : kRowNone;
+    if (ra.output != kRowNone) B_CHECK(get_buf(ctx, "ols_row", n, &ra.row));
     double rss = 0.0;
-    B_CHECK(run_moments(ctx, m, rm, &rss));
+    B_CHECK(run_residuals(ctx, ra, &rss));
     const double n_eff = n_effective > 0.0 ? n_effective : static_cast<double>(n);
     const double df_resid = std::max(0.0, n_eff - p);
     out->rss = rss;
@@ -2956,21 +2977,27 @@ int ols_impl(b200fe_context* ctx, const double* d_y, const double* d_X, int64_t 
     out->cov_scale = 1.0;
     std::vector<double> meat;
     if (se_type == 1) {
+        m.P = p;
+        m.f = ra.row;
+        std::vector<double> rm;
+        B_CHECK(run_gram(ctx, m, rm));
         meat = unpack_pairs(rm, p);
     } else if (se_type == 2) {
         // 3. cluster scores in cluster order (stable sort by cluster id)
-        int32_t *keys, *perm, *skeys, *iota, *off;
-        B_CHECK(get_buf(ctx, "ols_keys", n, &keys));
-        B_CHECK(get_buf(ctx, "ols_perm", n, &perm));
-        B_CHECK(get_buf(ctx, "ols_skeys", n, &skeys));
-        B_CHECK(get_buf(ctx, "ols_iota", n, &iota));
+        int32_t *perm = nullptr, *skeys, *iota, *off;
         B_CHECK(get_buf(ctx, "ols_off", static_cast<size_t>(G) + 1, &off));
-        iota_kernel<<<grid_for(ctx, n, 256), 256, 0, s>>>(iota, n);
+        const int32_t* sorted = d_cl;  // rows in cluster order already: no sort
+        if (!cl_sorted) {
+            B_CHECK(get_buf(ctx, "ols_perm", n, &perm));
+            B_CHECK(get_buf(ctx, "ols_skeys", n, &skeys));
+            B_CHECK(get_buf(ctx, "ols_iota", n, &iota));
+            iota_kernel<<<grid_for(ctx, n, 256), 256, 0, s>>>(iota, n);
+            B_LAUNCHED();
+            B_CHECK(cub_sort_pairs(ctx, d_cl, skeys, iota, perm, n, G));
+            sorted = skeys;
+        }
+        segment_offsets_kernel<<<grid_for(ctx, n + 1, 256), 256, 0, s>>>(sorted, n, G, off);
         B_LAUNCHED();
-        B_CHECK(cub_sort_pairs(ctx, d_cl, skeys, iota, perm, n, G));
-        segment_offsets_kernel<<<grid_for(ctx, n + 1, 256), 256, 0, s>>>(skeys, n, G, off);
-        B_LAUNCHED();
-        (void)keys;
         int32_t *nch, *ch_off, *mflag, *midx;
         B_CHECK(get_buf(ctx, "ols_nch", static_cast<size_t>(G) + 1, &nch));
         B_CHECK(get_buf(ctx, "ols_choff", static_cast<size_t>(G) + 1, &ch_off));
@@ -3016,19 +3043,20 @@ int ols_impl(b200fe_context* ctx, const double* d_y, const double* d_X, int64_t 
         c.p = p;
         c.X = d_X;
         c.ld = n;
-        c.y = d_y;
-        c.w = d_w;
-        for (int j = 0; j < p; ++j) c.beta[j] = out->coef[j];
+        c.we = ra.row;
+        c.G = G;
         c.scores = scores;
         c.chunk_part = cpart;
         c.small_max = kOlsSmallCluster;
-        cluster_small_kernel<<<grid_for(ctx, G, kOlsThreads, 8), kOlsThreads, 0, s>>>(c, off, G);
+        constexpr int kSmem = kOlsThreads / 32 * 2 * kClusterBuf * static_cast<int>(sizeof(double));
+        B_TRY(raise_smem_limit(reinterpret_cast<const void*>(&cluster_small_kernel), kSmem));
+        cluster_small_kernel<<<grid_for(ctx, G, kOlsThreads, 3), kOlsThreads, kSmem, s>>>(c, off, G);
         B_LAUNCHED();
         cluster_chunk_kernel<<<grid_for(ctx, nchunks * 32, kOlsThreads, 8), kOlsThreads, 0, s>>>(c);
         B_LAUNCHED();
         if (nmulti > 0) {
             cluster_combine_kernel<<<grid_for(ctx, nmulti * width, 256), 256, 0, s>>>(
-                nmulti, mgrp, mc0, mc1, cpart, width, scores);
+                nmulti, mgrp, mc0, mc1, cpart, width, G, scores);
             B_LAUNCHED();
         }
         int* cnt;
@@ -3039,17 +3067,15 @@ int ols_impl(b200fe_context* ctx, const double* d_y, const double* d_X, int64_t 
         int ncl = 0;
         B_CHECK(sync_read_int(ctx, cnt, 1, &ncl));
         // meat = sum_g s_g s_g', cluster_u2 = sum_g u_g^2: moments of the scores
-        MomentArgs q{};
+        GramArgs q{};
         q.n = G;
         q.P = p + 1;
         q.p = p;
         q.X = scores;
-        q.cs = 1;
-        q.rs = width;
-        q.y = scores + p;
-        q.mode = kMomPlain;
+        q.ld = G;
+        q.y = scores + static_cast<int64_t>(p) * G;
         std::vector<double> sm;
-        B_CHECK(run_moments(ctx, q, sm, nullptr));
+        B_CHECK(run_gram(ctx, q, sm));
         const std::vector<double> SM = unpack_pairs(sm, p + 1);
         meat.assign(static_cast<size_t>(p) * p, 0.0);
         for (int j = 0; j < p; ++j)
@@ -3105,21 +3131,23 @@ int b200fe_ols_device(b200fe_context* ctx, const double* d_y, const double* d_X,
         cudaGetLastError();
         return B200FE_UNAVAILABLE;
     }
+    bool cl_sorted = false;
     if (se_type == 2) {  // cluster ids must be dense in [0, G)
         int* bad;
         B_CHECK(get_buf(ctx, "ols_bad", 3, &bad));
         B_TRY(cudaMemsetAsync(bad, 0, 3 * sizeof(int), ctx->stream));
-        validate_ids_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(d_clusters, n, num_clusters, 0, bad);
+        validate_ids_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(d_clusters, n, num_clusters, 1, bad);
         B_LAUNCHED();
-        int hb = 0;
-        B_CHECK(sync_read_int(ctx, bad, 1, &hb));
-        if (hb) {
+        int hb[2] = {0, 0};
+        B_CHECK(sync_read_int(ctx, bad, 2, hb));
+        if (hb[0]) {
             ctx->err = "cluster ids out of range";
             return B200FE_INVALID_ARG;
         }
+        cl_sorted = hb[1] == 0;
     }
     return ols_impl(ctx, d_y, d_X, n, p, d_weights, se_type == 2 ? d_clusters : nullptr,
-                    num_clusters, se_type, n_effective, weights_are_frequencies, out);
+                    num_clusters, cl_sorted, se_type, n_effective, weights_are_frequencies, out);
 }
 
 int b200fe_ols(b200fe_context* ctx, const double* y, const double* X, int64_t n, int p,
