@@ -29,29 +29,33 @@ namespace {
 // their super-chunks (groups of more than kFinFewParts chunks: the Zipf-giant
 // firm owns thousands).  Fills the chunk fields of L; L.G is set by the
 // caller; buffer names end in sfx.
-int build_chunks(b200fe_context* ctx, const int32_t* grp_off, int32_t CH, const std::string& sfx,
-                 LargeDim& L) {
+struct ChunkScan {
+    int32_t *nch = nullptr, *ch_off = nullptr, *midx = nullptr;
+};
+// Counts only; the totals are ch_off[G] and midx[G].
+int count_chunks(b200fe_context* ctx, const int32_t* grp_off, int32_t CH, int64_t G, ChunkScan* c) {
     const cudaStream_t s = ctx->stream;
     const int T256 = 256;
-    // chunk list
-    int32_t *nch, *ch_off, *mflag, *midx;
-    B_CHECK(get_buf(ctx, "nch", static_cast<size_t>(L.G) + 1, &nch));
-    B_CHECK(get_buf(ctx, "ch_off", static_cast<size_t>(L.G) + 1, &ch_off));
-    B_CHECK(get_buf(ctx, "mflag", static_cast<size_t>(L.G) + 1, &mflag));
-    B_CHECK(get_buf(ctx, "midx", static_cast<size_t>(L.G) + 1, &midx));
-    B_TRY(cudaMemsetAsync(nch, 0, sizeof(int32_t) * (static_cast<size_t>(L.G) + 1), s));
-    B_TRY(cudaMemsetAsync(mflag, 0, sizeof(int32_t) * (static_cast<size_t>(L.G) + 1), s));
-    chunk_count_kernel<<<grid_for(ctx, L.G, T256), T256, 0, s>>>(grp_off, L.G, CH, nch);
+    const size_t g1 = static_cast<size_t>(G) + 1;
+    int32_t* mflag;
+    B_CHECK(get_buf(ctx, "nch", g1, &c->nch));
+    B_CHECK(get_buf(ctx, "ch_off", g1, &c->ch_off));
+    B_CHECK(get_buf(ctx, "mflag", g1, &mflag));
+    B_CHECK(get_buf(ctx, "midx", g1, &c->midx));
+    B_TRY(cudaMemsetAsync(c->nch + G, 0, sizeof(int32_t), s));
+    B_TRY(cudaMemsetAsync(mflag + G, 0, sizeof(int32_t), s));
+    chunk_count_kernel<<<grid_for(ctx, G, T256), T256, 0, s>>>(grp_off, static_cast<int32_t>(G), CH, c->nch);
     B_LAUNCHED();
-    B_CHECK(cub_exclusive_sum(ctx, nch, ch_off, static_cast<int64_t>(L.G) + 1));
-    multi_flag_kernel<<<grid_for(ctx, L.G, T256), T256, 0, s>>>(nch, L.G, mflag);
+    B_CHECK(cub_exclusive_sum(ctx, c->nch, c->ch_off, static_cast<int64_t>(g1)));
+    multi_flag_kernel<<<grid_for(ctx, G, T256), T256, 0, s>>>(c->nch, static_cast<int32_t>(G), mflag);
     B_LAUNCHED();
-    B_CHECK(cub_exclusive_sum(ctx, mflag, midx, static_cast<int64_t>(L.G) + 1));
-    int hc[2];
-    B_CHECK(sync_read_int(ctx, ch_off + L.G, 1, &hc[0]));
-    B_CHECK(sync_read_int(ctx, midx + L.G, 1, &hc[1]));
-    L.nchunks = hc[0];
-    L.nmulti = hc[1];
+    return cub_exclusive_sum(ctx, mflag, c->midx, static_cast<int64_t>(g1));
+}
+// The lists, L.nchunks and L.nmulti known.
+int fill_chunks(b200fe_context* ctx, const int32_t* grp_off, int32_t CH, const std::string& sfx, const ChunkScan& c,
+                LargeDim& L) {
+    const cudaStream_t s = ctx->stream;
+    const int T256 = 256;
     B_CHECK(get_buf(ctx, "chunk_grp" + sfx, L.nchunks, &L.chunk_grp));
     B_CHECK(get_buf(ctx, "chunk_beg" + sfx, L.nchunks, &L.chunk_beg));
     B_CHECK(get_buf(ctx, "chunk_end" + sfx, L.nchunks, &L.chunk_end));
@@ -60,42 +64,43 @@ int build_chunks(b200fe_context* ctx, const int32_t* grp_off, int32_t CH, const 
     B_CHECK(get_buf(ctx, "multi_c0" + sfx, L.nmulti, &L.multi_c0));
     B_CHECK(get_buf(ctx, "multi_c1" + sfx, L.nmulti, &L.multi_c1));
     chunk_fill_kernel<<<grid_for(ctx, L.G, T256), T256, 0, s>>>(
-        grp_off, L.G, CH, ch_off, L.chunk_grp, L.chunk_beg, L.chunk_end,
-        L.chunk_whole, midx, L.multi_grp, L.multi_c0, L.multi_c1);
+        grp_off, L.G, CH, c.ch_off, L.chunk_grp, L.chunk_beg, L.chunk_end, L.chunk_whole, c.midx, L.multi_grp,
+        L.multi_c0, L.multi_c1);
     B_LAUNCHED();
     // super-chunks: a group with many chunks (Zipf sizes: one firm may own
     // 10%+ of the runs) has its chunk partials summed in slices of
     // kSuperParts by many lane groups before finalize adds the slices
     L.nsup = 0;
     if (L.nmulti > 0) {
-        std::vector<int32_t> c0(L.nmulti), c1(L.nmulti);
-        B_TRY(cudaMemcpyAsync(c0.data(), L.multi_c0, sizeof(int32_t) * L.nmulti, cudaMemcpyDeviceToHost, s));
-        B_TRY(cudaMemcpyAsync(c1.data(), L.multi_c1, sizeof(int32_t) * L.nmulti, cudaMemcpyDeviceToHost, s));
-        B_TRY(cudaStreamSynchronize(s));
-        std::vector<int32_t> s0(L.nmulti), s1(L.nmulti), sb, se;
-        for (int64_t r = 0; r < L.nmulti; ++r) {
-            s0[r] = s1[r] = static_cast<int32_t>(sb.size());
-            if (c1[r] - c0[r] <= kFinFewParts) continue;
-            for (int32_t c = c0[r]; c < c1[r]; c += kSuperParts) {
-                sb.push_back(c);
-                se.push_back(std::min(c1[r], c + kSuperParts));
-            }
-            s1[r] = static_cast<int32_t>(sb.size());
-        }
-        L.nsup = static_cast<int64_t>(sb.size());
+        // at most one partly filled slice per group of more than kFinFewParts chunks
+        L.nsup = L.nchunks / kSuperParts + std::min<int64_t>(L.nmulti, L.nchunks / (kFinFewParts + 1));
+        int32_t *cnt, *off;
+        B_CHECK(get_buf(ctx, "sup_cnt", static_cast<size_t>(L.nmulti) + 1, &cnt));
+        B_CHECK(get_buf(ctx, "sup_off", static_cast<size_t>(L.nmulti) + 1, &off));
         B_CHECK(get_buf(ctx, "multi_s0" + sfx, L.nmulti, &L.multi_s0));
         B_CHECK(get_buf(ctx, "multi_s1" + sfx, L.nmulti, &L.multi_s1));
         B_CHECK(get_buf(ctx, "sup_c0" + sfx, std::max<int64_t>(L.nsup, 1), &L.sup_c0));
         B_CHECK(get_buf(ctx, "sup_c1" + sfx, std::max<int64_t>(L.nsup, 1), &L.sup_c1));
-        B_TRY(cudaMemcpyAsync(L.multi_s0, s0.data(), sizeof(int32_t) * L.nmulti, cudaMemcpyHostToDevice, s));
-        B_TRY(cudaMemcpyAsync(L.multi_s1, s1.data(), sizeof(int32_t) * L.nmulti, cudaMemcpyHostToDevice, s));
-        if (L.nsup > 0) {
-            B_TRY(cudaMemcpyAsync(L.sup_c0, sb.data(), sizeof(int32_t) * L.nsup, cudaMemcpyHostToDevice, s));
-            B_TRY(cudaMemcpyAsync(L.sup_c1, se.data(), sizeof(int32_t) * L.nsup, cudaMemcpyHostToDevice, s));
-        }
-        B_TRY(cudaStreamSynchronize(s));  // the host vectors leave scope
+        super_count_kernel<<<grid_for(ctx, L.nmulti + 1, T256), T256, 0, s>>>(L.nmulti, L.multi_c0, L.multi_c1, cnt);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, cnt, off, L.nmulti + 1));
+        super_fill_kernel<<<grid_for(ctx, std::max(L.nmulti, L.nsup), T256), T256, 0, s>>>(
+            L.nmulti, L.multi_c0, L.multi_c1, off, L.nsup, L.multi_s0, L.multi_s1, L.sup_c0, L.sup_c1);
+        B_LAUNCHED();
     }
     return B200FE_OK;
+}
+int build_chunks(b200fe_context* ctx, const int32_t* grp_off, int32_t CH, const std::string& sfx, LargeDim& L) {
+    ChunkScan c;
+    B_CHECK(count_chunks(ctx, grp_off, CH, L.G, &c));
+    int hc[2];
+    ReadBatch rb;
+    rb.add(c.ch_off + L.G, sizeof(int), &hc[0]);
+    rb.add(c.midx + L.G, sizeof(int), &hc[1]);
+    B_CHECK(rb.wait(ctx));
+    L.nchunks = hc[0];
+    L.nmulti = hc[1];
+    return fill_chunks(ctx, grp_off, CH, sfx, c, L);
 }
 
 // Records of the regular tiles for the bulk-copy data passes
@@ -117,8 +122,7 @@ int build_stream_meta(b200fe_context* ctx) {
     tile_regular_flag_kernel<<<grid_for(ctx, st.ntiles + 1, 256), 256, 0, s>>>(st.ntiles, st.tile_long, rflag);
     B_LAUNCHED();
     B_CHECK(cub_exclusive_sum(ctx, rflag, ridx, static_cast<int64_t>(t1)));
-    int nreg = 0;
-    B_CHECK(sync_read_int(ctx, ridx + st.ntiles, 1, &nreg));
+    const int nreg = static_cast<int>(st.ntiles - st.nlong);  // a long segment is a tile of its own
     st.stream_nreg = nreg;
     if (nreg == 0) return B200FE_OK;
     st.stream_aux_stride = stream_aux_stride(st.nL, st.SG, st.nS);
@@ -143,12 +147,13 @@ int build_stream_meta(b200fe_context* ctx) {
     tile_meta_kernel<<<grid_for(ctx, st.ntiles, 256), 256, 0, s>>>(m);
     B_LAUNCHED();
     B_CHECK(cub_exclusive_sum(ctx, bsize, st.stream_boff, static_cast<int64_t>(nreg) + 1));
-    int hf[2] = {0, 0}, units = 0;
-    B_CHECK(sync_read_int(ctx, flags, 2, hf));
-    B_CHECK(sync_read_int(ctx, st.stream_boff + nreg, 1, &units));
-    if (hf[0] != 0) return B200FE_OK;
-    st.stream_blob_max = hf[1];
-    B_CHECK(get_buf(ctx, "stream_blob", static_cast<size_t>(std::max(units, 1)) * 16, &st.stream_blob));
+    // room for every record without waiting for their sizes (blob_layout: each
+    // of at most ten sections is padded to 16 bytes)
+    size_t room = static_cast<size_t>(nreg) * (2 * st.stream_aux_stride + 160 + 8 * st.nL) +
+                  static_cast<size_t>(st.G[st.p]) * 10 + static_cast<size_t>(st.n) * 2 * st.nS;
+    for (int l = 0; l < st.nL; ++l) room += static_cast<size_t>(st.L[l].nruns) * (l == 0 ? 10 : 6);
+    B_CHECK(get_buf(ctx, "stream_blob", room + 16, &st.stream_blob));
+    st.stream_flags = flags;  // read with the last wait of the build
     TileBlobArgs x{};
     x.nreg = nreg;
     x.tmeta = st.stream_meta;
@@ -169,19 +174,29 @@ int build_stream_meta(b200fe_context* ctx) {
     x.blob = st.stream_blob;
     tile_blob_kernel<<<static_cast<int>((nreg + kBlobWarps - 1) / kBlobWarps), kBlobWarps * 32, 0, s>>>(x);
     B_LAUNCHED();
-    st.stream_ok = true;
     return B200FE_OK;
 }
 
-// The explicit S_ff of the one large dim (see sparse_kernels.cuh).  Leaves
-// st.sparse false (run-level matvec) when a segment has more than
-// kSparseMaxRuns runs or the contributions would exceed eight per run.
-int build_sparse_block(b200fe_context* ctx) {
+SparseRuns sparse_runs(const Structure& st) {
+    SparseRuns a{};
+    a.nd = st.nL;
+    for (int l = 0; l < st.nL && l < 2; ++l) {
+        a.run_base[l] = st.L[l].run_base;
+        a.run_grp[l] = st.L[l].run_grp;
+        a.run_start[l] = st.L[l].run_start;
+        a.run_w[l] = st.L[l].cw_run;
+        a.row0[l] = static_cast<int32_t>(st.lbase[l]);
+    }
+    return a;
+}
+
+// Counts the contributions of the explicit Schur block of the large dims
+// (sparse_kernels.cuh).  *pairs = -1 (another matvec form) when a segment has
+// more than kSparseMaxRuns runs or the contributions would exceed eight per run.
+int count_sparse_pairs(b200fe_context* ctx, int64_t* pairs) {
     Structure& st = ctx->st;
     const cudaStream_t s = ctx->stream;
-    const int T256 = 256;
     const int32_t Gp = st.G[st.p];
-    LargeDim& L = st.L[0];
     int32_t *count, *flag;
     unsigned long long* total;
     B_CHECK(get_buf(ctx, "sp_count", static_cast<size_t>(Gp) + 1, &count));
@@ -190,17 +205,33 @@ int build_sparse_block(b200fe_context* ctx) {
     B_TRY(cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
     B_TRY(cudaMemsetAsync(total, 0, sizeof(unsigned long long), s));
     B_TRY(cudaMemsetAsync(count + Gp, 0, sizeof(int32_t), s));
-    sparse_pair_count_kernel<<<grid_for(ctx, Gp, T256), T256, 0, s>>>(Gp, L.run_base, L.run_grp,
-                                                                        count, flag, total);
+    sparse_pair_count_kernel<<<grid_for(ctx, Gp, 256), 256, 0, s>>>(Gp, sparse_runs(st), count, flag, total);
     B_LAUNCHED();
     unsigned long long htot = 0;
     int hflag = 0;
-    B_TRY(cudaMemcpyAsync(&htot, total, sizeof(htot), cudaMemcpyDeviceToHost, s));
-    B_CHECK(sync_read_int(ctx, flag, 1, &hflag));  // synchronises htot too
-    const unsigned long long cap = std::min<unsigned long long>(
-        8ull * static_cast<unsigned long long>(L.nruns) + (1ull << 20), (1ull << 31) - 1);
-    if (hflag || htot > cap) return B200FE_OK;
-    st.sp_pairs = static_cast<int64_t>(htot);
+    ReadBatch rb;
+    rb.add(total, sizeof(htot), &htot);
+    rb.add(flag, sizeof(hflag), &hflag);
+    B_CHECK(rb.wait(ctx));
+    unsigned long long nruns = 0;
+    for (int l = 0; l < st.nL; ++l) nruns += static_cast<unsigned long long>(st.L[l].nruns);
+    const unsigned long long cap = std::min<unsigned long long>(8ull * nruns + (1ull << 20), (1ull << 31) - 1);
+    *pairs = hflag || htot > cap ? -1 : static_cast<int64_t>(htot);
+    return B200FE_OK;
+}
+
+// The explicit Schur block of the large dims from its counted contributions.
+int build_sparse_block(b200fe_context* ctx, int64_t pairs) {
+    Structure& st = ctx->st;
+    const cudaStream_t s = ctx->stream;
+    const int T256 = 256;
+    const int32_t Gp = st.G[st.p];
+    LargeDim L;  // all rows
+    L.G = static_cast<int32_t>(st.lrows);
+    int32_t *count, *flag;
+    B_CHECK(get_buf(ctx, "sp_count", static_cast<size_t>(Gp) + 1, &count));
+    B_CHECK(get_buf(ctx, "sp_flag", 4, &flag));
+    st.sp_pairs = pairs;
     st.sp.G = L.G;
     const int64_t np = std::max<int64_t>(st.sp_pairs, 1);
     int32_t* off;
@@ -215,7 +246,7 @@ int build_sparse_block(b200fe_context* ctx) {
     int32_t *ustart, *urow;
     if (st.sp_pairs > 0) {
         sparse_pair_fill_kernel<<<grid_for(ctx, Gp, T256), T256, 0, s>>>(
-            Gp, L.run_base, L.run_grp, L.cw_run, st.inv_wp, count, off, L.G, k_in, v_in);
+            Gp, sparse_runs(st), st.inv_wp, st.wp64, count, off, st.lrows, k_in, v_in);
         B_LAUNCHED();
         // stable sort by (row, column): equal keys keep segment order
         const unsigned long long gmax = static_cast<unsigned long long>(L.G) * L.G;
@@ -243,7 +274,7 @@ int build_sparse_block(b200fe_context* ctx) {
         B_CHECK(get_buf(ctx, "sp_urow", nnz, &urow));
         B_CHECK(get_buf(ctx, "sp_col", nnz, &st.sp_col));
         sparse_unique_fill_kernel<<<grid_for(ctx, st.sp_pairs, T256), T256, 0, s>>>(
-            k_out, st.sp_pairs, flags, uid, L.G, ustart, urow, st.sp_col);
+            k_out, st.sp_pairs, flags, uid, st.lrows, ustart, urow, st.sp_col);
         B_LAUNCHED();
         int32_t* long_list;
         B_CHECK(get_buf(ctx, "sp_val64", nnz, &st.sp_val64));
@@ -270,7 +301,8 @@ int build_sparse_block(b200fe_context* ctx) {
     segment_offsets_kernel<<<grid_for(ctx, st.sp_nnz + 1, T256), T256, 0, s>>>(urow, st.sp_nnz, L.G,
                                                                               st.sp_row_off);
     B_LAUNCHED();
-    B_CHECK(build_chunks(ctx, st.sp_row_off, kSparseChunk, "_sp", st.sp));
+    ChunkScan csc;
+    B_CHECK(count_chunks(ctx, st.sp_row_off, kSparseChunk, L.G, &csc));
     // work lists of the persistent PCG: short rows, long rows and their chunks
     {
         const size_t g1 = static_cast<size_t>(L.G) + 1;
@@ -294,16 +326,23 @@ int build_sparse_block(b200fe_context* ctx) {
         B_CHECK(cub_exclusive_sum(ctx, is_short, short_idx, static_cast<int64_t>(g1)));
         B_CHECK(cub_exclusive_sum(ctx, is_long, long_idx, static_cast<int64_t>(g1)));
         B_CHECK(cub_exclusive_sum(ctx, nch, chunk_off, static_cast<int64_t>(g1)));
-        int cnt[4];
-        B_CHECK(sync_read_int(ctx, huge_idx + L.G, 1, &cnt[3]));
-        st.pc_nhuge = cnt[3];
-        B_CHECK(get_buf(ctx, "pc_huge_li", std::max<int64_t>(st.pc_nhuge, 1), &st.pc_huge_li));
-        B_CHECK(sync_read_int(ctx, short_idx + L.G, 1, &cnt[0]));
-        B_CHECK(sync_read_int(ctx, long_idx + L.G, 1, &cnt[1]));
-        B_CHECK(sync_read_int(ctx, chunk_off + L.G, 1, &cnt[2]));
+        int cnt[4], hc[2];
+        ReadBatch rb;
+        rb.add(short_idx + L.G, sizeof(int), &cnt[0]);
+        rb.add(long_idx + L.G, sizeof(int), &cnt[1]);
+        rb.add(chunk_off + L.G, sizeof(int), &cnt[2]);
+        rb.add(huge_idx + L.G, sizeof(int), &cnt[3]);
+        rb.add(csc.ch_off + L.G, sizeof(int), &hc[0]);
+        rb.add(csc.midx + L.G, sizeof(int), &hc[1]);
+        B_CHECK(rb.wait(ctx));
+        st.sp.nchunks = hc[0];
+        st.sp.nmulti = hc[1];
+        B_CHECK(fill_chunks(ctx, st.sp_row_off, kSparseChunk, "_sp", csc, st.sp));
         st.pc_nshort = cnt[0];
         st.pc_nlong = cnt[1];
         st.pc_nlchunks = cnt[2];
+        st.pc_nhuge = cnt[3];
+        B_CHECK(get_buf(ctx, "pc_huge_li", std::max<int64_t>(st.pc_nhuge, 1), &st.pc_huge_li));
         B_CHECK(get_buf(ctx, "pc_short_row", std::max<int64_t>(st.pc_nshort, 1), &st.pc_short_rows));
         B_CHECK(get_buf(ctx, "pc_long_meta", std::max<int64_t>(st.pc_nlong, 1), &st.pc_long_meta));
         B_CHECK(get_buf(ctx, "pc_lchunk_meta", std::max<int64_t>(st.pc_nlchunks, 1), &st.pc_lchunk_meta));
@@ -456,8 +495,10 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         B_CHECK(cub_exclusive_sum(ctx, tflag, tidx, g1));
         B_CHECK(cub_exclusive_sum(ctx, lflag, lidx, g1));
         int cnt[2];
-        B_CHECK(sync_read_int(ctx, tidx + G[p], 1, &cnt[0]));
-        B_CHECK(sync_read_int(ctx, lidx + G[p], 1, &cnt[1]));
+        ReadBatch rb;
+        rb.add(tidx + G[p], sizeof(int), &cnt[0]);
+        rb.add(lidx + G[p], sizeof(int), &cnt[1]);
+        B_CHECK(rb.wait(ctx));
         st.ntiles = cnt[0];
         st.nlong = cnt[1];
         B_CHECK(get_buf(ctx, "tile_seg", static_cast<size_t>(st.ntiles) + 1, &st.tile_seg));
@@ -492,6 +533,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         st.lbase[l] = row;
         row += st.L[l].G;
     }
+    st.lrows = row;
     st.SG = 0;
     for (int j = 0; j < st.nS; ++j) {
         st.sbase[j] = row;
@@ -527,16 +569,11 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         B_CHECK(get_buf(ctx, "run_grp" + sfx, nr, &run_grp));
         L.run_grp = run_grp;
         B_CHECK(get_buf(ctx, "run_start" + sfx, static_cast<size_t>(nr) + 1, &run_start));
-        B_CHECK(get_buf(ctx, "run_seg", nr, &run_seg));
+        B_CHECK(get_buf(ctx, "run_seg" + sfx, nr, &run_seg));
         L.run_start = run_start;
         run_fill_kernel<<<grid_for(ctx, n, T256), T256, 0, s>>>(rflags, run_id, gp, L.rid, n,
                                                                 run_grp, run_start, run_seg);
         B_LAUNCHED();
-        {
-            const int32_t n32 = static_cast<int32_t>(n);
-            B_TRY(cudaMemcpyAsync(run_start + nr, &n32, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-            B_TRY(cudaStreamSynchronize(s));  // n32 lives on this stack frame
-        }
         B_CHECK(get_buf(ctx, "run_base" + sfx, static_cast<size_t>(G[p]) + 1, &L.run_base));
         run_base_kernel<<<grid_for(ctx, static_cast<int64_t>(G[p]) + 1, T256), T256, 0, s>>>(
             seg_off, G[p], run_id, n, nr, L.run_base);
@@ -545,7 +582,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         int32_t *riota, *sorted_runs, *sorted_grp;
         B_CHECK(get_buf(ctx, "tmp_n_a", n, &riota));  // flags no longer needed
         B_CHECK(get_buf(ctx, "sorted_runs", nr, &sorted_runs));
-        B_CHECK(get_buf(ctx, "sorted_grp", nr, &sorted_grp));
+        B_CHECK(get_buf(ctx, "sorted_grp" + sfx, nr, &sorted_grp));
         iota_kernel<<<grid_for(ctx, nr, T256), T256, 0, s>>>(riota, nr);
         B_LAUNCHED();
         B_CHECK(cub_sort_pairs(ctx, run_grp, sorted_grp, riota, sorted_runs, nr, L.G));
@@ -596,10 +633,23 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     // the dense small-dim coupling of the CG matvec (block level, one small
     // dim with at most kCoupleMaxSG levels, coupling rows no larger than the
     // run rows): its setup also yields the exact small-dim diagonal
+    // With two large dims the explicit block replaces the pass over the
+    // observations in solves that run in FP64 throughout, wherever its
+    // contributions fit (2M rows, worker/firm/year/occupation, 9 columns: an
+    // iteration of 560 us becomes one of 83).  The FP32 inner solves of the
+    // mixed scheme keep the pass: their answers carry its roundings (R in FP32
+    // per run), up to 1e-7 of a column in badly identified rows.  The pairs are
+    // counted here, since the small dim's diagonal then comes from the coupling.
     const bool block_ok = st.GR > 0 && st.nL <= 1 && st.nS <= 1;
+    int64_t pairs = -1, coupled_rows = st.lrows * st.SG, run_room = 0;
+    for (int l = 0; l < st.nL; ++l) run_room += st.L[l].nruns * 16;
+    const bool couple_fits = st.SG <= kCoupleMaxSG && (st.nL == 0 || coupled_rows <= run_room);
+    if (st.nL == 2 && st.nS <= 1 && ctx->sparse_two && (st.nS == 0 || couple_fits)) {
+        B_CHECK(count_sparse_pairs(ctx, &pairs));
+        st.two_large = pairs >= 0;
+    }
     const bool will_couple =
-        block_ok && ctx->pass_kernel == 0 && st.nS == 1 && st.SG <= kCoupleMaxSG &&
-        (st.nL == 0 || static_cast<int64_t>(st.L[0].G) * st.SG <= st.L[0].nruns * 16);
+        (block_ok && ctx->pass_kernel == 0 && st.nS == 1 && couple_fits) || (st.two_large && st.nS == 1);
 
     // small dims: packed ids and diagonal
     if (st.nS > 0) {
@@ -633,12 +683,13 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
 
     // blocks and packed metadata of the block-level pass
     st.block_ok = block_ok;
-    if (st.block_ok) {
+    if (st.block_ok || will_couple) {
         int32_t *bflags, *bid, *bstart;
         B_CHECK(get_buf(ctx, "tmp_n_a", n, &bflags));
         B_CHECK(get_buf(ctx, "tmp_n_b", n, &bid));
         block_flags_kernel<<<grid_for(ctx, n, T256), T256, 0, s>>>(
-            gp, st.nL == 1 ? st.L[0].rid : nullptr, st.nS == 1 ? st.sid : nullptr, st.wp64, n, bflags);
+            gp, st.nL >= 1 ? st.L[0].rid : nullptr, st.nL == 2 ? st.L[1].rid : nullptr,
+            st.nS == 1 ? st.sid : nullptr, st.wp64, n, bflags);
         B_LAUNCHED();
         B_CHECK(cub_inclusive_sum(ctx, bflags, bid, n));
         int nb = 0;
@@ -656,12 +707,12 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
             bstart, nb, n, st.nS == 1 ? st.sid : nullptr, st.wp64, st.block_meta, st.block_w64,
             st.block_w32);
         B_LAUNCHED();
-        const int64_t npr = st.nL == 1 ? st.L[0].nruns : static_cast<int64_t>(G[p]);
+        const int64_t npr = st.nL >= 1 ? st.L[0].nruns : static_cast<int64_t>(G[p]);
         B_CHECK(get_buf(ctx, "seg_meta", static_cast<size_t>(G[p]) + 1, &st.seg_meta));
         B_CHECK(get_buf(ctx, "run_meta", npr, &st.run_meta));
         B_CHECK(get_buf(ctx, "run_w64", npr, &st.run_w64));
         B_CHECK(get_buf(ctx, "run_w32", npr, &st.run_w32));
-        const bool lg = st.nL == 1;
+        const bool lg = st.nL >= 1;
         pack_meta_kernel<<<grid_for(ctx, std::max<int64_t>(npr, static_cast<int64_t>(G[p]) + 1), T256),
                            T256, 0, s>>>(
             seg_off, lg ? st.L[0].run_base : nullptr, G[p], lg ? st.L[0].run_grp : nullptr,
@@ -677,28 +728,40 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
             st.SGP = static_cast<int>((SG + 3) & ~int64_t(3));
             const int64_t SGP = st.SGP;
             if (lg) {
-                const LargeDim& L = st.L[0];
+                B_CHECK(get_buf(ctx, "cfy64", static_cast<size_t>(st.lrows) * SGP, &st.cfy64));
+                B_CHECK(get_buf(ctx, "cfy32", static_cast<size_t>(st.lrows) * SGP, &st.cfy32));
+            }
+            for (int l = 0; l < st.nL; ++l) {
+                const LargeDim& L = st.L[l];
+                const std::string sfx = std::to_string(l);
+                double* cfy = st.cfy64 + st.lbase[l] * SGP;
+                int2* seg_meta = st.seg_meta;
+                int4* run_meta = st.run_meta;
+                if (l > 0) {  // the second dim's runs over the same blocks
+                    double* rw64;
+                    float* rw32;
+                    B_CHECK(get_buf(ctx, "seg_meta1", static_cast<size_t>(G[p]) + 1, &seg_meta));
+                    B_CHECK(get_buf(ctx, "run_meta1", L.nruns, &run_meta));
+                    B_CHECK(get_buf(ctx, "run_w64_1", L.nruns, &rw64));
+                    B_CHECK(get_buf(ctx, "run_w32_1", L.nruns, &rw32));
+                    pack_meta_kernel<<<grid_for(ctx, std::max<int64_t>(L.nruns, static_cast<int64_t>(G[p]) + 1), T256),
+                                       T256, 0, s>>>(seg_off, L.run_base, G[p], L.run_grp, L.run_dest, L.run_start,
+                                                     L.nruns, L.cw_run, bid, nb, n, seg_meta, run_meta, rw64, rw32);
+                    B_LAUNCHED();
+                }
                 int32_t *sorted_grp, *run_seg, *grp_off;
                 int4* frec;
                 double* frec_cf;
-                B_CHECK(get_buf(ctx, "sorted_grp", L.nruns, &sorted_grp));
+                B_CHECK(get_buf(ctx, "sorted_grp" + sfx, L.nruns, &sorted_grp));
                 B_CHECK(get_buf(ctx, "fy_rec", L.nruns, &frec));
                 B_CHECK(get_buf(ctx, "fy_rec_cf", L.nruns, &frec_cf));
-                B_CHECK(get_buf(ctx, "run_seg", L.nruns, &run_seg));
-                B_CHECK(get_buf(ctx, "grp_off0", static_cast<size_t>(L.G) + 1, &grp_off));
-                // ranges of 512 runs where that gives every resident warp one,
-                // shorter ones on small panels (300k rows: 111 warps of 512 runs
-                // took 210 us)
-                const int64_t per_warp = L.nruns / (static_cast<int64_t>(ctx->num_sms) * 2 * kCoupleWarps);
-                const int range = static_cast<int>(
-                    std::min<int64_t>(kFyRangeRuns, std::max<int64_t>(kFyRangeRunsMin, per_warp / 32 * 32)));
-                const int64_t nranges = (L.nruns + range - 1) / range;
+                B_CHECK(get_buf(ctx, "run_seg" + sfx, L.nruns, &run_seg));
+                B_CHECK(get_buf(ctx, "grp_off" + sfx, static_cast<size_t>(L.G) + 1, &grp_off));
+                const int64_t nranges = (L.nruns + kFyRangeRuns - 1) / kFyRangeRuns;
                 double* cpart;
-                B_CHECK(get_buf(ctx, "cfy64", static_cast<size_t>(L.G) * SGP, &st.cfy64));
-                B_CHECK(get_buf(ctx, "cfy32", static_cast<size_t>(L.G) * SGP, &st.cfy32));
                 B_CHECK(get_buf(ctx, "cfy_part", static_cast<size_t>(std::max<int64_t>(nranges, 1)) * 2 * SGP, &cpart));
                 if (nranges == 0) {
-                    B_TRY(cudaMemsetAsync(st.cfy64, 0, sizeof(double) * static_cast<size_t>(L.G) * SGP, s));
+                    B_TRY(cudaMemsetAsync(cfy, 0, sizeof(double) * static_cast<size_t>(L.G) * SGP, s));
                 } else {
                     const size_t fsmem = static_cast<size_t>(kCoupleWarps) * 32 * couple_pitch(static_cast<int>(SG)) * sizeof(double);
                     B_TRY(raise_smem_limit(reinterpret_cast<const void*>(&coupling_fy_range_kernel), static_cast<int>(fsmem)));
@@ -709,23 +772,34 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                         1, std::min<int64_t>((nranges + kCoupleWarps - 1) / kCoupleWarps,
                                              static_cast<int64_t>(ctx->num_sms) * std::max(fps, 1))));
                     fy_run_record_kernel<<<grid_for(ctx, L.nruns, T256), T256, 0, s>>>(
-                        L.nruns, L.run_dest, run_seg, st.run_meta, st.seg_meta, L.cw_run, st.inv_wp, frec,
+                        L.nruns, L.run_dest, run_seg, run_meta, seg_meta, L.cw_run, st.inv_wp, frec,
                         frec_cf);
                     B_LAUNCHED();
-                    coupling_fy_range_kernel<<<fgrid, kCoupleWarps * 32, fsmem, s>>>(
-                        L.nruns, nranges, range, L.G, frec, frec_cf, sorted_grp, grp_off, st.block_meta,
-                        st.block_w64, st.SG, st.SGP, st.cfy64, cpart);
+                    // a CTA per range where ranges would leave most resident warps without one
+                    const size_t wsmem = fy_wide_smem(static_cast<int>(SG));
+                    if (nranges * 4 <= static_cast<int64_t>(ctx->num_sms) * fps * kCoupleWarps && wsmem <= 200 * 1024) {
+                        B_TRY(raise_smem_limit(reinterpret_cast<const void*>(&coupling_fy_wide_kernel),
+                                               static_cast<int>(wsmem)));
+                        coupling_fy_wide_kernel<<<static_cast<int>(nranges), kFyRangeRuns, wsmem, s>>>(
+                            L.nruns, nranges, L.G, frec, frec_cf, sorted_grp, grp_off, st.block_meta, st.block_w64,
+                            st.SG, st.SGP, cfy, cpart);
+                    } else {
+                        coupling_fy_range_kernel<<<fgrid, kCoupleWarps * 32, fsmem, s>>>(
+                            L.nruns, nranges, L.G, frec, frec_cf, sorted_grp, grp_off, st.block_meta, st.block_w64,
+                            st.SG, st.SGP, cfy, cpart);
+                    }
                     B_LAUNCHED();
                     if (nranges > 1) {
                         coupling_fy_join_kernel<<<static_cast<int>(std::min<int64_t>(
                                                       nranges, static_cast<int64_t>(ctx->num_sms) * 8)),
-                                                  256, 0, s>>>(L.nruns, nranges, range, sorted_grp, grp_off, cpart,
-                                                               st.SGP, st.cfy64);
+                                                  256, 0, s>>>(L.nruns, nranges, sorted_grp, grp_off, cpart,
+                                                               st.SGP, cfy);
                         B_LAUNCHED();
                     }
                 }
-                to_float_kernel<<<grid_for(ctx, static_cast<int64_t>(L.G) * SGP, T256), T256, 0, s>>>(
-                    st.cfy64, static_cast<int64_t>(L.G) * SGP, st.cfy32);
+            }
+            if (lg) {
+                to_float_kernel<<<grid_for(ctx, st.lrows * SGP, T256), T256, 0, s>>>(st.cfy64, st.lrows * SGP, st.cfy32);
                 B_LAUNCHED();
             }
             // C_yy partials: the register-tiled kernel where SG fits one of its
@@ -760,7 +834,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                 B_CHECK(launch_yy(&coupling_yy_kernel, kCoupleYyWarps,
                                   static_cast<size_t>(kCoupleYyWarps) * couple_yy_warp_words(static_cast<int>(SG)) *
                                       sizeof(double)));
-            coupling_yy_reduce_kernel<<<static_cast<int>((SG * SG + 31) / 32), 32 * kYySlices, 0, s>>>(
+            coupling_yy_reduce_kernel<<<static_cast<int>((SG * SG + 31) / 32), 32 * kYyWarps, 0, s>>>(
                 ypart, ny, st.SG, st.cyy, Wall + st.sbase[0], Eall + st.sbase[0]);
             B_LAUNCHED();
         }
@@ -769,7 +843,8 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     // explicit Schur block of the large dim (sparse_kernels.cuh): replaces the
     // per-iteration pass over the runs when the movers' pairs fit
     if (st.block_ok && ctx->sparse_schur && st.nL == 1 && (st.nS == 0 || st.coupled))
-        B_CHECK(build_sparse_block(ctx));
+        B_CHECK(count_sparse_pairs(ctx, &pairs));
+    if (pairs >= 0) B_CHECK(build_sparse_block(ctx, pairs));
 
     B_CHECK(build_stream_meta(ctx));
 
@@ -780,7 +855,9 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                                                                  st.dinv32);
         B_LAUNCHED();
     }
-    // ||D'W||_F^2 = D * sum w^2
+    // ||D'W||_F^2 = D * sum w^2, and what the tile records came to
+    ReadBatch rb;
+    st.sum_w2 = static_cast<double>(n);
     if (w) {
         double *part, *outv;
         unsigned int* ticket;
@@ -791,16 +868,16 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         row_dot_kernel<double, double><<<grid_for(ctx, n, kRowThreads), kRowThreads, 0, s>>>(
             n, 1, w, w, part, ticket, outv);
         B_LAUNCHED();
-        double sw2 = 0.0;
-        B_CHECK(sync_read_double(ctx, outv, 1, &sw2));
-        st.sum_w2 = sw2;
-    } else {
-        st.sum_w2 = static_cast<double>(n);
+        rb.add(outv, sizeof(double), &st.sum_w2);
     }
+    int stream_flags[2] = {1, 0};
+    if (st.stream_flags) rb.add(st.stream_flags, sizeof(stream_flags), stream_flags);
+    B_CHECK(rb.wait(ctx));
+    st.stream_ok = st.stream_flags && stream_flags[0] == 0;
+    st.stream_blob_max = stream_flags[1];
     // levels present per dim (groups with positive weight): primary from
     // segment weights; the others from the diagonal's weight sums.
     for (int d = 0; d < D; ++d) st.present[d] = G[d];
-    B_TRY(cudaStreamSynchronize(s));
     st.valid = true;
     return B200FE_OK;
 }
@@ -846,6 +923,12 @@ struct Work {
     int64_t sp_fin_rows;
     int sp_fin_grid;
 };
+
+// Partial slots of the passes over the regular tiles: the largest grid.
+template <typename T>
+int pass_slots(const Work<T>& wk) {
+    return std::max(std::max(wk.tile_grid, wk.run_grid), wk.data_grid);
+}
 
 template <typename T, int CQ, int MODE>
 int set_pass_smem(b200fe_context* ctx, int tile_smem, int long_smem) {
@@ -902,12 +985,12 @@ int prepare_work(b200fe_context* ctx, const std::string& tag, Work<T>& wk) {
         const int64_t groups = (st.nlong + (32 / CQ) - 1) / (32 / CQ);
         wk.long_grid = grid_for(ctx, groups * 32, kPassThreads, 4);
     }
-    wk.nbins_ctas = std::max(std::max(wk.tile_grid, wk.run_grid), wk.data_grid) + wk.long_grid;
+    wk.nbins_ctas = pass_slots(wk) + wk.long_grid;
     wk.couple_grid = 0;
-    if (st.coupled && wk.run_grid > 0 && st.nL == 1)
+    if (st.coupled && ((wk.run_grid > 0 && st.nL == 1) || st.two_large))
         wk.couple_grid = static_cast<int>(std::max<int64_t>(
             1, std::min<int64_t>({static_cast<int64_t>(wk.nbins_ctas),
-                                  static_cast<int64_t>(ctx->num_sms) * 8, st.L[0].G})));
+                                  static_cast<int64_t>(ctx->num_sms) * 8, st.lrows})));
     B_CHECK(get_buf(ctx, tag + "bins", static_cast<size_t>(wk.nbins_ctas) * std::max(st.SG, 1) * CP,
                     &wk.bins_partial));
     B_CHECK(get_buf(ctx, tag + "colsq", static_cast<size_t>(wk.nbins_ctas) * CP, &wk.colsq_partial));
@@ -1081,7 +1164,7 @@ template <typename T, int CQ, int MODE>
 int launch_pass(b200fe_context* ctx, const Work<T>& wk, PassArgs<T> a) {
     const Structure& st = ctx->st;
     constexpr int CP = 4 * CQ;
-    const int slots = std::max(std::max(wk.tile_grid, wk.run_grid), wk.data_grid);
+    const int slots = pass_slots(wk);
     int used;
     a.bins_cta0 = 0;
     if constexpr (std::is_same<T, double>::value && MODE != kMatvec) {
@@ -1119,7 +1202,7 @@ int launch_matvec_pass(b200fe_context* ctx, const Work<T>& wk, PassArgs<T> a, co
                        const T* block_w) {
     const Structure& st = ctx->st;
     constexpr int CP = 4 * CQ;
-    const int slots = std::max(std::max(wk.tile_grid, wk.run_grid), wk.data_grid);
+    const int slots = pass_slots(wk);
     if (wk.run_grid > 0 && st.coupled) {
         // large dim only over every segment (C_fy' x_f follows in matvec)
         if (st.nL == 1) {
@@ -1385,10 +1468,10 @@ int matvec(b200fe_context* ctx, const Work<T>& wk, const T* wp, const T* run_w,
         if (st.coupled && st.nS == 1) {
             // C_fy' x_f into the coupling partials (read by finalize)
             ProfScope ps(ctx, B200FE_PROF_COUPLE,
-                         static_cast<double>(st.L[0].G) * (st.SGP + CP) * double(sizeof(T)) +
+                         static_cast<double>(st.lrows) * (st.SGP + CP) * double(sizeof(T)) +
                              static_cast<double>(wk.couple_grid) * st.SG * CP * 8.0);
             coupling_xf_kernel<T, CQ><<<wk.couple_grid, 256, 0, ctx->stream>>>(
-                st.L[0].G, st.SG, st.SGP, pick_prec<T>(st.cfy32, st.cfy64), x + st.lbase[0] * CP,
+                st.lrows, st.SG, st.SGP, pick_prec<T>(st.cfy32, st.cfy64), x + st.lbase[0] * CP,
                 wk.bins_partial);
             B_LAUNCHED();
         }
@@ -1600,7 +1683,7 @@ int pcg(b200fe_context* ctx, const Work<T>& wk, const T* wp, const T* run_w, con
 // q, dinv read; x, r, z written; z, p read and p written for the directions).
 double pcg_iter_bytes(const Structure& st, int CP, size_t tsize) {
     const double tb = static_cast<double>(tsize);
-    const double gf = static_cast<double>(st.L[0].G);
+    const double gf = static_cast<double>(st.lrows);
     const double gr = static_cast<double>(st.GR);
     double b = static_cast<double>(st.sp_nnz) * (4.0 + tb) + gf * 4.0 + 2.0 * gf * CP * tb;
     if (st.coupled && st.nS == 1) b += gf * st.SGP * tb;
@@ -1613,12 +1696,13 @@ double pcg_gather_bytes(const Structure& st, int CP, size_t tsize) {
     return (static_cast<double>(st.sp_nnz) + static_cast<double>(st.GR)) * CP * static_cast<double>(tsize);
 }
 
-// Inner PCG as one cooperative launch (pcg_kernels.cuh).  Returns
+// Inner PCG as one launch (pcg_kernels.cuh), not waited for: *ctl_out are two
+// device words {iterations, status} for pcg_outcome.  Returns
 // B200FE_UNAVAILABLE (nothing run) when the launch cannot be made, so the
 // caller falls back to the multi-kernel PCG.
 template <typename T, int CQ>
 int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, T* r, T* p, T* q,
-                   const std::vector<double>& thr_host, int max_iter, int* iters_out) {
+                   const std::vector<double>& thr_host, int max_iter, const int32_t** ctl_out) {
     const Structure& st = ctx->st;
     constexpr int CP = 4 * CQ;
     const cudaStream_t s = ctx->stream;
@@ -1646,7 +1730,7 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     const int nb_max = std::max(kPcgMinCtas, ctx->num_sms);
     PcgArgs<T> a{};
     a.CP = CP;
-    a.Gf = st.L[0].G;
+    a.Gf = st.lrows;
     a.SG = SG;
     a.SGP = SGP;
     a.row_off = st.sp_row_off;
@@ -1733,14 +1817,24 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
             return B200FE_UNAVAILABLE;
         }
         ++ctx->launches;
-        int hc[2] = {0, 0};
-        B_CHECK(sync_read_int(ctx, ctl, 2, hc));
-        if (hc[1] != 0) {
-            ctx->err = "persistent PCG: grid barrier wait timed out";
-            return B200FE_CUDA_ERROR;
-        }
-        *iters_out = hc[0];
-        ps.bytes = static_cast<double>(hc[0]) * pcg_iter_bytes(st, CP, sizeof(T));
+    }
+    *ctl_out = ctl;
+    return B200FE_OK;
+}
+
+// What the words of a finished pcg_persistent say.
+int pcg_outcome(b200fe_context* ctx, const int (&hc)[2], int CP, size_t tsize, int* iters_out) {
+    if (hc[1] != 0) {
+        ctx->err = "persistent PCG: grid barrier wait timed out";
+        return B200FE_CUDA_ERROR;
+    }
+    *iters_out = hc[0];
+    if (ctx->profiling) {  // the bytes of the launch's record, now that its iterations are known
+        for (auto it = ctx->prof.rbegin(); it != ctx->prof.rend(); ++it)
+            if (it->cat == B200FE_PROF_PASS) {
+                it->bytes = static_cast<double>(hc[0]) * pcg_iter_bytes(ctx->st, CP, tsize);
+                break;
+            }
     }
     return B200FE_OK;
 }
@@ -1796,8 +1890,11 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
     Work<double> w64{};
     B_CHECK(prepare_work<double, CQ>(ctx, "w64_", w64));
     const bool mixed = (o.precision == B200FE_PREC_MIXED) && GR > 0;
+    // the inner solves of the mixed scheme run in FP32; in FP64 on a reused
+    // structure that holds the explicit block of two large dims
+    const bool inner32 = mixed && !st.two_large;
     Work<float> w32{};
-    if (mixed) B_CHECK(prepare_work<float, CQ>(ctx, "w32_", w32));
+    if (inner32) B_CHECK(prepare_work<float, CQ>(ctx, "w32_", w32));
 
     double *b64, *a64, *r64, *q64, *z64 = nullptr, *p64 = nullptr, *x64 = nullptr,
            *rin64 = nullptr;
@@ -1806,7 +1903,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
     B_CHECK(get_buf(ctx, "r64", GR * CP, &r64));
     B_CHECK(get_buf(ctx, "q64", GR * CP, &q64));
     float *x32 = nullptr, *r32 = nullptr, *z32 = nullptr, *p32 = nullptr, *q32 = nullptr;
-    if (mixed) {
+    if (inner32) {
         B_CHECK(get_buf(ctx, "x32", GR * CP, &x32));
         B_CHECK(get_buf(ctx, "r32", GR * CP, &r32));
         B_CHECK(get_buf(ctx, "z32", GR * CP, &z32));
@@ -1839,12 +1936,19 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                          runs_write_bytes(st, CP, 8));
         B_CHECK((launch_pass<double, CQ, kRhs>(ctx, w64, a)));
     }
-    std::vector<double> vnorm2(CP, 0.0);
+    std::vector<double> vnorm2(CP, 0.0), bb(CP, 0.0);
     {
         std::vector<double> hp(static_cast<size_t>(w64.nbins_ctas) * CP);
-        if (GR > 0)
+        ReadBatch rb;
+        if (GR > 0) {
             B_CHECK(reduce_runs<double, CQ>(ctx, w64, b64, nullptr, B200FE_PROF_RHS, B200FE_PROF_RHS));
-        B_CHECK(small_d2h(ctx, w64.colsq_partial, sizeof(double) * hp.size(), hp.data()));
+            row_dot_kernel<double, double><<<rgrid, kRowThreads, 0, s>>>(GR, CP, b64, b64, dot_part, dot_ticket,
+                                                                         dot_res);
+            B_LAUNCHED();
+            rb.add(dot_res, sizeof(double) * CP, bb.data());
+        }
+        rb.add(w64.colsq_partial, sizeof(double) * hp.size(), hp.data());
+        B_CHECK(rb.wait(ctx));
         for (int b = 0; b < w64.nbins_ctas; ++b)
             for (int c = 0; c < CP; ++c) vnorm2[c] += hp[static_cast<size_t>(b) * CP + c];
     }
@@ -1854,12 +1958,8 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
     const double* dinv64_use = st.dinv64;  // Jacobi diagonal (scaled by the learned warm start)
     const float* dinv32_use = st.dinv32;
     double rel_res = 0.0;
-    std::vector<double> bb(CP, 0.0), rr(CP, 0.0);
+    std::vector<double> rr(CP, 0.0);
     if (GR > 0) {
-        row_dot_kernel<double, double><<<rgrid, kRowThreads, 0, s>>>(GR, CP, b64, b64, dot_part,
-                                                                     dot_ticket, dot_res);
-        B_LAUNCHED();
-        B_CHECK(sync_read_double(ctx, dot_res, CP, bb.data()));
         B_TRY(cudaMemsetAsync(a64, 0, sizeof(double) * GR * CP, s));
         B_TRY(cudaMemcpyAsync(r64, b64, sizeof(double) * GR * CP, cudaMemcpyDeviceToDevice, s));
         rr = bb;
@@ -1984,13 +2084,13 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
             B_CHECK(small_h2d(ctx, scale_d, scale.data(), sizeof(double) * CP));
             B_CHECK(small_h2d(ctx, inv_scale_d, inv_scale.data(), sizeof(double) * CP));
             int its = 0;
-            if (mixed) {
+            const int32_t* ctl = nullptr;  // words of a persistent inner solve
+            if (inner32) {
                 scale_rows_kernel<float><<<rgrid, kRowThreads, 0, s>>>(GR, CP, r64, inv_scale_d, r32);
                 B_LAUNCHED();
                 int prc = B200FE_UNAVAILABLE;
                 if (st.sparse && ctx->persistent)
-                    prc = pcg_persistent<float, CQ>(ctx, w32, dinv32_use, x32, r32, p32, q32, thr,
-                                                    round_cap, &its);
+                    prc = pcg_persistent<float, CQ>(ctx, w32, dinv32_use, x32, r32, p32, q32, thr, round_cap, &ctl);
                 if (prc == B200FE_UNAVAILABLE)
                     B_CHECK((pcg<float, CQ>(ctx, w32, st.wp32, st.run_w32, st.block_w32, dinv32_use, x32, r32, z32, p32, q32, thr,
                                             round_cap, std::max(1, o.check_interval),
@@ -2004,8 +2104,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                 B_LAUNCHED();
                 int prc = B200FE_UNAVAILABLE;
                 if (st.sparse && ctx->persistent)
-                    prc = pcg_persistent<double, CQ>(ctx, w64, dinv64_use, x64, rin64, p64, q64, thr,
-                                                     round_cap, &its);
+                    prc = pcg_persistent<double, CQ>(ctx, w64, dinv64_use, x64, rin64, p64, q64, thr, round_cap, &ctl);
                 if (prc == B200FE_UNAVAILABLE)
                     B_CHECK((pcg<double, CQ>(ctx, w64, st.wp64, st.run_w64, st.block_w64, dinv64_use, x64, rin64, z64, p64, q64, thr,
                                              round_cap, std::max(1, o.check_interval),
@@ -2015,7 +2114,6 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                 axpy_rows_kernel<double><<<rgrid, kRowThreads, 0, s>>>(GR, CP, x64, scale_d, a64);
                 B_LAUNCHED();
             }
-            total_iters += its;
             // true residual in FP64: r = b - S a
             B_CHECK((matvec<double, CQ>(ctx, w64, st.wp64, st.run_w64, st.block_w64, a64, q64)));
             sub_kernel<<<rgrid, kRowThreads, 0, s>>>(GR * CP, b64, q64, r64);
@@ -2023,7 +2121,15 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
             row_dot_kernel<double, double><<<rgrid, kRowThreads, 0, s>>>(GR, CP, r64, r64, dot_part,
                                                                          dot_ticket, dot_res);
             B_LAUNCHED();
-            B_CHECK(sync_read_double(ctx, dot_res, CP, rr.data()));
+            {
+                int hc[2] = {0, 0};
+                ReadBatch rb;
+                rb.add(dot_res, sizeof(double) * CP, rr.data());
+                if (ctl) rb.add(ctl, sizeof(hc), hc);
+                B_CHECK(rb.wait(ctx));
+                if (ctl) B_CHECK(pcg_outcome(ctx, hc, CP, inner32 ? sizeof(float) : sizeof(double), &its));
+            }
+            total_iters += its;
             if (outer == 0) first_round_its = its;
             if (linf_on && linf_only) {
                 bool worse = false;
@@ -2094,20 +2200,25 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                          (cert ? runs_write_bytes(st, CP, 8) : 0.0));
         B_CHECK((launch_pass<double, CQ, kFinal>(ctx, w64, a)));
     }
-    B_CHECK(check_stream_status(ctx));
     double abs_res = 0.0, abs_rel = 0.0;
+    if (!cert) B_CHECK(check_stream_status(ctx));
     if (cert) {
         std::vector<double> hp(static_cast<size_t>(w64.nbins_ctas) * CP);
         std::vector<double> res2(CP, 0.0);
+        int hs = 0;
+        ReadBatch rb;
         if (GR > 0) {
             B_CHECK(reduce_runs<double, CQ>(ctx, w64, q64, nullptr, B200FE_PROF_FINAL,
                                             B200FE_PROF_FINAL));
             row_dot_kernel<double, double><<<rgrid, kRowThreads, 0, s>>>(GR, CP, q64, q64, dot_part,
                                                                          dot_ticket, dot_res);
             B_LAUNCHED();
-            B_CHECK(sync_read_double(ctx, dot_res, CP, res2.data()));
+            rb.add(dot_res, sizeof(double) * CP, res2.data());
         }
-        B_CHECK(small_d2h(ctx, w64.colsq_partial, sizeof(double) * hp.size(), hp.data()));
+        rb.add(w64.colsq_partial, sizeof(double) * hp.size(), hp.data());
+        if (ctx->stream_status) rb.add(ctx->stream_status, sizeof(int), &hs);
+        B_CHECK(rb.wait(ctx));
+        if (hs != 0) B_CHECK(check_stream_status(ctx));
         for (int b = 0; b < w64.nbins_ctas; ++b)
             for (int c = 0; c < CP; ++c) res2[c] += hp[static_cast<size_t>(b) * CP + c];
         const double opn = std::sqrt(static_cast<double>(st.D) * st.sum_w2);
@@ -2208,6 +2319,7 @@ int absorb_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int co
     // 3: the run-level matvec of the automatic choice, without the explicit block
     ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
     ctx->sparse_schur = o.pass_kernel == 0;
+    ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
     ctx->prof.clear();
     ctx->ev_used = 0;
     if (!reuse) {
@@ -2337,6 +2449,7 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
         B_TRY(cudaEventCreate(&e1));
         ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
         ctx->sparse_schur = o.pass_kernel == 0;
+    ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
         B_TRY(cudaEventRecord(e0, s));
         rc = build_structure(ctx, n, num_dims, dg, G, dw);
         B_TRY(cudaEventRecord(e1, s));

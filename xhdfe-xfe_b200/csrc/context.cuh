@@ -123,6 +123,8 @@ struct Structure {
     // of S_ff over the large dim's levels; the CG matvec then gathers these
     // rows instead of passing over the runs
     bool sparse = false;
+    bool two_large = false;            // ... over two large dims, their rows one after the other
+    int64_t lrows = 0;                 // rows of the large dims
     int64_t sp_pairs = 0;              // contributions before merging
     int64_t sp_nnz = 0;
     int32_t* sp_row_off = nullptr;     // [G_f + 1]
@@ -147,6 +149,7 @@ struct Structure {
     unsigned char* stream_blob = nullptr;  // the records (stream_kernels.cuh: tile_blob_kernel)
     int stream_blob_max = 0;               // largest record (bytes)
     int stream_aux_stride = 0;
+    const int* stream_flags = nullptr;     // device words: a tile exceeds the stage; largest record
 };
 
 constexpr int32_t kChunkRuns = 64;
@@ -190,6 +193,7 @@ struct b200fe_context {
     bool profiling = false;
     int pass_kernel = 0;
     bool sparse_schur = true;  // explicit Schur block of the large dim when it applies
+    bool sparse_two = false;   // ... of two large dims
     std::vector<cudaEvent_t> ev_pool;
     size_t ev_used = 0;
     std::vector<ProfRec> prof;
@@ -466,6 +470,58 @@ inline int small_h2d(b200fe_context* ctx, void* dptr, const void* host, size_t b
     ctx->xin_pos += slot;
     return B200FE_OK;
 }
+
+// Several small reads with one kernel and one wait: a wait costs the round
+// trip and the gap until the next launch arrives, some 15-20 us.
+constexpr int kReadBatchMax = 8;
+struct XferList {
+    const uint32_t* src[kReadBatchMax];
+    uint32_t* dst[kReadBatchMax];
+    int64_t words[kReadBatchMax];
+};
+static __global__ void xfer_list_kernel(const XferList l) {
+    const int i = blockIdx.y;
+    for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < l.words[i];
+         k += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        l.dst[i][k] = l.src[i][k];
+}
+struct ReadBatch {
+    XferList list{};
+    void* host[kReadBatchMax] = {nullptr};
+    size_t bytes[kReadBatchMax] = {0}, off[kReadBatchMax] = {0};
+    int n = 0;
+    size_t pos = 0;
+    // `bytes_` (a multiple of 4) from device memory to host memory at wait()
+    void add(const void* dptr, size_t bytes_, void* host_) {
+        list.src[n] = static_cast<const uint32_t*>(dptr);
+        list.words[n] = static_cast<int64_t>(bytes_ / 4);
+        host[n] = host_;
+        bytes[n] = bytes_;
+        off[n] = pos;
+        pos += (bytes_ + 255) & ~size_t(255);
+        ++n;
+    }
+    int wait(b200fe_context* ctx) {
+        if (n == 0) return B200FE_OK;
+        if (!ctx->h_xout || pos > kXferOutBytes) {
+            for (int i = 0; i < n; ++i)
+                B_TRY(cudaMemcpyAsync(host[i], list.src[i], bytes[i], cudaMemcpyDeviceToHost, ctx->stream));
+            B_TRY(cudaStreamSynchronize(ctx->stream));
+            return B200FE_OK;
+        }
+        int64_t most = 1;
+        for (int i = 0; i < n; ++i) {
+            list.dst[i] = reinterpret_cast<uint32_t*>(ctx->h_xout_dev + off[i]);
+            most = std::max(most, list.words[i]);
+        }
+        const int gx = static_cast<int>(std::min<int64_t>((most + 255) / 256, 64));
+        xfer_list_kernel<<<dim3(gx, n), 256, 0, ctx->stream>>>(list);
+        B_LAUNCHED();
+        B_TRY(cudaStreamSynchronize(ctx->stream));
+        for (int i = 0; i < n; ++i) std::memcpy(host[i], ctx->h_xout + off[i], bytes[i]);
+        return B200FE_OK;
+    }
+};
 
 inline int sync_read_int(b200fe_context* ctx, const int32_t* dptr, int count, int* host) {
     return small_d2h(ctx, dptr, sizeof(int) * count, host);

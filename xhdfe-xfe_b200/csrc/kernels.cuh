@@ -1487,6 +1487,37 @@ struct FinalizeArgs {
 constexpr int kFinFewParts = 16;  // rows with at most this many partials take one lane group
 constexpr int kSuperParts = 64;   // chunk partials per super-chunk
 
+// Super-chunks of the groups of more than kFinFewParts chunks: their number
+// per group, then (from its exclusive scan) their chunk ranges.  The lists are
+// as long as they can get; the ranges past the last are empty.
+__global__ void super_count_kernel(int64_t nmulti, const int32_t* __restrict__ c0, const int32_t* __restrict__ c1,
+                                   int32_t* __restrict__ count) {
+    for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r <= nmulti;
+         r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int32_t np = r < nmulti ? c1[r] - c0[r] : 0;
+        count[r] = np > kFinFewParts ? (np + kSuperParts - 1) / kSuperParts : 0;
+    }
+}
+__global__ void super_fill_kernel(int64_t nmulti, const int32_t* __restrict__ c0, const int32_t* __restrict__ c1,
+                                  const int32_t* __restrict__ off, int64_t nsup, int32_t* __restrict__ s0,
+                                  int32_t* __restrict__ s1, int32_t* __restrict__ sup_c0,
+                                  int32_t* __restrict__ sup_c1) {
+    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t r = i0; r < nmulti; r += step) {
+        const int32_t b = off[r], e = off[r + 1];
+        s0[r] = b;
+        s1[r] = e;
+        for (int32_t k = b; k < e; ++k) {
+            const int32_t c = c0[r] + (k - b) * kSuperParts;
+            sup_c0[k] = c;
+            sup_c1[k] = min(c1[r], c + kSuperParts);
+        }
+    }
+    for (int64_t k = i0; k < nsup; k += step)
+        if (k >= off[nmulti]) sup_c0[k] = sup_c1[k] = 0;
+}
+
 // Super-chunks: one lane group (CP lanes) sums kSuperParts chunk partials of
 // a large group with four interleaved accumulators combined in a fixed order.
 __global__ void __launch_bounds__(kRowThreads)

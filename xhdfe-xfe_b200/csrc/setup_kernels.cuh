@@ -98,6 +98,7 @@ __global__ void run_fill_kernel(const int32_t* __restrict__ flags, const int32_t
             run_start[m] = static_cast<int32_t>(k);
             run_seg[m] = gp[k];
         }
+        if (k == n - 1) run_start[run_id[k]] = static_cast<int32_t>(n);  // [nruns]
     }
 }
 
@@ -199,12 +200,14 @@ __global__ void run_sorted_weights_kernel(const int32_t* __restrict__ sorted_run
 // it starts its primary segment or its large-dim run, when its small-dim
 // level is not the previous obs's level + 1, or when its weight differs.
 __global__ void block_flags_kernel(const int32_t* __restrict__ gp, const int32_t* __restrict__ rid,
-                                   const uint32_t* __restrict__ sid, const double* __restrict__ wp,
+                                   const int32_t* __restrict__ rid1, const uint32_t* __restrict__ sid,
+                                   const double* __restrict__ wp,
                                    int64_t n, int32_t* __restrict__ flags) {
     for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
          k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         bool st = (k == 0) || gp[k] != gp[k - 1];
         if (!st && rid) st = rid[k] != rid[k - 1];
+        if (!st && rid1) st = rid1[k] != rid1[k - 1];
         if (!st && sid) st = (sid[k] & 0xffu) != (sid[k - 1] & 0xffu) + 1u;
         if (!st && wp) st = wp[k] != wp[k - 1];
         flags[k] = st ? 1 : 0;
@@ -383,6 +386,7 @@ __global__ void dinv_kernel(const double* __restrict__ W, const double* __restri
 }
 
 // Column-wise dot of two alpha-row arrays with a last-CTA fixed-order reduce.
+constexpr int kDotAhead = 2048;  // partials read ahead (a multiple of every CP)
 template <typename A, typename B>
 __global__ void __launch_bounds__(kRowThreads)
 row_dot_kernel(int64_t GR, int CP, const A* __restrict__ a, const B* __restrict__ b,
@@ -395,31 +399,40 @@ row_dot_kernel(int64_t GR, int CP, const A* __restrict__ a, const B* __restrict_
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowThreads + threadIdx.x; i < total;
          i += stride)
         s = fma(static_cast<double>(a[i]), static_cast<double>(b[i]), s);
-    // CTA sums by a tree, the CTAs' partials by the whole last CTA (a thread per
-    // column adding them one read at a time took 25-100 us)
-    const int j = threadIdx.x / CP, c = threadIdx.x - j * CP;  // CP is a power of two or 1
-    auto tree = [&](double v) {
-        red[threadIdx.x] = v;
-        __syncthreads();
-        for (int h = kRowThreads / CP / 2; h > 0; h >>= 1) {
-            if (j < h) red[threadIdx.x] += red[threadIdx.x + h * CP];
-            __syncthreads();
-        }
-    };
-    tree(s);
-    if (threadIdx.x < CP) partial[static_cast<int64_t>(blockIdx.x) * CP + threadIdx.x] = red[threadIdx.x];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < CP) {
+        double t = 0.0;
+        for (int k = threadIdx.x; k < kRowThreads; k += CP) t += red[k];
+        partial[static_cast<int64_t>(blockIdx.x) * CP + threadIdx.x] = t;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last) return;
     __threadfence();
+    // the partials one after the other (the refinement's scale factors come from
+    // here: another order of these sums would show, 1e5 times larger, in the
+    // next round's residual), but read ahead by the whole CTA: one dependent
+    // read at a time took 25-100 us
+    __shared__ double ahead[2][kDotAhead];
+    const int total_parts = static_cast<int>(gridDim.x) * CP;
     double t = 0.0;
-#pragma unroll 4
-    for (int bb = j; bb < static_cast<int>(gridDim.x); bb += kRowThreads / CP)
-        t += __ldcg(partial + static_cast<int64_t>(bb) * CP + c);
-    tree(t);
-    if (threadIdx.x < CP) out[threadIdx.x] = red[threadIdx.x];
+    int buf = 0;
+    for (int i = threadIdx.x; i < min(kDotAhead, total_parts); i += kRowThreads) ahead[0][i] = __ldcg(partial + i);
+    __syncthreads();
+    for (int i0 = 0; i0 < total_parts; i0 += kDotAhead, buf ^= 1) {
+        for (int i = threadIdx.x; i < kDotAhead && i0 + kDotAhead + i < total_parts; i += kRowThreads)
+            ahead[buf ^ 1][i] = __ldcg(partial + i0 + kDotAhead + i);
+        if (threadIdx.x < CP) {
+            const int e = min(kDotAhead, total_parts - i0);
+#pragma unroll 8
+            for (int i = threadIdx.x; i < e; i += CP) t += ahead[buf][i];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < CP) out[threadIdx.x] = t;
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
@@ -527,8 +540,7 @@ __host__ __device__ __forceinline__ int couple_pitch(int SG) { return SG | 1; }
 // ids with no runs (between two consecutive firms of the order, or before the
 // first or after the last) get zero rows from the warp that passes them.
 constexpr int kCoupleWarps = 8;
-constexpr int kFyRangeRuns = 512;     // runs per range at most, and at least:
-constexpr int kFyRangeRunsMin = 32;
+constexpr int kFyRangeRuns = 512;
 constexpr int kFyPrefetch = 4;
 
 __device__ __forceinline__ void couple_put_row(double* dst, double a0, double a1, int lane, int SG, int SGP) {
@@ -564,7 +576,7 @@ __global__ void fy_run_record_kernel(int64_t nruns, const int32_t* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kCoupleWarps * 32)
-coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int range, int32_t G, const int4* __restrict__ rec,
+coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int32_t G, const int4* __restrict__ rec,
                          const double* __restrict__ rec_cf, const int32_t* __restrict__ sorted_grp,
                          const int32_t* __restrict__ grp_off, const int2* __restrict__ block_meta,
                          const double* __restrict__ block_w, int SG, int SGP, double* __restrict__ out_fy,
@@ -578,7 +590,7 @@ coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int range, int32_t G, c
     __syncwarp();
     const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kCoupleWarps;
     for (int64_t rg = static_cast<int64_t>(blockIdx.x) * kCoupleWarps + warp; rg < nranges; rg += nwarps) {
-        const int64_t rb = rg * range, re = min(rb + range, nruns);
+        const int64_t rb = rg * kFyRangeRuns, re = min(rb + kFyRangeRuns, nruns);
         int32_t cur = sorted_grp[rb];
         const int32_t prev = rb > 0 ? sorted_grp[rb - 1] : -1;
         if (cur != prev) couple_zero_rows(out_fy, prev + 1, cur, lane, SGP);
@@ -660,23 +672,84 @@ coupling_fy_range_kernel(int64_t nruns, int64_t nranges, int range, int32_t G, c
     }
 }
 
+// The same for small panels, whose ranges are too few for a warp each (300k
+// rows: 111 warps of 512 runs took 210 us): a CTA per range.  Every thread
+// builds the row of one run in shared memory; then the warps share out the
+// firms of the range (by the place of their first run in it), each adding a
+// firm's rows in run order, so that the sums are those of the other form.
+__host__ __device__ __forceinline__ size_t fy_wide_smem(int SG) {
+    return static_cast<size_t>(kFyRangeRuns) * (couple_pitch(SG) * sizeof(double) + sizeof(int32_t));
+}
+__global__ void __launch_bounds__(kFyRangeRuns)
+coupling_fy_wide_kernel(int64_t nruns, int64_t nranges, int32_t G, const int4* __restrict__ rec,
+                        const double* __restrict__ rec_cf, const int32_t* __restrict__ sorted_grp,
+                        const int32_t* __restrict__ grp_off, const int2* __restrict__ block_meta,
+                        const double* __restrict__ block_w, int SG, int SGP, double* __restrict__ out_fy,
+                        double* __restrict__ part) {
+    extern __shared__ double cw_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int SGQ = couple_pitch(SG);
+    double* rows = cw_smem;
+    int32_t* grp = reinterpret_cast<int32_t*>(rows + kFyRangeRuns * SGQ);
+    for (int64_t rg = blockIdx.x; rg < nranges; rg += gridDim.x) {
+        const int64_t rb = rg * kFyRangeRuns, re = min(rb + kFyRangeRuns, nruns);
+        const int nr = static_cast<int>(re - rb);
+        __syncthreads();  // the range before is done with the rows
+        double* myrow = rows + threadIdx.x * SGQ;
+        for (int h = 0; h < SGQ; ++h) myrow[h] = 0.0;
+        if (threadIdx.x < nr) {
+            const int4 rc = rec[rb + threadIdx.x];
+            const double cf = rec_cf[rb + threadIdx.x];
+            grp[threadIdx.x] = sorted_grp[rb + threadIdx.x];
+            for (int bb = rc.z; bb < rc.w; ++bb) couple_row_add(myrow, block_meta[bb], block_w ? block_w[bb] : 1.0);
+#pragma unroll 4
+            for (int bb = rc.x; bb < rc.y; ++bb)
+                couple_row_add(myrow, block_meta[bb], -cf * (block_w ? block_w[bb] : 1.0));
+        }
+        __syncthreads();
+        const int i0 = warp * 32 + lane;
+        const bool start = i0 < nr && (i0 == 0 || grp[i0] != grp[i0 - 1]);
+        unsigned starts = __ballot_sync(0xffffffffu, start);
+        while (starts) {
+            const int i = warp * 32 + __ffs(starts) - 1;
+            starts &= starts - 1;
+            const int32_t f = grp[i];
+            const int32_t prev = i > 0 ? grp[i - 1] : rb > 0 ? sorted_grp[rb - 1] : -1;
+            const int32_t fb = grp_off[f], fe = grp_off[f + 1];
+            if (f != prev) couple_zero_rows(out_fy, static_cast<int64_t>(prev) + 1, f, lane, SGP);
+            const int end = static_cast<int>(min(static_cast<int64_t>(fe), re) - rb);
+            double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 4
+            for (int j = i; j < end; ++j) {
+                if (lane < SG) acc0 += rows[j * SGQ + lane];
+                if (lane + 32 < SG) acc1 += rows[j * SGQ + lane + 32];
+            }
+            double* dst = (fb >= rb && fe <= re) ? out_fy + static_cast<int64_t>(f) * SGP
+                          : (fb < rb)            ? part + (rg * 2 + 0) * SGP
+                                                 : part + (rg * 2 + 1) * SGP;
+            couple_put_row(dst, acc0, acc1, lane, SG, SGP);
+            if (rb + end == nruns) couple_zero_rows(out_fy, static_cast<int64_t>(f) + 1, G, lane, SGP);
+        }
+    }
+}
+
 // Rows of the firms split across ranges: the range holding a firm's first run
 // sees it as its last firm, continuing past the range; its row is slot 1 of that
 // range plus slot 0 of each following range up to the firm's last run, added in
 // range order (warp w sums ranges r + 1 + w, r + 9 + w, ...; the eight warp sums
 // are then added to slot 1 in warp order).  One CTA per range.
 __global__ void __launch_bounds__(256)
-coupling_fy_join_kernel(int64_t nruns, int64_t nranges, int range, const int32_t* __restrict__ sorted_grp,
+coupling_fy_join_kernel(int64_t nruns, int64_t nranges, const int32_t* __restrict__ sorted_grp,
                         const int32_t* __restrict__ grp_off, const double* __restrict__ part, int SGP,
                         double* __restrict__ out_fy) {
     __shared__ double ws[8][kCoupleMaxSG];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t r = blockIdx.x; r < nranges; r += gridDim.x) {
-        const int64_t rb = r * range, re = min(rb + range, nruns);
+        const int64_t rb = r * kFyRangeRuns, re = min(rb + kFyRangeRuns, nruns);
         const int32_t f = sorted_grp[re - 1];
         const int64_t fb = grp_off[f], fe = grp_off[f + 1];
         if (fb < rb || fe <= re) continue;  // uniform over the CTA
-        const int64_t r1 = (fe - 1) / range;
+        const int64_t r1 = (fe - 1) / kFyRangeRuns;
         double acc[2] = {0.0, 0.0};
         for (int64_t q = r + 1 + warp; q <= r1; q += 8) {
 #pragma unroll
@@ -874,43 +947,57 @@ coupling_yy_tile_kernel(int32_t Gp, const int2* __restrict__ seg_meta, const int
         partial[static_cast<int64_t>(blockIdx.x) * (SS + SG) + i] = red[i];
 }
 
-// C_yy = diag(W) - sum_s Y_s Y_s' / W_s from the CTA partials; the level
-// weights W_h and E_h = sum_s Y_s[h]^2 / W_s also go to the diagonal arrays of
-// the Jacobi preconditioner (diag C_yy = W_h - E_h, exact).  A CTA takes 32
-// entries, its warps every kYySlices-th partial, added in warp order (one
-// thread per entry: 47-90 us of dependent reads for 300-444 partials).
-constexpr int kYySlices = 16;
-__global__ void __launch_bounds__(32 * kYySlices)
+// C_yy = diag(W) - sum_s Y_s Y_s' / W_s, CTA partials summed in CTA order; the
+// level weights W_h and E_h = sum_s Y_s[h]^2 / W_s also go to the diagonal
+// arrays of the Jacobi preconditioner (diag C_yy = W_h - E_h, exact).  A CTA
+// takes 32 entries; its warps read kYyRows partials of them at a time into
+// shared memory, one warp adds them in order (a thread per entry reading on
+// its own took 47-90 us for 300-444 partials).
+constexpr int kYyWarps = 16;
+constexpr int kYyRows = 2 * kYyWarps;
+__global__ void __launch_bounds__(32 * kYyWarps)
 coupling_yy_reduce_kernel(const double* __restrict__ partial, int nparts, int SG, double* __restrict__ out_yy,
                           double* __restrict__ W_out, double* __restrict__ E_out) {
-    __shared__ double red[2][kYySlices][32];
+    __shared__ double rows[2][2][kYyRows][32];  // {buffer}{entry, weight of its level}
+    __shared__ double Ws[32];
     const int SS = SG * SG;
-    const int e = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int e = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + e;
     const int h = i / SG, h2 = i - h * SG;
-    const bool diag = i < SS && h == h2;
+    const bool in = i < SS, diag = in && h == h2;
+    auto load = [&](int b0, int buf) {
+#pragma unroll
+        for (int u = 0; u < kYyRows / kYyWarps; ++u) {
+            const int r = w + kYyWarps * u, b = b0 + r;
+            if (b < nparts) {
+                const double* src = partial + static_cast<int64_t>(b) * (SS + SG);
+                if (in) rows[buf][0][r][e] = src[i];
+                if (diag) rows[buf][1][r][e] = src[SS + h];
+            }
+        }
+    };
     double acc = 0.0, W = 0.0;
-    if (i < SS) {
-#pragma unroll 4
-        for (int b = sl; b < nparts; b += kYySlices) acc += partial[static_cast<int64_t>(b) * (SS + SG) + i];
-    }
-    if (diag) {
-#pragma unroll 4
-        for (int b = sl; b < nparts; b += kYySlices) W += partial[static_cast<int64_t>(b) * (SS + SG) + SS + h];
-    }
-    red[0][sl][e] = acc;
-    red[1][sl][e] = W;
+    load(0, 0);
     __syncthreads();
-    if (sl != 0 || i >= SS) return;
-    acc = W = 0.0;
-    for (int k = 0; k < kYySlices; ++k) {
-        acc += red[0][k][e];
-        W += red[1][k][e];
+    for (int b0 = 0, buf = 0; b0 < nparts; b0 += kYyRows, buf ^= 1) {
+        if (b0 + kYyRows < nparts) load(b0 + kYyRows, buf ^ 1);
+        const int n = min(kYyRows, nparts - b0);
+        if (w == 0 && in) {
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) acc += rows[buf][0][r][e];
+        } else if (w == 1 && diag) {
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) W += rows[buf][1][r][e];
+        }
+        __syncthreads();
     }
+    if (w == 1) Ws[e] = W;
+    __syncthreads();
+    if (w != 0 || !in) return;
     if (diag) {
-        W_out[h] = W;
+        W_out[h] = Ws[e];
         E_out[h] = acc;
-        out_yy[i] = W - acc;
+        out_yy[i] = Ws[e] - acc;
     } else {
         out_yy[i] = -acc;
     }

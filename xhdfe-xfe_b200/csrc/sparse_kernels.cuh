@@ -39,29 +39,64 @@ constexpr int kSparseMaxRuns = 64;     // runs per segment the pair build handle
 constexpr int kSparseChunk = 64;       // nonzeros per gather chunk
 constexpr int kSparseMergeSerial = 512;  // contributions one thread merges serially
 
-// Per segment: the number of contributions it emits (u^2 for u >= 2 distinct
-// groups among its runs, else 0).  flag |= 1 when a segment has more runs than
-// kSparseMaxRuns (the caller then keeps the run-level matvec).
-__global__ void sparse_pair_count_kernel(int32_t Gp, const int32_t* __restrict__ run_base,
-                                         const int32_t* __restrict__ run_grp,
-                                         int32_t* __restrict__ count, int32_t* __restrict__ flag,
-                                         unsigned long long* __restrict__ total) {
+// One or two large dims (nd), their rows one after the other (row0 of dim 1 =
+// levels of dim 0).  With two, the block of dims f and g also holds
+//
+//     S_fg = D_f' W D_g - sum_s C_s E_s' / W_s
+//
+// whose first term is the weight that a run of f and a run of g share.  A dim
+// with one distinct group in a segment drops out of that segment: its items'
+// products with everything cancel exactly (C = W_s).
+struct SparseRuns {
+    int nd;
+    const int32_t* run_base[2];
+    const int32_t* run_grp[2];
+    const int32_t* run_start[2];  // read with two dims only
+    const double* run_w[2];
+    int32_t row0[2];
+};
+
+// Per segment: the number of contributions it emits: (sum over the dims with
+// u >= 2 distinct groups of u)^2, and twice the shared pieces of the runs of
+// two such dims.  flag |= 1 when a segment has more runs than kSparseMaxRuns
+// (the caller then keeps the other matvec).
+__global__ void sparse_pair_count_kernel(int32_t Gp, const SparseRuns a, int32_t* __restrict__ count,
+                                         int32_t* __restrict__ flag, unsigned long long* __restrict__ total) {
     unsigned long long mine = 0;
     for (int64_t s = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s < Gp;
          s += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t b = run_base[s], e = run_base[s + 1];
-        int32_t u = 0;
-        if (e - b > kSparseMaxRuns) {
-            atomicOr(flag, 1);
-        } else if (e - b >= 2) {
-            for (int32_t a = b; a < e; ++a) {
-                const int32_t g = run_grp[a];
+        int32_t items = 0, runs = 0, live = 0;
+        for (int d = 0; d < a.nd; ++d) {
+            const int32_t b = a.run_base[d][s], e = a.run_base[d][s + 1];
+            runs += e - b;
+            if (runs > kSparseMaxRuns) break;
+            int32_t u = 0;
+            for (int32_t i = b; i < e; ++i) {
+                const int32_t g = a.run_grp[d][i];
                 bool seen = false;
-                for (int32_t c = b; c < a && !seen; ++c) seen = run_grp[c] == g;
+                for (int32_t c = b; c < i && !seen; ++c) seen = a.run_grp[d][c] == g;
                 u += seen ? 0 : 1;
             }
+            if (u >= 2) {
+                items += u;
+                ++live;
+            }
         }
-        const int32_t cnt = u >= 2 ? u * u : 0;
+        int32_t cnt = items * items;
+        if (runs > kSparseMaxRuns) {
+            atomicOr(flag, 1);
+            cnt = 0;
+        } else if (live == 2) {
+            // shared pieces: one per distinct run start of either dim
+            int32_t i = a.run_base[0][s], j = a.run_base[1][s];
+            const int32_t ie = a.run_base[0][s + 1], je = a.run_base[1][s + 1];
+            while (i < ie && j < je) {
+                const int32_t ei = a.run_start[0][i + 1], ej = a.run_start[1][j + 1];
+                cnt += 2;
+                i += ei <= ej;
+                j += ej <= ei;
+            }
+        }
         count[s] = cnt;
         mine += static_cast<unsigned long long>(cnt);
     }
@@ -71,48 +106,73 @@ __global__ void sparse_pair_count_kernel(int32_t Gp, const int32_t* __restrict__
 }
 
 // Per contributing segment: its distinct groups in order of first appearance,
-// their weights C_i (runs of one group summed in run order), and the u^2
-// contributions at off[s] .. off[s] + u^2, row-major in that order.
-__global__ void sparse_pair_fill_kernel(int32_t Gp, const int32_t* __restrict__ run_base,
-                                        const int32_t* __restrict__ run_grp,
-                                        const double* __restrict__ run_w,
-                                        const double* __restrict__ inv_wp,
-                                        const int32_t* __restrict__ count,
-                                        const int32_t* __restrict__ off, int32_t G,
-                                        unsigned long long* __restrict__ keys,
-                                        double* __restrict__ vals) {
+// dim after dim, their weights C_i (runs of one group summed in run order), and
+// its contributions from off[s] on: the products, row-major in that order,
+// then the shared pieces in observation order.  wp: observation weights or null.
+__global__ void sparse_pair_fill_kernel(int32_t Gp, const SparseRuns a, const double* __restrict__ inv_wp,
+                                        const double* __restrict__ wp, const int32_t* __restrict__ count,
+                                        const int32_t* __restrict__ off, int64_t G,
+                                        unsigned long long* __restrict__ keys, double* __restrict__ vals) {
     for (int64_t s = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s < Gp;
          s += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         if (count[s] == 0) continue;
-        const int32_t b = run_base[s], e = run_base[s + 1];
         int32_t grp[kSparseMaxRuns];
         double cw[kSparseMaxRuns];
-        int u = 0;
-        for (int32_t a = b; a < e; ++a) {
-            const int32_t g = run_grp[a];
-            const double c = run_w[a];
-            int i = 0;
-            while (i < u && grp[i] != g) ++i;
-            if (i == u) {
-                grp[u] = g;
-                cw[u] = c;
-                ++u;
-            } else {
-                cw[i] += c;
+        int u = 0, first = 0, live = 0;  // items; the first of dim 1
+        for (int d = 0; d < a.nd; ++d) {
+            const int32_t b = a.run_base[d][s], e = a.run_base[d][s + 1];
+            const int u0 = u;
+            if (d == 1) first = u;
+            for (int32_t r = b; r < e; ++r) {
+                const int32_t g = a.row0[d] + a.run_grp[d][r];
+                const double c = a.run_w[d][r];
+                int i = u0;
+                while (i < u && grp[i] != g) ++i;
+                if (i == u) {
+                    grp[u] = g;
+                    cw[u] = c;
+                    ++u;
+                } else {
+                    cw[i] += c;
+                }
             }
+            if (u - u0 < 2) u = u0;  // one group only: the dim drops out
+            else ++live;
         }
+        if (a.nd == 1 || u == first) first = u;  // no items of dim 1
         const double iw = inv_wp[s];
         int64_t o = off[s];
         for (int i = 0; i < u; ++i) {
             double others = 0.0;
-            for (int j = 0; j < u; ++j)
+            const int db = i < first ? 0 : first, de = i < first ? first : u;
+            for (int j = db; j < de; ++j)
                 if (j != i) others += cw[j];
-            const unsigned long long row = static_cast<unsigned long long>(grp[i]) *
-                                           static_cast<unsigned long long>(G);
+            const unsigned long long row = static_cast<unsigned long long>(grp[i]) * static_cast<unsigned long long>(G);
             for (int j = 0; j < u; ++j) {
                 keys[o] = row + static_cast<unsigned long long>(grp[j]);
                 vals[o] = (j == i) ? cw[i] * others * iw : -(cw[i] * cw[j]) * iw;
                 ++o;
+            }
+        }
+        if (live == 2) {
+            int32_t i = a.run_base[0][s], j = a.run_base[1][s];
+            const int32_t ie = a.run_base[0][s + 1], je = a.run_base[1][s + 1];
+            int32_t k = a.run_start[0][i];
+            while (i < ie && j < je) {
+                const int32_t ei = a.run_start[0][i + 1], ej = a.run_start[1][j + 1], e = min(ei, ej);
+                double w = static_cast<double>(e - k);
+                if (wp) {
+                    w = 0.0;
+                    for (int32_t q = k; q < e; ++q) w += wp[q];
+                }
+                const unsigned long long f = a.row0[0] + a.run_grp[0][i], g = a.row0[1] + a.run_grp[1][j];
+                keys[o] = f * G + g;
+                vals[o++] = w;
+                keys[o] = g * G + f;
+                vals[o++] = w;
+                k = e;
+                i += ei <= ej;
+                j += ej <= ei;
             }
         }
     }
@@ -130,7 +190,7 @@ __global__ void sparse_key_flags_kernel(const unsigned long long* __restrict__ k
 // row and column.  ustart[nnz] = n is written by the thread of the last key.
 __global__ void sparse_unique_fill_kernel(const unsigned long long* __restrict__ keys, int64_t n,
                                           const int32_t* __restrict__ flags,
-                                          const int32_t* __restrict__ uid, int32_t G,
+                                          const int32_t* __restrict__ uid, int64_t G,
                                           int32_t* __restrict__ ustart, int32_t* __restrict__ urow,
                                           int32_t* __restrict__ ucol) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
