@@ -6,6 +6,7 @@
 // blocks of CG iterations.
 
 #include "context.cuh"
+#include "host_stage.cuh"
 #include "kernels.cuh"
 #include "setup_kernels.cuh"
 #include "ols_kernels.cuh"
@@ -2392,6 +2393,21 @@ int copy_pieces(b200fe_context* ctx, void* dst, const void* src, size_t bytes, c
     return B200FE_OK;
 }
 
+// Whether a call's arrays are copied by the stager: all of them pageable (what
+// the runtime can copy directly, or has to refuse, stays with it), and columns
+// enough to pay for the threads.
+bool stage_columns(int64_t n, int cols, const double* y, const double* X,
+                   const int32_t* const* group_ids, int num_dims, const double* weights, double* y_out, double* X_out,
+                   double* const* fe_out) {
+    if (sizeof(double) * static_cast<size_t>(n) * cols < kStageMinBytes || !pageable(y) || !pageable(y_out))
+        return false;
+    if (cols > 1 && (!pageable(X) || !pageable(X_out))) return false;
+    if (weights && !pageable(weights)) return false;
+    for (int d = 0; d < num_dims; ++d)
+        if (!pageable(group_ids[d]) || (fe_out && !pageable(fe_out[d]))) return false;
+    return true;
+}
+
 int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X, int64_t n, int k,
                           int num_dims, const int32_t* const* group_ids, const int32_t* G,
                           const double* weights, const b200fe_options& o, double* y_out, double* X_out,
@@ -2427,18 +2443,41 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
     cudaEvent_t ev_ids;
     B_TRY(cudaEventCreateWithFlags(&ev_ids, cudaEventDisableTiming));
     B_TRY(cudaEventRecord(h0, sin));
-    for (int d = 0; d < num_dims; ++d)
-        B_CHECK(copy_pieces(ctx, dg[d], group_ids[d], sizeof(int32_t) * n, cudaMemcpyHostToDevice, sin));
-    if (weights) B_CHECK(copy_pieces(ctx, dw, weights, sizeof(double) * n, cudaMemcpyHostToDevice, sin));
-    B_TRY(cudaEventRecord(ev_ids, sin));
+    // pageable columns go through worker threads (host_stage.cuh); group 0 of
+    // the stager are the ids, group 1 + g the columns of group g
+    HostStager stager;
+    const bool staged = stage_columns(n, cols, y, X, group_ids, num_dims, weights, y_out, X_out, nullptr) &&
+                        stager.start(ctx, sin, sout, ngroups + 1);
+    auto copy_in = [&](void* dst, const void* src, size_t bytes, int group) -> int {
+        if (staged) {
+            stager.add_in(dst, src, bytes, group);
+            return B200FE_OK;
+        }
+        return copy_pieces(ctx, dst, src, bytes, cudaMemcpyHostToDevice, sin);
+    };
+    auto close_group = [&](int group, cudaEvent_t ev) -> int {
+        if (staged) stager.close_group(group, ev);
+        else B_TRY(cudaEventRecord(ev, sin));
+        return B200FE_OK;
+    };
+    auto arrived = [&](int group) -> int {  // the group's event is recorded
+        if (staged && !stager.wait_in(group)) {
+            ctx->err = "staged copies in failed";
+            return B200FE_CUDA_ERROR;
+        }
+        return B200FE_OK;
+    };
+    for (int d = 0; d < num_dims; ++d) B_CHECK(copy_in(dg[d], group_ids[d], sizeof(int32_t) * n, 0));
+    if (weights) B_CHECK(copy_in(dw, weights, sizeof(double) * n, 0));
+    B_CHECK(close_group(0, ev_ids));
     for (int g = 0; g < ngroups; ++g) {
         const int c0 = gb[g], c1 = gb[g + 1];
         for (int c = c0; c < c1; ++c)
-            B_CHECK(copy_pieces(ctx, dv + static_cast<int64_t>(c) * n, host_col(c), sizeof(double) * n,
-                                cudaMemcpyHostToDevice, sin));
-        B_TRY(cudaEventRecord(ev_in[g], sin));
+            B_CHECK(copy_in(dv + static_cast<int64_t>(c) * n, host_col(c), sizeof(double) * n, 1 + g));
+        B_CHECK(close_group(1 + g, ev_in[g]));
     }
-    B_TRY(cudaEventRecord(h1, sin));
+    if (!staged) B_TRY(cudaEventRecord(h1, sin));
+    B_CHECK(arrived(0));
     // the FE structure as soon as the ids are in, while the columns arrive
     int rc = B200FE_OK;
     if (!(o.reuse_structure && ctx->st.valid && ctx->st.n == n && ctx->st.D == num_dims &&
@@ -2449,7 +2488,7 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
         B_TRY(cudaEventCreate(&e1));
         ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
         ctx->sparse_schur = o.pass_kernel == 0;
-    ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
+        ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
         B_TRY(cudaEventRecord(e0, s));
         rc = build_structure(ctx, n, num_dims, dg, G, dw);
         B_TRY(cudaEventRecord(e1, s));
@@ -2468,6 +2507,8 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
     bool first_out = true;
     for (int g = 0; g < ngroups && (rc == B200FE_OK || rc == B200FE_NOT_CONVERGED); ++g) {
         const int c0 = gb[g], c1 = gb[g + 1];
+        B_CHECK(arrived(1 + g));
+        if (staged && g == ngroups - 1) B_TRY(cudaEventRecord(h1, sin));
         B_TRY(cudaStreamWaitEvent(s, ev_in[g], 0));
         b200fe_options og = o;
         og.reuse_structure = num_dims > 0 ? 1 : o.reuse_structure;
@@ -2486,9 +2527,11 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
             B_TRY(cudaEventRecord(d0, sout));
             first_out = false;
         }
-        for (int c = c0; c < c1; ++c)
-            B_CHECK(copy_pieces(ctx, out_col(c), dout + static_cast<int64_t>(c) * n, sizeof(double) * n,
-                                cudaMemcpyDeviceToHost, sout));
+        for (int c = c0; c < c1; ++c) {
+            const double* src = dout + static_cast<int64_t>(c) * n;
+            if (staged) stager.add_out(src, out_col(c), sizeof(double) * n);
+            else B_CHECK(copy_pieces(ctx, out_col(c), src, sizeof(double) * n, cudaMemcpyDeviceToHost, sout));
+        }
         // merge
         r->iterations = std::max(r->iterations, rg.iterations);
         r->outer_iterations = std::max(r->outer_iterations, rg.outer_iterations);
@@ -2508,8 +2551,9 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
             r->prof_launches[c] += rg.prof_launches[c];
         }
     }
+    const cudaError_t e0 = stager.finish();
     B_TRY(cudaEventRecord(d1, sout));
-    const cudaError_t e1 = cudaStreamSynchronize(sout);
+    const cudaError_t e1 = e0 != cudaSuccess ? e0 : cudaStreamSynchronize(sout);
     const cudaError_t e2 = cudaStreamSynchronize(sin);
     if (e1 == cudaSuccess && e2 == cudaSuccess && !first_out) {
         r->h2d_ms = elapsed_ms(h0, h1);
@@ -2612,6 +2656,7 @@ void b200fe_context_destroy(b200fe_context* ctx) {
     if (ctx->h_pinned_d) cudaFreeHost(ctx->h_pinned_d);
     if (ctx->h_xout) cudaFreeHost(ctx->h_xout);
     if (ctx->h_xin) cudaFreeHost(ctx->h_xin);
+    if (ctx->stage_pinned) cudaFreeHost(ctx->stage_pinned);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     cudaGetLastError();
     delete ctx;
@@ -2732,13 +2777,32 @@ int b200fe_absorb_fe(b200fe_context* ctx, const double* y, const double* X, int6
         B_TRY(cudaEventCreate(&d0));
         B_TRY(cudaEventCreate(&d1));
         B_TRY(cudaEventRecord(h0, s));
-        for (int d = 0; d < num_dims; ++d)
-            B_TRY(cudaMemcpyAsync(dg[d], group_ids[d], sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-        if (weights) B_TRY(cudaMemcpyAsync(dw, weights, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-        B_TRY(cudaMemcpyAsync(dv, y, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-        if (k > 0)
-            B_TRY(cudaMemcpyAsync(dv + n, X, sizeof(double) * n * k, cudaMemcpyHostToDevice, s));
-        B_TRY(cudaEventRecord(h1, s));
+        HostStager stager;
+        const bool staged = stage_columns(n, cols, y, X, group_ids, num_dims, weights, y_out, X_out, fe_out) &&
+                            stager.start(ctx, s, s, 1);
+        auto copy_in = [&](void* dst, const void* src, size_t bytes) -> int {
+            if (staged) stager.add_in(dst, src, bytes, 0);
+            else B_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+            return B200FE_OK;
+        };
+        auto copy_out = [&](void* dst, const void* src, size_t bytes) -> int {
+            if (staged) stager.add_out(src, dst, bytes);
+            else B_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+            return B200FE_OK;
+        };
+        for (int d = 0; d < num_dims; ++d) B_CHECK(copy_in(dg[d], group_ids[d], sizeof(int32_t) * n));
+        if (weights) B_CHECK(copy_in(dw, weights, sizeof(double) * n));
+        B_CHECK(copy_in(dv, y, sizeof(double) * n));
+        if (k > 0) B_CHECK(copy_in(dv + n, X, sizeof(double) * n * k));
+        if (staged) {
+            stager.close_group(0, h1);
+            if (!stager.wait_in(0)) {
+                ctx->err = "staged copies in failed";
+                return B200FE_CUDA_ERROR;
+            }
+        } else {
+            B_TRY(cudaEventRecord(h1, s));
+        }
         if (fe_out) {
             for (int d = 0; d < num_dims; ++d)
                 B_CHECK(get_buf(ctx, "fe_out" + std::to_string(d), static_cast<size_t>(num_groups[d]) * cols,
@@ -2751,15 +2815,14 @@ int b200fe_absorb_fe(b200fe_context* ctx, const double* y, const double* X, int6
             return rc2;
         }
         B_TRY(cudaEventRecord(d0, s));
-        B_TRY(cudaMemcpyAsync(y_out, dout, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-        if (k > 0)
-            B_TRY(cudaMemcpyAsync(X_out, dout + n, sizeof(double) * n * k, cudaMemcpyDeviceToHost, s));
+        B_CHECK(copy_out(y_out, dout, sizeof(double) * n));
+        if (k > 0) B_CHECK(copy_out(X_out, dout + n, sizeof(double) * n * k));
         if (fe_out) {
             for (int d = 0; d < num_dims; ++d)
-                B_TRY(cudaMemcpyAsync(fe_out[d], ctx->fe_dev[d], sizeof(double) * num_groups[d] * cols,
-                                      cudaMemcpyDeviceToHost, s));
+                B_CHECK(copy_out(fe_out[d], ctx->fe_dev[d], sizeof(double) * num_groups[d] * cols));
             for (double*& q : ctx->fe_dev) q = nullptr;
         }
+        B_TRY(stager.finish());
         B_TRY(cudaEventRecord(d1, s));
         B_TRY(cudaEventSynchronize(d1));
         r->h2d_ms = elapsed_ms(h0, h1);

@@ -213,6 +213,7 @@ struct b200fe_context {
     // overlapped with the solves of other groups; off when B200FE_PIPELINE=0
     bool pipeline = true;
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
+    void* stage_pinned = nullptr;  // slots of the staged copies (host_stage.cuh)
     // FP64 data passes fed by bulk copies (stream_kernels.cuh); off when
     // B200FE_STREAM=0 at context creation.  stream_status is set by a pass
     // whose pipeline wait ran out; stream_smem_set marks the kernels whose
