@@ -26,6 +26,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "mma_f64.cuh"
+
 #include "common_kernels.cuh"
 
 namespace b200fe {
@@ -50,12 +52,6 @@ struct GramArgs {
 };
 
 __host__ __device__ constexpr int gram_tiles(int NB) { return NB * (NB + 1) / 2; }
-
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
 
 // NB column blocks of 8; tile (bi, bj), bi <= bj, in row order of the upper
 // triangle.  Lane (c, k) = (lane / 4, lane % 4) holds column 8 b + c of four of

@@ -4,6 +4,7 @@
 
 #include "context.cuh"
 #include "slope_kernels.cuh"
+#include "slope_space_kernels.cuh"
 #include "common_kernels.cuh"
 
 using namespace b200fe;
@@ -32,6 +33,57 @@ struct GiDev {
     const int32_t* igrp;   // [E]
     const double* scale;   // [n]
 };
+
+// The Schur form in coefficient space (slope_space_kernels.cuh): what its
+// iterations read, set up by slopes_device_impl.
+struct SpaceForm {
+    bool on = false;
+    int L = -1;        // the large dimension; the others of the CG are small
+    int kp = 1, kd = 1;
+    int64_t NL = 0;    // its basis columns
+    int Y = 0, Yp = 0; // the small dims' basis columns, rounded up to 8
+    int64_t runs = 0;
+    int32_t* start = nullptr;
+    SlopeSpace sp{};
+    SlopeDim chunks{};  // chunks of runs of L's groups (grp_ch, part, big)
+    int32_t* big_list = nullptr;
+    int n_big = 0;
+    SlopeWorkerArgs wk{};
+    SlopeFirmArgs fm{};
+    SlopeDenseArgs dn{};
+    double *x = nullptr, *s = nullptr, *t = nullptr, *p = nullptr, *Syy = nullptr;
+};
+
+// Whether the CG dims (all but the primary p) suit the coefficient form: one
+// dimension of any size, the others of at most kSpaceMaxSmall basis columns, and
+// S_Ly no larger than the residual and its image (it is read once an iteration,
+// they four times by the observation passes).  Setting S_Ly up costs Y / C
+// iterations of the observation passes, hence the bound on Y per column: a solve
+// takes 40 to 80.  Lock steps of more columns than a warp's lanes stay with the
+// observation passes.
+bool space_applies(const SlopeDim* dims, const std::vector<int>& cg, int C, int64_t n, SpaceForm& f) {
+    if (C > kSpaceMaxCols || cg.empty()) return false;
+    f.L = cg[0];
+    for (int d : cg)
+        if (dims[d].G > dims[f.L].G) f.L = d;
+    f.NL = static_cast<int64_t>(dims[f.L].G) * dims[f.L].nb;
+    int64_t Y = 0;
+    for (int d : cg)
+        if (d != f.L) Y += static_cast<int64_t>(dims[d].G) * dims[d].nb;
+    if (Y > kSpaceMaxSmall || Y > 16 * C || f.NL * Y > 2 * n * C) return false;
+    f.Y = static_cast<int>(Y);
+    f.Yp = (f.Y + 7) / 8 * 8;
+    return true;
+}
+
+template <int KD>
+void launch_dense(const SlopeDenseArgs& a, int grid, cudaStream_t s) {
+    const int nt = (a.C + 7) / 8;
+    if (nt == 1) slope_dense_kernel<1, KD><<<grid, kSlopeThreads, 0, s>>>(a);
+    else if (nt == 2) slope_dense_kernel<2, KD><<<grid, kSlopeThreads, 0, s>>>(a);
+    else if (nt == 3) slope_dense_kernel<3, KD><<<grid, kSlopeThreads, 0, s>>>(a);
+    else slope_dense_kernel<4, KD><<<grid, kSlopeThreads, 0, s>>>(a);
+}
 
 int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C, int nd,
                        const int32_t* const* d_gids, const int32_t* G,
@@ -293,10 +345,13 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         B_LAUNCHED();
         P.minv = minv_c;
     }
+    SpaceForm sf;
+    sf.on = schur && space_applies(dims, cg, C, n, sf);
     if (schur) {
         for (int d : cg) {
             SlopeDim& D = dims[d];
             const std::string sx = std::to_string(d);
+            const bool keep = sf.on && d == sf.L;  // its runs stay for the solve
             int32_t *flag, *pid, *start, *off;
             double* contrib;
             B_CHECK(get_buf(ctx, "sl_pflag", n, &flag));
@@ -306,7 +361,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             B_CHECK(cub_inclusive_sum(ctx, flag, pid, n));
             int np = 0;
             B_CHECK(sync_read_int(ctx, pid + (n - 1), 1, &np));
-            B_CHECK(get_buf(ctx, "sl_pstart", static_cast<size_t>(np) + 1, &start));
+            B_CHECK(get_buf(ctx, keep ? "sl_xstart" : "sl_pstart", static_cast<size_t>(np) + 1, &start));
             pair_start_kernel<<<grid_for(ctx, n + 1, T), T, 0, s>>>(flag, pid, n, start);
             B_LAUNCHED();
             B_CHECK(get_buf(ctx, "sl_contrib", static_cast<size_t>(np) * 3, &contrib));
@@ -317,7 +372,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             // per group sums of the pair planes: one block per group, fixed order
             int32_t* poff;
             double* csum;
-            B_CHECK(get_buf(ctx, "sl_poff", static_cast<size_t>(D.G) + 1, &poff));
+            B_CHECK(get_buf(ctx, keep ? "sl_xoff" : "sl_poff", static_cast<size_t>(D.G) + 1, &poff));
             B_CHECK(get_buf(ctx, "sl_csum", static_cast<size_t>(D.G) * 3, &csum));
             pair_offsets_kernel<<<grid_for(ctx, static_cast<int64_t>(D.G) + 1, T), T, 0, s>>>(
                 off, pid, D.G, n, np, poff);
@@ -341,6 +396,16 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             schur_block_inverse_kernel<<<gb, T, 0, s>>>(D, cm, csum, const_cast<double*>(D.minv),
                                                         pop);
             B_LAUNCHED();
+            if (keep) {
+                sf.runs = np;
+                sf.start = start;
+                sf.fm.ch_beg = poff;  // replaced by the chunks' below
+                double* blk;
+                B_CHECK(get_buf(ctx, "sl_xblk", static_cast<size_t>(sf.NL) * D.nb, &blk));
+                slope_group_block_kernel<<<grid_for(ctx, D.G, T, 4), T, 0, s>>>(D, cm, blk);
+                B_LAUNCHED();
+                sf.dn.blk = blk;
+            }
         }
     }
     // Schur gather: the primary groups spread over several chunks, and their chunks
@@ -373,6 +438,107 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
                 multi_chunks = list;
                 n_multi_chunks = total;
             }
+        }
+    }
+    // coefficient form: the runs in both orders and their chunks in L's order
+    if (sf.on) {
+        const SlopeDim &P = dims[p], &L = dims[sf.L];
+        sf.kp = P.nb;
+        sf.kd = L.nb;
+        const int K = sf.kp * sf.kd;
+        const int64_t np = sf.runs;
+        const int32_t* poff = sf.fm.ch_beg;
+        double *mom, *mom_p;
+        int32_t *prim, *keys, *ord, *grp, *woff, *most, *nch, *gch;
+        B_CHECK(get_buf(ctx, "sl_xmom", static_cast<size_t>(np) * K, &mom));
+        B_CHECK(get_buf(ctx, "sl_xmomp", static_cast<size_t>(np) * K, &mom_p));
+        B_CHECK(get_buf(ctx, "sl_xprim", np, &prim));
+        B_CHECK(get_buf(ctx, "sl_sorted", n, &keys));
+        B_CHECK(get_buf(ctx, "sl_xord", np, &ord));
+        B_CHECK(get_buf(ctx, "sl_xgrp", np, &grp));
+        B_CHECK(get_buf(ctx, "sl_xwoff", static_cast<size_t>(P.G) + 1, &woff));
+        B_CHECK(get_buf(ctx, "sl_xmost", 1, &most));
+        slope_run_moments_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, P, w, sf.start, np, mom, prim);
+        B_LAUNCHED();
+        B_CHECK(cub_sort_pairs(ctx, prim, keys, iota, ord, np, P.G));
+        segment_offsets_kernel<<<grid_for(ctx, np + 1, T), T, 0, s>>>(keys, np, P.G, woff);
+        B_LAUNCHED();
+        slope_run_order_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, sf.start, ord, np, K, mom, grp, mom_p);
+        B_LAUNCHED();
+        B_TRY(cudaMemsetAsync(most, 0, sizeof(int32_t), s));
+        longest_range_kernel<<<grid_for(ctx, P.G, T, 4), T, 0, s>>>(woff, P.G, most);
+        B_LAUNCHED();
+        B_CHECK(get_buf(ctx, "sl_nch", static_cast<size_t>(L.G) + 1, &nch));
+        B_CHECK(get_buf(ctx, "sl_xgch", static_cast<size_t>(L.G) + 1, &gch));
+        slope_chunk_count_kernel<<<grid_for(ctx, L.G + 1, T), T, 0, s>>>(poff, L.G, nch);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, nch, gch, static_cast<int64_t>(L.G) + 1));
+        int32_t *flag, *idx;
+        B_CHECK(get_buf(ctx, "sl_bflag", L.G, &flag));
+        B_CHECK(get_buf(ctx, "sl_bidx", L.G, &idx));
+        multi_chunk_flags_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(gch, nullptr, L.G, flag, kFinSerialChunks);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, flag, idx, L.G));
+        int h_most = 0, h_nch = 0, h_last[2] = {0, 0};
+        ReadBatch rb;
+        rb.add(most, sizeof(int), &h_most);
+        rb.add(gch + L.G, sizeof(int), &h_nch);
+        rb.add(idx + (L.G - 1), sizeof(int), &h_last[0]);
+        rb.add(flag + (L.G - 1), sizeof(int), &h_last[1]);
+        B_CHECK(rb.wait(ctx));
+        sf.on = h_most <= kSpaceMaxRuns;
+        if (sf.on) {
+            SlopeDim& X = sf.chunks;
+            X.G = L.G;
+            X.nb = L.nb;
+            X.has_a = L.has_a;
+            X.has_b = L.has_b;
+            X.grp_ch = gch;
+            X.nch = h_nch;
+            int32_t *cb, *ce;
+            B_CHECK(get_buf(ctx, "sl_xchb", h_nch, &cb));
+            B_CHECK(get_buf(ctx, "sl_xche", h_nch, &ce));
+            slope_chunk_fill_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(poff, L.G, gch, cb, ce, nullptr);
+            B_LAUNCHED();
+            B_CHECK(get_buf(ctx, "sl_xpart", static_cast<size_t>(h_nch) * L.nb * C, &X.part));
+            sf.n_big = h_last[0] + h_last[1];
+            if (sf.n_big > 0) {
+                B_CHECK(get_buf(ctx, "sl_xblist", sf.n_big, &sf.big_list));
+                compact_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(flag, idx, L.G, sf.big_list);
+                B_LAUNCHED();
+                B_CHECK(get_buf(ctx, "sl_xbig", static_cast<size_t>(sf.NL) * C, &X.big));
+            }
+            // the CG dims' coefficients: L's rows, then the small dims'
+            sf.sp.C = C;
+            sf.sp.RB = RB;
+            int64_t row = 0;
+            for (int pass = 0; pass < 2; ++pass)
+                for (int d : cg) {
+                    if ((d == sf.L) != (pass == 0)) continue;
+                    const int i = sf.sp.nd++;
+                    sf.sp.G[i] = dims[d].G;
+                    sf.sp.nb[i] = dims[d].nb;
+                    sf.sp.has_a[i] = dims[d].has_a;
+                    sf.sp.row0[i] = row;
+                    sf.sp.minv[i] = dims[d].minv;
+                    row += static_cast<int64_t>(dims[d].G) * dims[d].nb;
+                }
+            const size_t cw = static_cast<size_t>(row) * C;
+            B_CHECK(get_buf(ctx, "sl_xx", cw, &sf.x));
+            B_CHECK(get_buf(ctx, "sl_xs", cw, &sf.s));
+            B_CHECK(get_buf(ctx, "sl_xt", cw, &sf.t));
+            B_CHECK(get_buf(ctx, "sl_xp", cw, &sf.p));
+            sf.wk = SlopeWorkerArgs{woff, grp, mom_p, P.minv, P.has_a, P.G, C, sf.p, P.zv};
+            sf.fm = SlopeFirmArgs{cb, ce, h_nch, prim, mom, P.zv, C, X.part};
+            sf.dn.NL = sf.NL;
+            sf.dn.Y = sf.Y;
+            sf.dn.Yp = sf.Yp;
+            sf.dn.C = C;
+            sf.dn.p = sf.p;
+            sf.dn.grp_ch = gch;
+            sf.dn.part = X.part;
+            sf.dn.big = X.big;
+            sf.dn.t = sf.t;
         }
     }
     // ---- input norms and stop thresholds
@@ -567,7 +733,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         sga.Q = Q;
         sga.dpart = pq;
     }
-    auto schur_gather = [&]() -> int {
+    auto schur_gather = [&](const SchurGatherArgs& sga) -> int {
         {
             ProfScope ps(ctx, B200FE_PROF_GATHER, gather_bytes);
             if (CW == 1) {
@@ -608,17 +774,166 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         return B200FE_OK;
     };
 
+    // ---- coefficient form: S_Ly and S_yy, its vectors and its steps
+    SchurGatherArgs sgx = sga;  // the image of the coefficients x
+    SlopeStepArgs sa{};
+    SlopeScalars scal[2] = {};
+    double* ones = nullptr;
+    const int gD = sf.on ? static_cast<int>(std::max<int64_t>(
+                               1, std::min<int64_t>((sf.NL + 63) / 64, 2 * static_cast<int64_t>(ctx->num_sms))))
+                         : 0;
+    auto chunk_sums = [&](int d, int cols, int64_t pitch, double* out) -> int {
+        const SlopeDim& D = dims[d];
+        if (n_big[d] > 0) {
+            slope_big_reduce_kernel<<<grid_for(ctx, static_cast<int64_t>(n_big[d]) * D.nb * C * 32, T, 16), T, 0, s>>>(
+                D, big_list[d], n_big[d], C);
+            B_LAUNCHED();
+        }
+        slope_sums_kernel<<<grid_for(ctx, static_cast<int64_t>(D.G) * D.nb * cols, T), T, 0, s>>>(D, C, cols, pitch,
+                                                                                                  out);
+        B_LAUNCHED();
+        return B200FE_OK;
+    };
+    auto space_dim = [&](int d) {  // index of dim d in sf.sp
+        int i = 0;
+        if (d == sf.L) return 0;
+        for (int e : cg) {
+            if (e != sf.L) ++i;
+            if (e == d) break;
+        }
+        return i;
+    };
+    if (sf.on) {
+        const int64_t rows = sf.NL + sf.Y;
+        for (int i = 0; i < sgx.nd; ++i) sgx.dim[i].p = sf.x + sf.sp.row0[space_dim(cg[i])] * C;
+        double *Sly, *one_buf, *xsc;
+        int* xact;
+        const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
+        B_CHECK(get_buf(ctx, "sl_xly", std::max<size_t>(sly, 1), &Sly));
+        B_CHECK(get_buf(ctx, "sl_xyy", std::max(1, sf.Y * sf.Y), &sf.Syy));
+        B_CHECK(get_buf(ctx, "sl_xone", C, &one_buf));
+        B_CHECK(get_buf(ctx, "sl_xsc", static_cast<size_t>(4) * C, &xsc));
+        B_CHECK(get_buf(ctx, "sl_xact", static_cast<size_t>(2) * C, &xact));
+        const std::vector<double> h1(C, 1.0);
+        B_TRY(cudaMemcpyAsync(one_buf, h1.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
+        ones = one_buf;
+        for (int i = 0; i < 2; ++i) scal[i] = SlopeScalars{xsc + i * C, xsc + (2 + i) * C, xact + i * C};
+        if (sly) B_TRY(cudaMemsetAsync(Sly, 0, sizeof(double) * sly, s));
+        for (int y0 = 0; y0 < sf.Y; y0 += C) {
+            const int cols = std::min(C, sf.Y - y0);
+            if (y0 == 0) B_TRY(cudaMemsetAsync(sf.x, 0, sizeof(double) * sf.NL * C, s));
+            slope_unit_kernel<<<grid_for(ctx, static_cast<int64_t>(sf.Y) * C, T), T, 0, s>>>(sf.x + sf.NL * C, sf.Y, C,
+                                                                                         y0);
+            B_LAUNCHED();
+            B_CHECK(schur_gather(sgx));
+            for (int d : cg) {
+                B_CHECK(segment(d, false, Q));
+                if (d == sf.L) B_CHECK(chunk_sums(d, cols, sf.Yp, Sly + y0));
+                else B_CHECK(chunk_sums(d, cols, sf.Y, sf.Syy + (sf.sp.row0[space_dim(d)] - sf.NL) * sf.Y + y0));
+            }
+        }
+        sf.dn.Sly = Sly;
+        double *dot, *py;
+        B_CHECK(get_buf(ctx, "sl_xdot", static_cast<size_t>(gD) * C, &dot));
+        B_CHECK(get_buf(ctx, "sl_xpy", std::max<size_t>(static_cast<size_t>(gD) * sf.Y * C, 1), &py));
+        sf.dn.dot = dot;
+        sf.dn.part_y = py;
+        sa.sp = sf.sp;
+        sa.NL = sf.NL;
+        sa.Y = sf.Y;
+        sa.thr = d_thr;
+        sa.dot = dot;
+        sa.ndot = gD;
+        sa.p = sf.p;
+        sa.x = sf.x;
+        sa.s = sf.s;
+        sa.t = sf.t;
+        sa.grid = grid_for(ctx, (rows + RB - 1) / RB, 1, 2);
+        sa.done = done;
+        B_CHECK(get_buf(ctx, "sl_xpg", static_cast<size_t>(sa.grid) * C, &sa.part_g));
+    }
+    int side = 0;  // which set of scalars the next step reads
+    auto space_step = [&](bool first) -> int {
+        if (!first) {
+            const double rb = sf.runs * (4.0 + 8.0 * sf.kp * sf.kd);
+            ProfScope ps(ctx, B200FE_PROF_PASS,
+                         2.0 * rb + 8.0 * C * (2.0 * sf.NL + 2.0 * dims[p].G * sf.kp) + 8.0 * sf.NL * sf.Yp);
+            const int gw = grid_for(ctx, (static_cast<int64_t>(dims[p].G) + 32 / C - 1) / (32 / C) * 32, T);
+            const int gf = grid_for(ctx, static_cast<int64_t>(sf.fm.nch) * 32, T);
+            if (sf.kp == 1 && sf.kd == 1) {
+                slope_worker_kernel<1, 1><<<gw, T, 0, s>>>(sf.wk);
+                slope_firm_kernel<1, 1><<<gf, T, 0, s>>>(sf.fm);
+            } else if (sf.kp == 1) {
+                slope_worker_kernel<1, 2><<<gw, T, 0, s>>>(sf.wk);
+                slope_firm_kernel<1, 2><<<gf, T, 0, s>>>(sf.fm);
+            } else if (sf.kd == 1) {
+                slope_worker_kernel<2, 1><<<gw, T, 0, s>>>(sf.wk);
+                slope_firm_kernel<2, 1><<<gf, T, 0, s>>>(sf.fm);
+            } else {
+                slope_worker_kernel<2, 2><<<gw, T, 0, s>>>(sf.wk);
+                slope_firm_kernel<2, 2><<<gf, T, 0, s>>>(sf.fm);
+            }
+            B_LAUNCHED();
+            B_LAUNCHED();
+            if (sf.n_big > 0) {
+                const int64_t warps = static_cast<int64_t>(sf.n_big) * sf.kd * C;
+                slope_big_reduce_kernel<<<grid_for(ctx, warps * 32, T, 16), T, 0, s>>>(sf.chunks, sf.big_list,
+                                                                                        sf.n_big, C);
+                B_LAUNCHED();
+            }
+            if (sf.kd == 1) launch_dense<1>(sf.dn, gD, s);
+            else launch_dense<2>(sf.dn, gD, s);
+            B_LAUNCHED();
+            if (sf.Y > 0) {
+                slope_small_kernel<<<(sf.Y * C + T / 32 - 1) / (T / 32), T, 0, s>>>(
+                    sf.dn.part_y, gD, sf.Syy, sf.p + sf.NL * C, sf.Y, C, sf.t + sf.NL * C);
+                B_LAUNCHED();
+            }
+        }
+        ProfScope ps(ctx, B200FE_PROF_VECTOR, 64.0 * (sf.NL + sf.Y) * C);
+        sa.first = first ? 1 : 0;
+        sa.in = scal[side];
+        sa.out = scal[side ^ 1];
+        slope_space_update_kernel<<<sa.grid, T, 0, s>>>(sa);
+        B_LAUNCHED();
+        slope_space_direction_kernel<<<sa.grid, T, 0, s>>>(sa);
+        B_LAUNCHED();
+        side ^= 1;
+        return B200FE_OK;
+    };
+
     if (schur) B_CHECK(project(R, false));
     B_CHECK(gradient(false, true));
     const int ci = std::max(1, o.check_interval);
     const int max_it = o.max_iter > 0 ? o.max_iter : 10000;
     int it = 0, hd = 0;
     B_CHECK(sync_read_int(ctx, done, 1, &hd));
+    // the residual follows the coefficients, and its gradient decides; what two
+    // more starts from it do not settle is left to the observation passes
+    for (int start = 0; sf.on && start < 3 && !hd && it < max_it; ++start) {
+        for (int d : cg) B_CHECK(chunk_sums(d, C, C, sf.s + sf.sp.row0[space_dim(d)] * C));
+        B_CHECK(space_step(true));
+        int stop = 0;
+        while (!stop && it < max_it) {
+            const int steps = std::min(ci, max_it - it);
+            for (int k = 0; k < steps; ++k) B_CHECK(space_step(false));
+            it += steps;
+            B_CHECK(sync_read_int(ctx, done, 1, &stop));
+        }
+        B_CHECK(schur_gather(sgx));
+        {
+            ProfScope ps(ctx, B200FE_PROF_VECTOR, 24.0 * n * C);
+            slope_update_kernel<<<grid_for(ctx, n * C, T), T, 0, s>>>(R, Q, ones, n, C);
+            B_LAUNCHED();
+        }
+        B_CHECK(gradient(false, true));
+        B_CHECK(sync_read_int(ctx, done, 1, &hd));
+    }
     while (!hd && it < max_it) {
         const int steps = std::min(ci, max_it - it);
         for (int k = 0; k < steps; ++k) {
             if (schur) {
-                B_CHECK(schur_gather());
+                B_CHECK(schur_gather(sga));
             } else {
                 ProfScope ps(ctx, B200FE_PROF_GATHER, gather_bytes);
                 if (ga.nd == 1) slope_gather_kernel<1><<<gG, C * RB, 0, s>>>(ga);
