@@ -1126,8 +1126,15 @@ slope_big_reduce_kernel(const SlopeDim d, const int32_t* __restrict__ groups, in
         const int b = rem / C, c = rem - b * C;
         const int32_t g = groups[i];
         double v = 0.0;
-        for (int32_t j = d.grp_ch[g] + lane; j < d.grp_ch[g + 1]; j += 32)
-            v += d.part[(static_cast<int64_t>(j) * d.nb + b) * C + c];
+        const int32_t e = d.grp_ch[g + 1];
+        for (int32_t j = d.grp_ch[g] + lane; j < e; j += 128) {  // four loads in flight
+            double x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                x[u] = j + 32 * u < e ? d.part[(static_cast<int64_t>(j + 32 * u) * d.nb + b) * C + c] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v += x[u];
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0) d.big[(static_cast<int64_t>(g) * d.nb + b) * C + c] = v;

@@ -17,7 +17,7 @@
 // The passes over the observations took 1,330 us an iteration (4M rows, 13
 // columns, worker + firm##c.tenure + year: Q written, R read and written, both
 // read through a permutation, 2.5 GB) - the runs (900,000) and S_Ly (41 MB) are
-// a tenth of that and stay in L2.
+// a tenth of that and stay in L2: 185 us.
 // The recursion's s can drift from the true gradient by rounding; the caller
 // updates the residual with the image of the accumulated coefficients, takes the
 // gradient of that, and starts again from it where it misses the threshold.
@@ -32,7 +32,9 @@ namespace b200fe {
 constexpr int kSpaceMaxCols = 32;      // columns of a lock step (a warp's lanes)
 constexpr int kSpaceMaxSmall = 64;     // basis columns of the small dims
 constexpr int kSpaceMaxRuns = 512;     // runs of one primary group (one lane slot walks them)
-constexpr int kSpaceRunBatch = 4;      // runs a slot has in flight
+constexpr int kSpaceRunBatch = 4;      // runs a slot has in flight (8: 76 us for 58 in the large dim's pass)
+constexpr int kSpaceSerialChunks = 4;  // more chunks of a group: a warp sums them first
+constexpr int kSpaceGroupBatch = 4;    // groups a thread of the vector updates has in flight
 
 // per pair (j, g) in d's order: mom[q][m * d.nb + f] = sum of w times the primary's
 // basis function m times g's basis function f, and j
@@ -162,7 +164,8 @@ struct SlopeWorkerArgs {
 
 // a_j = M_j^-1 V_j p.  Bound by the latency of the gathers (a group has two or
 // three runs): a lane slot of C lanes per primary group - two groups a warp at 13
-// columns - and kSpaceRunBatch runs in flight.
+// columns - and kSpaceRunBatch runs in flight; 50 us for 400,000 groups, 240 MB
+// out of L2.
 template <int KP, int KD>
 __global__ void __launch_bounds__(kSlopeThreads) slope_worker_kernel(const SlopeWorkerArgs a) {
     const int lane = threadIdx.x & 31;
@@ -217,10 +220,15 @@ struct SlopeFirmArgs {
     double* part;            // [nch][KD][C]
 };
 
+// resident CTAs an SM of slope_firm_kernel (the grid is one wave of them)
+__host__ __device__ constexpr int space_firm_ctas(int kp) { return kp == 1 ? 6 : 4; }
+
 // chunk sums of V_j' a_j over the runs of L's groups: a warp per chunk, a lane
-// slot per run, kSpaceRunBatch runs a slot in flight
+// slot per run, kSpaceRunBatch runs a slot in flight and the next batch's groups
+// read ahead (a chunk of 64 runs is 8 steps: 58 us without, 47 with; a wave of
+// CTAs with the registers for it)
 template <int KP, int KD>
-__global__ void __launch_bounds__(kSlopeThreads) slope_firm_kernel(const SlopeFirmArgs a) {
+__global__ void __launch_bounds__(kSlopeThreads, space_firm_ctas(KP)) slope_firm_kernel(const SlopeFirmArgs a) {
     __shared__ double sred[kSlopeThreads / 32][KD][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int C = a.C, S = 32 / C, slot = lane / C, c = lane - slot * C;
@@ -230,12 +238,22 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_firm_kernel(const SlopeFi
         double v[KD];
 #pragma unroll
         for (int f = 0; f < KD; ++f) v[f] = 0.0;
-        if (slot < S)
+        if (slot < S) {
+            int32_t next[kSpaceRunBatch];
+#pragma unroll
+            for (int u = 0; u < kSpaceRunBatch; ++u) {
+                const int32_t i = b + slot + u * S;
+                next[u] = i < e ? a.primary[i] : -1;
+            }
             for (int32_t i = b + slot; i < e; i += kSpaceRunBatch * S) {
                 int32_t g[kSpaceRunBatch];
                 double x[kSpaceRunBatch][KP];
 #pragma unroll
-                for (int u = 0; u < kSpaceRunBatch; ++u) g[u] = i + u * S < e ? a.primary[i + u * S] : -1;
+                for (int u = 0; u < kSpaceRunBatch; ++u) {
+                    g[u] = next[u];
+                    const int32_t in = i + (kSpaceRunBatch + u) * S;
+                    next[u] = in < e ? a.primary[in] : -1;
+                }
 #pragma unroll
                 for (int u = 0; u < kSpaceRunBatch; ++u)
 #pragma unroll
@@ -251,6 +269,7 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_firm_kernel(const SlopeFi
                             for (int f = 0; f < KD; ++f) v[f] = fma(mr[m * KD + f], x[u][m], v[f]);
                     }
             }
+        }
 #pragma unroll
         for (int f = 0; f < KD; ++f) sred[wid][f][lane] = v[f];
         __syncwarp();
@@ -274,7 +293,7 @@ struct SlopeDenseArgs {
     const double* p;         // [NL + Y][C]
     const int32_t* grp_ch;   // chunks of L's groups in part
     const double* part;      // [nch][KD][C]
-    const double* big;       // groups of more than kFinSerialChunks chunks
+    const double* big;       // groups of more than kSpaceSerialChunks chunks
     double* t;               // [NL][C] out
     double* dot;             // [grid][C] sums of p t
     double* part_y;          // [grid][Y * C] sums of S_Ly' p_L
@@ -284,7 +303,9 @@ struct SlopeDenseArgs {
 // S_Ly' p_L.  A warp takes 8 rows at a time, the two products with S_Ly on the
 // FP64 matrix instruction: the tile of S_Ly is read for the first and again, out
 // of L1, transposed for the second, whose Yp x C sums stay in registers for the
-// whole kernel.  Bound by reading S_Ly (41 MB at 129,000 rows, 36 years).
+// whole kernel.  S_Ly is 41 MB at 129,000 rows, 36 years; 29 us, bound by
+// latency (two CTAs an SM for the registers of the sums).  Groups of 5 to 32
+// chunks summed here, one chunk after the other, kept a few warps busy until 46 us.
 template <int NT, int KD>
 __global__ void __launch_bounds__(kSlopeThreads) slope_dense_kernel(const SlopeDenseArgs a) {
     constexpr int MT = kSpaceMaxSmall / 8;
@@ -312,6 +333,7 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_dense_kernel(const SlopeD
         double u[NT][2];
 #pragma unroll
         for (int j = 0; j < NT; ++j) u[j][0] = u[j][1] = 0.0;
+#pragma unroll 5
         for (int k = 0; k < a.Yp; k += 4) {
             const double s = Sr[q * a.Yp + k + r];
 #pragma unroll
@@ -322,8 +344,7 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_dense_kernel(const SlopeD
             const int64_t g = row / KD;
             const int f = static_cast<int>(row - g * KD);
             const int32_t cb = a.grp_ch[g], ce = a.grp_ch[g + 1];
-            const bool big = ce - cb > kFinSerialChunks;
-            double bl[KD];
+            double v[NT][2], ph[NT][2][KD], bl[KD];
 #pragma unroll
             for (int h = 0; h < KD; ++h) bl[h] = a.blk[row * KD + h];
 #pragma unroll
@@ -331,20 +352,36 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_dense_kernel(const SlopeD
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int c = 8 * j + 2 * r + e;
+                    v[j][e] = 0.0;
+#pragma unroll
+                    for (int h = 0; h < KD; ++h) ph[j][e][h] = c < C ? a.p[(g * KD + h) * C + c] : 0.0;
+                }
+            // the chunks outside, the columns' loads together
+            const bool big = ce - cb > kSpaceSerialChunks;
+            const double* src = big ? a.big + row * C : a.part + (static_cast<int64_t>(cb) * KD + f) * C;
+            const int nc = big ? 1 : ce - cb;
+#pragma unroll 2
+            for (int ch = 0; ch < nc; ++ch, src += KD * C)
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int c = 8 * j + 2 * r + e;
+                        if (c < C) v[j][e] += src[c];
+                    }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int c = 8 * j + 2 * r + e;
                     if (c >= C) continue;
-                    double v = 0.0;
-                    if (big)
-                        v = a.big[row * C + c];
-                    else
-                        for (int32_t ch = cb; ch < ce; ++ch) v += a.part[(static_cast<int64_t>(ch) * KD + f) * C + c];
                     double own = 0.0, pr = 0.0;
 #pragma unroll
                     for (int h = 0; h < KD; ++h) {
-                        const double ph = a.p[(g * KD + h) * C + c];
-                        own = fma(bl[h], ph, own);
-                        if (h == f) pr = ph;
+                        own = fma(bl[h], ph[j][e][h], own);
+                        if (h == f) pr = ph[j][e][h];
                     }
-                    const double t = (own - v) + u[j][e];
+                    const double t = (own - v[j][e]) + u[j][e];
                     a.t[row * C + c] = t;
                     dot[j][e] = fma(pr, t, dot[j][e]);
                 }
@@ -437,24 +474,116 @@ struct SlopeStepArgs {
     int* done;
 };
 
-__device__ __forceinline__ void space_zv(const SlopeSpace& sp, int i, int64_t g, double sa, double sb, double& za,
-                                         double& zb) {
-    const double* m = sp.minv[i] + g * 3;
-    if (sp.nb[i] == 2) {
-        za = fma(m[0], sa, m[1] * sb);
-        zb = fma(m[1], sa, m[2] * sb);
-    } else {
-        za = (sp.has_a[i] ? m[0] : m[2]) * sa;
-        zb = 0.0;
+// out[c] = sum over b of part[b * C + c]: thread (column, row) takes every RB-th
+// partial, eight loads in flight, then the rows in order.  All threads call it.
+__device__ __forceinline__ void block_column_sums(const double* __restrict__ part, int nparts, int C, int RB,
+                                                  double* red, double* out) {
+    const int col = threadIdx.x % C, rr = threadIdx.x / C;
+    double s = 0.0;
+    if (rr < RB)
+        for (int b = rr; b < nparts; b += 8 * RB) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = b + u * RB < nparts ? part[static_cast<int64_t>(b + u * RB) * C + col] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+    column_reduce(red, s, C, RB, out);
+}
+
+// s -= alpha t and the sum of s' M^-1 s over the groups of one dim, column `col`
+template <int NB>
+__device__ __forceinline__ double space_update(const SlopeStepArgs& a, int i, int rr, int col, double alpha) {
+    constexpr int U = kSpaceGroupBatch;
+    const int C = a.sp.C;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * a.sp.RB;
+    double acc = 0.0;
+    for (int64_t g0 = static_cast<int64_t>(blockIdx.x) * a.sp.RB + rr; g0 < a.sp.G[i]; g0 += U * stride) {
+        double s[U][NB], t[U][NB], m[U][3];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t g = g0 + u * stride, o = (a.sp.row0[i] + g * NB) * C + col;
+            const bool in = g < a.sp.G[i];
+#pragma unroll
+            for (int h = 0; h < 3; ++h) m[u][h] = in ? a.sp.minv[i][g * 3 + h] : 0.0;
+#pragma unroll
+            for (int f = 0; f < NB; ++f) {
+                s[u][f] = in ? a.s[o + f * C] : 0.0;
+                t[u][f] = in && !a.first ? a.t[o + f * C] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t g = g0 + u * stride, o = (a.sp.row0[i] + g * NB) * C + col;
+            if (g >= a.sp.G[i]) break;
+#pragma unroll
+            for (int f = 0; f < NB; ++f) {
+                s[u][f] = fma(-alpha, t[u][f], s[u][f]);
+                if (!a.first) a.s[o + f * C] = s[u][f];
+            }
+            if (NB == 2) {
+                const double za = fma(m[u][0], s[u][0], m[u][1] * s[u][NB - 1]);
+                const double zb = fma(m[u][1], s[u][0], m[u][2] * s[u][NB - 1]);
+                acc = fma(s[u][0], za, fma(s[u][NB - 1], zb, acc));
+            } else {
+                acc = fma(s[u][0], (a.sp.has_a[i] ? m[u][0] : m[u][2]) * s[u][0], acc);
+            }
+        }
+    }
+    return acc;
+}
+
+// x += alpha p, p = M^-1 s + beta p over the groups of one dim
+template <int NB>
+__device__ __forceinline__ void space_direction(const SlopeStepArgs& a, int i, int rr, int col, double alpha,
+                                                double beta) {
+    constexpr int U = kSpaceGroupBatch;
+    const int C = a.sp.C;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * a.sp.RB;
+    for (int64_t g0 = static_cast<int64_t>(blockIdx.x) * a.sp.RB + rr; g0 < a.sp.G[i]; g0 += U * stride) {
+        double s[U][NB], p[U][NB], x[U][NB], m[U][3];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t g = g0 + u * stride, o = (a.sp.row0[i] + g * NB) * C + col;
+            const bool in = g < a.sp.G[i];
+#pragma unroll
+            for (int h = 0; h < 3; ++h) m[u][h] = in ? a.sp.minv[i][g * 3 + h] : 0.0;
+#pragma unroll
+            for (int f = 0; f < NB; ++f) {
+                s[u][f] = in ? a.s[o + f * C] : 0.0;
+                p[u][f] = in && !a.first ? a.p[o + f * C] : 0.0;
+                x[u][f] = in && !a.first ? a.x[o + f * C] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t g = g0 + u * stride, o = (a.sp.row0[i] + g * NB) * C + col;
+            if (g >= a.sp.G[i]) break;
+            double z[NB];
+            if (NB == 2) {
+                z[0] = fma(m[u][0], s[u][0], m[u][1] * s[u][NB - 1]);
+                z[NB - 1] = fma(m[u][1], s[u][0], m[u][2] * s[u][NB - 1]);
+            } else {
+                z[0] = (a.sp.has_a[i] ? m[u][0] : m[u][2]) * s[u][0];
+            }
+#pragma unroll
+            for (int f = 0; f < NB; ++f) {
+                a.x[o + f * C] = fma(alpha, p[u][f], x[u][f]);
+                a.p[o + f * C] = fma(beta, p[u][f], z[f]);
+            }
+        }
     }
 }
 
 // alpha = gamma / p't, s -= alpha t, partials of gamma = s' M^-1 s.  Every CTA
 // sums the dot partials itself (a few hundred): cheaper than a launch for it.
+// Bound by latency, hence two CTAs an SM (few partials) with kSpaceGroupBatch
+// groups a thread in flight: 11 us, 35 with one at a time (129,000 x 13).
 __global__ void __launch_bounds__(kSlopeThreads) slope_space_update_kernel(const SlopeStepArgs a) {
     __shared__ double red[kSlopeThreads];
-    __shared__ double al[kSpaceMaxCols];
-    const int C = a.sp.C, lane = threadIdx.x & 31;
+    __shared__ double dl[kSpaceMaxCols], al[kSpaceMaxCols];
+    const int C = a.sp.C, RB = a.sp.RB, lane = threadIdx.x & 31;
+    if (!a.first) block_column_sums(a.dot, a.ndot, C, RB, red, dl);
     for (int c = threadIdx.x >> 5; c < C; c += kSlopeThreads / 32) {
         double alpha = 0.0;
         if (!a.first) {
@@ -462,7 +591,7 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_space_update_kernel(const
             for (int y = lane; y < a.Y; y += 32) v = fma(a.p[(a.NL + y) * C + c], a.t[(a.NL + y) * C + c], v);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            v += warp_column_sum(a.dot, a.ndot, C, c);
+            v += dl[c];
             alpha = a.in.active[c] && v > 0.0 ? a.in.gamma[c] / v : 0.0;
         }
         if (lane == 0) {
@@ -473,81 +602,39 @@ __global__ void __launch_bounds__(kSlopeThreads) slope_space_update_kernel(const
     __syncthreads();
     const int col = threadIdx.x % C, rr = threadIdx.x / C;
     double acc = 0.0;
-    if (rr < a.sp.RB) {
-        const double alpha = al[col];
+    if (rr < RB)
         for (int i = 0; i < a.sp.nd; ++i)
-            for (int64_t g = static_cast<int64_t>(blockIdx.x) * a.sp.RB + rr; g < a.sp.G[i];
-                 g += static_cast<int64_t>(gridDim.x) * a.sp.RB) {
-                const int64_t o = (a.sp.row0[i] + g * a.sp.nb[i]) * C + col;
-                double sa = a.s[o], sb = a.sp.nb[i] == 2 ? a.s[o + C] : 0.0, za, zb;
-                if (!a.first) {
-                    sa = fma(-alpha, a.t[o], sa);
-                    a.s[o] = sa;
-                    if (a.sp.nb[i] == 2) {
-                        sb = fma(-alpha, a.t[o + C], sb);
-                        a.s[o + C] = sb;
-                    }
-                }
-                space_zv(a.sp, i, g, sa, sb, za, zb);
-                acc = fma(sa, za, fma(sb, zb, acc));
-            }
-    }
-    column_reduce(red, acc, C, a.sp.RB, a.part_g + static_cast<int64_t>(blockIdx.x) * C);
+            acc += a.sp.nb[i] == 2 ? space_update<2>(a, i, rr, col, al[col]) : space_update<1>(a, i, rr, col, al[col]);
+    column_reduce(red, acc, C, RB, a.part_g + static_cast<int64_t>(blockIdx.x) * C);
 }
 
 // x += alpha p, beta, p = M^-1 s + beta p, the stop test
 __global__ void __launch_bounds__(kSlopeThreads) slope_space_direction_kernel(const SlopeStepArgs a) {
-    __shared__ double be[kSpaceMaxCols], al[kSpaceMaxCols];
-    __shared__ int act[kSpaceMaxCols];
-    const int C = a.sp.C, lane = threadIdx.x & 31;
-    for (int c = threadIdx.x >> 5; c < C; c += kSlopeThreads / 32) {
-        const double g = warp_column_sum(a.part_g, a.grid, C, c);
-        if (lane == 0) {
-            const double old = a.in.gamma[c];
-            const int was = a.first ? 1 : a.in.active[c];
-            al[c] = a.in.alpha[c];
-            be[c] = !a.first && was && old > 0.0 ? g / old : 0.0;
-            act[c] = was && g > a.thr[c];
-            if (blockIdx.x == 0) {
-                a.out.gamma[c] = was ? g : old;
-                a.out.active[c] = act[c];
-            }
+    __shared__ double red[kSlopeThreads];
+    __shared__ double gm[kSpaceMaxCols], be[kSpaceMaxCols], al[kSpaceMaxCols];
+    const int C = a.sp.C, RB = a.sp.RB;
+    block_column_sums(a.part_g, a.grid, C, RB, red, gm);
+    int go = 0;
+    if (static_cast<int>(threadIdx.x) < C) {
+        const int c = threadIdx.x;
+        const double g = gm[c], old = a.in.gamma[c];
+        const int was = a.first ? 1 : a.in.active[c];
+        go = was && g > a.thr[c];
+        al[c] = a.in.alpha[c];
+        be[c] = !a.first && was && old > 0.0 ? g / old : 0.0;
+        if (blockIdx.x == 0) {
+            a.out.gamma[c] = was ? g : old;
+            a.out.active[c] = go;
         }
     }
-    __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int any = 0;
-        for (int c = 0; c < C; ++c) any |= act[c];
-        *a.done = any ? 0 : 1;
-    }
+    go = __syncthreads_or(go);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.done = go ? 0 : 1;
     const int col = threadIdx.x % C, rr = threadIdx.x / C;
-    if (rr >= a.sp.RB) return;
-    const double alpha = al[col], beta = be[col];
-    for (int i = 0; i < a.sp.nd; ++i)
-        for (int64_t g = static_cast<int64_t>(blockIdx.x) * a.sp.RB + rr; g < a.sp.G[i];
-             g += static_cast<int64_t>(gridDim.x) * a.sp.RB) {
-            const int64_t o = (a.sp.row0[i] + g * a.sp.nb[i]) * C + col;
-            const bool two = a.sp.nb[i] == 2;
-            double za, zb;
-            space_zv(a.sp, i, g, a.s[o], two ? a.s[o + C] : 0.0, za, zb);
-            if (a.first) {
-                a.x[o] = 0.0;
-                a.p[o] = za;
-                if (two) {
-                    a.x[o + C] = 0.0;
-                    a.p[o + C] = zb;
-                }
-            } else {
-                const double pa = a.p[o];
-                a.x[o] = fma(alpha, pa, a.x[o]);
-                a.p[o] = fma(beta, pa, za);
-                if (two) {
-                    const double pb = a.p[o + C];
-                    a.x[o + C] = fma(alpha, pb, a.x[o + C]);
-                    a.p[o + C] = fma(beta, pb, zb);
-                }
-            }
-        }
+    if (rr >= RB) return;
+    for (int i = 0; i < a.sp.nd; ++i) {
+        if (a.sp.nb[i] == 2) space_direction<2>(a, i, rr, col, al[col], be[col]);
+        else space_direction<1>(a, i, rr, col, al[col], be[col]);
+    }
 }
 
 }  // namespace b200fe

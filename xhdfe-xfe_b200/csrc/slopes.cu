@@ -476,7 +476,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         int32_t *flag, *idx;
         B_CHECK(get_buf(ctx, "sl_bflag", L.G, &flag));
         B_CHECK(get_buf(ctx, "sl_bidx", L.G, &idx));
-        multi_chunk_flags_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(gch, nullptr, L.G, flag, kFinSerialChunks);
+        multi_chunk_flags_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(gch, nullptr, L.G, flag, kSpaceSerialChunks);
         B_LAUNCHED();
         B_CHECK(cub_exclusive_sum(ctx, flag, idx, L.G));
         int h_most = 0, h_nch = 0, h_last[2] = {0, 0};
@@ -859,7 +859,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             ProfScope ps(ctx, B200FE_PROF_PASS,
                          2.0 * rb + 8.0 * C * (2.0 * sf.NL + 2.0 * dims[p].G * sf.kp) + 8.0 * sf.NL * sf.Yp);
             const int gw = grid_for(ctx, (static_cast<int64_t>(dims[p].G) + 32 / C - 1) / (32 / C) * 32, T);
-            const int gf = grid_for(ctx, static_cast<int64_t>(sf.fm.nch) * 32, T);
+            const int gf = grid_for(ctx, static_cast<int64_t>(sf.fm.nch) * 32, T, space_firm_ctas(sf.kp));
             if (sf.kp == 1 && sf.kd == 1) {
                 slope_worker_kernel<1, 1><<<gw, T, 0, s>>>(sf.wk);
                 slope_firm_kernel<1, 1><<<gf, T, 0, s>>>(sf.fm);
