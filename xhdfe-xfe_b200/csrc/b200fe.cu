@@ -1110,18 +1110,15 @@ int launch_stream_pass(b200fe_context* ctx, const PassArgs<double>& a, int* grid
     const int bins_bytes = std::max(a.SG, 1) * 16 * 8;
     const int red_bytes = kStreamWarps * 16 * 8;
     const int yt_bytes = (MODE == kFinal && a.nS > 0) ? a.SG * 16 * 8 : 0;
-    const int afb_bytes = (MODE == kFinal && a.nL == 1) ? kStreamWarps * kStreamRunRows * 16 * 8 : 0;
     int budget = 0;
     B_TRY(cudaDeviceGetAttribute(&budget, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    const int ns = std::min(kStreamMaxStages, (budget - L.off_stages - bins_bytes - red_bytes - yt_bytes - afb_bytes) /
-                                                  L.stage_bytes);
+    const int ns = std::min(kStreamMaxStages, (budget - L.off_stages - bins_bytes - red_bytes - yt_bytes) / L.stage_bytes);
     if (ns < 2) return B200FE_OK;
     L.NS = ns;
     L.off_bins = L.off_stages + ns * L.stage_bytes;
     L.off_red = L.off_bins + bins_bytes;
     L.off_yt = L.off_red + red_bytes;
-    L.off_afb = L.off_yt + yt_bytes;
-    const int smem = L.off_afb + afb_bytes;
+    const int smem = L.off_yt + yt_bytes;
     L.tmeta = st.stream_meta;
     L.nreg = st.stream_nreg;
     L.boff = st.stream_boff;
@@ -1132,8 +1129,14 @@ int launch_stream_pass(b200fe_context* ctx, const PassArgs<double>& a, int* grid
         B_TRY(cudaMemsetAsync(ctx->stream_status, 0, 4 * sizeof(int), ctx->stream));
     }
     L.status = ctx->stream_status;
-    auto kern = weighted ? stream_pass_kernel<MODE, true> : stream_pass_kernel<MODE, false>;
-    const unsigned bit = 1u << (2 * (MODE == kFinal ? 1 : 0) + (weighted ? 1 : 0));
+    // one large dim with up to one small one (worker, firm and year): the dims
+    // known at compile time
+    const int form = a.nL == 1 && a.nS <= 1 ? a.nS : 2;
+    auto kern = form == 0   ? (weighted ? stream_pass_kernel<MODE, true, 1, 0> : stream_pass_kernel<MODE, false, 1, 0>)
+                : form == 1 ? (weighted ? stream_pass_kernel<MODE, true, 1, 1> : stream_pass_kernel<MODE, false, 1, 1>)
+                            : (weighted ? stream_pass_kernel<MODE, true, -1, -1>
+                                        : stream_pass_kernel<MODE, false, -1, -1>);
+    const unsigned bit = 1u << (4 * form + 2 * (MODE == kFinal ? 1 : 0) + (weighted ? 1 : 0));
     if (!(ctx->stream_smem_set & bit)) {
         B_TRY(raise_smem_limit(reinterpret_cast<const void*>(kern), budget));
         ctx->stream_smem_set |= bit;

@@ -26,9 +26,17 @@
 //   2. one tile later (after all warps are through step 1 of that tile, a
 //      per-stage mbarrier that has normally completed by then), sums z over
 //      the buckets of equal small-dim level (half-warp group g takes levels
-//      g, g + 32, ...), each bucket a run of the tile's sorted order, into
+//      g, g + 2 kStreamWarps, ...), each bucket a run of the tile's sorted order, into
 //      the CTA's bins, so no two groups ever add to the same bin.
 // Every reduction has a fixed order, so results do not depend on timing.
+//
+// Bound by instruction issue and fixed latencies in the short loops over a run
+// (four observations), far from the memory's rate: 5M rows, 13 columns, 36 years
+// take 331 us (kRhs, 0.52 GB) and 587 us (kFinal, 1.04 GB); weighted 351 and 630.
+// What counts: the dims known at compile time (860 -> 612 us in kFinal), loops
+// over a run left rolled (418 -> 395 in kRhs), 24 consumer warps for 16 (372 ->
+// 331), and four stages: with three a weighted kFinal took 1,027 us, so the rows
+// of dim 0 stay in registers.
 // Outputs are those of data_pass_kernel (kernels.cuh) in the same modes.
 
 #pragma once
@@ -41,16 +49,16 @@
 namespace b200fe {
 
 #ifndef B200FE_STREAM_WARPS
-#define B200FE_STREAM_WARPS 16
+#define B200FE_STREAM_WARPS 24
 #endif
-constexpr int kStreamWarps = B200FE_STREAM_WARPS;        // consumer warps per CTA
+constexpr int kStreamWarps = B200FE_STREAM_WARPS;        // consumer warps per CTA (80 registers a thread)
 constexpr int kStreamThreads = (kStreamWarps + 1) * 32;  // + the producer warp
 constexpr int kStreamMaxStages = 4;
 constexpr int kStreamPitchD = kTileObs + 2;   // doubles per staged column (span of <= kTileObs - 1 obs)
 constexpr int kStreamPitchI = kTileObs + 8;   // 4-byte words per staged int array
 constexpr int kStreamHeader = 64;             // tile record at the start of every stage
 constexpr int kStreamGather = 8;              // observations per half-warp and batch of the kFinal gather
-constexpr int kStreamRunRows = 8;             // rows of dim 0 a consumer warp holds (kFinal, one large dim)
+constexpr int kStreamRunRows = 4;             // rows of dim 0 a lane holds, and has in flight (kFinal, one large dim)
 constexpr long long kStreamWaitCycles = 4000000000LL;  // bound of every mbarrier wait
 static_assert(kStreamPitchD % 2 == 0 && kStreamPitchI % 4 == 0, "16-byte rows");
 
@@ -125,7 +133,6 @@ struct StreamLayout {
     int off_cols, off_blob, off_wp, off_sid;
     int off_rid[kMaxLarge];
     int off_yt;             // kFinal: small-dim rows of a [SG][16]
-    int off_afb;            // kFinal, one large dim: rows of dim 0 [kStreamWarps][kStreamRunRows][16]
     int off_stages;         // first stage from the start of shared memory
     int off_bins;           // bins [SG][16]
     int off_red;            // column-sum reduction [kStreamWarps][16]
@@ -219,10 +226,13 @@ __device__ __forceinline__ void span_of(const void* base, int64_t i0, int64_t cn
     *bytes = cnt > 0 ? static_cast<uint32_t>(a1 - a0) : 0u;
 }
 
-template <int MODE, bool WEIGHTED>
+// KL large and KS small dims, both known to the compiler (the common forms), or
+// -1, -1: taken from the arguments.
+template <int MODE, bool WEIGHTED, int KL, int KS>
 __global__ void __launch_bounds__(kStreamThreads, 1)
 stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
     constexpr unsigned kFull = 0xffffffffu;
+    const int nL = KL >= 0 ? KL : a.nL, nS = KS >= 0 ? KS : a.nS;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + kStreamMaxStages;
@@ -234,7 +244,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
     const int lane = threadIdx.x & 31;
     const int NS = L.NS;
     const bool scatter = (MODE == kRhs) || a.scatter;
-    const bool buckets = scatter && a.nS > 0;
+    const bool buckets = scatter && nS > 0;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; ++i) {
@@ -245,9 +255,9 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         *abort_flag = 0;
         mbar_fence_init();
     }
-    if (a.nS > 0)
+    if (nS > 0)
         for (int i = threadIdx.x; i < a.SG * 16; i += kStreamThreads) bins[i] = 0.0;
-    if (MODE == kFinal && a.nS > 0) {
+    if (MODE == kFinal && nS > 0) {
         double* yt = reinterpret_cast<double*>(smem + L.off_yt);
         for (int i = threadIdx.x; i < a.SG * 16; i += kStreamThreads) {
             const int row = i >> 4, cc = i & 15;
@@ -278,14 +288,14 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                 }
                 j -= 1;
             }
-            if (MODE == kFinal && a.nS > 0) {
+            if (MODE == kFinal && nS > 0) {
                 if (j == 0) {
                     kind = 3;
                     dst = L.off_sid;
                 }
                 j -= 1;
             }
-            if (MODE == kFinal && a.nL > 1 && j >= 0 && j < a.nL) {
+            if (MODE == kFinal && nL > 1 && j >= 0 && j < nL) {
                 kind = 4 + j;
                 dst = L.off_rid[j];
             }
@@ -404,7 +414,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         const int4 m0 = reinterpret_cast<const int4*>(st)[0];
         const int4 m1 = reinterpret_cast<const int4*>(st)[1];
         const int k0 = m0.x, nk = m0.y;
-        const BlobLayout B = blob_layout(L.aux_stride, nk, m0.w, a.nL, m1.y, m1.w, a.nS);
+        const BlobLayout B = blob_layout(L.aux_stride, nk, m0.w, nL, m1.y, m1.w, nS);
         const unsigned char* blob = st + L.off_blob;
         const uint16_t* aux = reinterpret_cast<const uint16_t*>(blob);
         const double* col = reinterpret_cast<const double*>(st + L.off_cols + c * kStreamPitchD * 8) +
@@ -412,16 +422,17 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         const double* wv = nullptr;
         if (MODE == kFinal && WEIGHTED)
             wv = reinterpret_cast<const double*>(st + L.off_wp) + span_phase<8>(a.wp, k0);
-        int abase = (1 + a.nL) * (kStreamWarps + 1);
+        int abase = (1 + nL) * (kStreamWarps + 1);
 #pragma unroll
         for (int s = 0; s < kMaxSmall; ++s) {
-            if (s >= a.nS) break;
+            if (s >= nS) break;
             const uint16_t* ord = reinterpret_cast<const uint16_t*>(blob + B.ord[s]);
-            const int levels = (s + 1 < a.nS ? a.sgoff[s + 1] : a.SG) - a.sgoff[s];
+            const int levels = (s + 1 < nS ? a.sgoff[s + 1] : a.SG) - a.sgoff[s];
             for (int hh = grp; hh < levels; hh += 2 * kStreamWarps) {
                 const int j0 = aux[abase + hh], j1 = aux[abase + hh + 1];
                 if (j1 <= j0) continue;
                 double acc = 0.0;
+#pragma unroll 1
                 for (int jj = j0; jj < j1; ++jj) {
                     const int k = ord[jj];
                     const double v = col_lane ? col[k] : 0.0;
@@ -445,7 +456,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         const int4 m0 = reinterpret_cast<const int4*>(st)[0];
         const int4 m1 = reinterpret_cast<const int4*>(st)[1];
         const int k0 = m0.x, nk = m0.y, s0 = m0.z;
-        const BlobLayout B = blob_layout(L.aux_stride, nk, m0.w, a.nL, m1.y, m1.w, a.nS);
+        const BlobLayout B = blob_layout(L.aux_stride, nk, m0.w, nL, m1.y, m1.w, nS);
         const unsigned char* blob = st + L.off_blob;
         const uint16_t* aux = reinterpret_cast<const uint16_t*>(blob);
         const uint16_t* sego = reinterpret_cast<const uint16_t*>(blob + B.seg);
@@ -458,15 +469,15 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         const int sa = aux[warp], sb = aux[warp + 1];
         const int kb = sego[sa], ke = sego[sb];
 
-        if (MODE == kFinal && a.nL > 1 && kb < ke) {
+        if (MODE == kFinal && nL > 1 && kb < ke) {
             // v - D_r a for this warp's observations, a batch of loads at a time
-            const uint32_t* sidv = a.nS > 0 ? reinterpret_cast<const uint32_t*>(st + L.off_sid) +
+            const uint32_t* sidv = nS > 0 ? reinterpret_cast<const uint32_t*>(st + L.off_sid) +
                                                   span_phase<4>(a.sid, k0)
                                             : nullptr;
-            const int32_t* ridv0 = a.nL > 0 ? reinterpret_cast<const int32_t*>(st + L.off_rid[0]) +
+            const int32_t* ridv0 = nL > 0 ? reinterpret_cast<const int32_t*>(st + L.off_rid[0]) +
                                                   span_phase<4>(a.rid[0], k0)
                                             : nullptr;
-            const int32_t* ridv1 = a.nL > 1 ? reinterpret_cast<const int32_t*>(st + L.off_rid[1]) +
+            const int32_t* ridv1 = nL > 1 ? reinterpret_cast<const int32_t*>(st + L.off_rid[1]) +
                                                   span_phase<4>(a.rid[1], k0)
                                             : nullptr;
             for (int base = kb; base < ke; base += 2 * kStreamGather) {
@@ -476,11 +487,11 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                     const int k = base + 2 * q + h;
                     u[q] = 0.0;
                     if (k < ke && col_lane) {
-                        if (a.nL > 0) u[q] += __ldg(a.x + (a.lbase[0] + ridv0[k]) * CP + c);
-                        if (a.nL > 1) u[q] += __ldg(a.x + (a.lbase[1] + ridv1[k]) * CP + c);
-                        if (a.nS > 0) {
+                        if (nL > 0) u[q] += __ldg(a.x + (a.lbase[0] + ridv0[k]) * CP + c);
+                        if (nL > 1) u[q] += __ldg(a.x + (a.lbase[1] + ridv1[k]) * CP + c);
+                        if (nS > 0) {
                             const uint32_t packed = sidv[k];
-                            for (int s = 0; s < a.nS; ++s)
+                            for (int s = 0; s < nS; ++s)
                                 u[q] += __ldg(a.x + (a.sbase[s] + ((packed >> (8 * s)) & 0xffu)) * CP + c);
                         }
                     }
@@ -500,32 +511,41 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         const uint16_t* rs1 = nullptr;
         const int32_t* rd1 = nullptr;
         int r0c = 0, r1c = 0;
-        if ((scatter || MODE == kFinal) && a.nL > 0) {
+        if ((scatter || MODE == kFinal) && nL > 0) {
             rs0 = reinterpret_cast<const uint16_t*>(blob + B.runs[0]);
             rd0 = reinterpret_cast<const int32_t*>(blob + B.rd[0]);
             r0c = aux[(kStreamWarps + 1) + warp];
         }
-        if (scatter && a.nL > 1) {
+        if (scatter && nL > 1) {
             rs1 = reinterpret_cast<const uint16_t*>(blob + B.runs[1]);
             rd1 = reinterpret_cast<const int32_t*>(blob + B.rd[1]);
             r1c = aux[2 * (kStreamWarps + 1) + warp];
         }
-        if (MODE == kFinal && a.nL <= 1) {
-            // v - D_r a - mean with one row of dim 0 per run (held in afb, up to
-            // kStreamRunRows runs loaded at a time) and the small-dim rows from yt
-            const uint32_t* sidv = a.nS > 0 ? reinterpret_cast<const uint32_t*>(st + L.off_sid) +
+        if (MODE == kFinal && nL <= 1) {
+            // v - D_r a - mean with one row of dim 0 per run (in registers, the
+            // next kStreamRunRows runs' on their way) and the small-dim rows from yt
+            const uint32_t* sidv = nS > 0 ? reinterpret_cast<const uint32_t*>(st + L.off_sid) +
                                                   span_phase<4>(a.sid, k0)
                                             : nullptr;
             const double* yt = reinterpret_cast<const double*>(smem + L.off_yt);
-            double* afb = reinterpret_cast<double*>(smem + L.off_afb) + warp * kStreamRunRows * 16;
             const int32_t* rg0 = reinterpret_cast<const int32_t*>(blob + B.rg);
-            const int rend = a.nL > 0 ? aux[(kStreamWarps + 1) + warp + 1] : 0;
-            int fb = r0c, fe = r0c;
+            const int rend = nL > 0 ? aux[(kStreamWarps + 1) + warp + 1] : 0;
+            int fb = r0c;
+            double cur[kStreamRunRows], nxt[kStreamRunRows];
+            auto load_rows = [&](int f, double (&rows)[kStreamRunRows]) {
+#pragma unroll
+                for (int q = 0; q < kStreamRunRows; ++q)
+                    rows[q] = (f + q < rend && c < CP) ? __ldg(a.x + (a.lbase[0] + rg0[f + q]) * CP + c) : 0.0;
+            };
+            if (nL == 1) {
+                load_rows(fb, cur);
+                load_rows(fb + kStreamRunRows, nxt);
+            }
             auto small_rows = [&](int k) {
                 double y = 0.0;
-                if (a.nS > 0) {
+                if (nS > 0) {
                     const uint32_t packed = sidv[k];
-                    for (int s = 0; s < a.nS; ++s) y += yt[(a.sgoff[s] + ((packed >> (8 * s)) & 0xffu)) * 16 + c];
+                    for (int s = 0; s < nS; ++s) y += yt[(a.sgoff[s] + ((packed >> (8 * s)) & 0xffu)) * 16 + c];
                 }
                 return y;
             };
@@ -533,24 +553,21 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                 const int b = sego[j], e = sego[j + 1];
                 const int rstart = r0c;
                 double acc = 0.0;
-                if (a.nL == 1) {
+                if (nL == 1) {
+#pragma unroll 1
                     while (rs0[r0c] < e) {
-                        if (r0c >= fe) {
-                            __syncwarp();
+                        if (r0c - fb == kStreamRunRows) {
                             fb = r0c;
-                            fe = min(rend, r0c + kStreamRunRows);
-                            double rows[kStreamRunRows / 2];
 #pragma unroll
-                            for (int q = 0; q < kStreamRunRows / 2; ++q) {
-                                const int rr = fb + 2 * q + h;
-                                rows[q] = (rr < fe && c < CP) ? __ldg(a.x + (a.lbase[0] + rg0[rr]) * CP + c) : 0.0;
-                            }
-#pragma unroll
-                            for (int q = 0; q < kStreamRunRows / 2; ++q) afb[(2 * q + h) * 16 + c] = rows[q];
-                            __syncwarp();
+                            for (int q = 0; q < kStreamRunRows; ++q) cur[q] = nxt[q];
+                            load_rows(fb + kStreamRunRows, nxt);
                         }
-                        const double af = afb[(r0c - fb) * 16 + c];
+                        double af = cur[0];
+#pragma unroll
+                        for (int q = 1; q < kStreamRunRows; ++q)
+                            if (r0c - fb == q) af = cur[q];
                         const int q0 = rs0[r0c], q1 = rs0[r0c + 1];
+#pragma unroll 1
                         for (int k = q0 + h; k < q1; k += 2) {
                             if (col_lane) {
                                 const double u = col[k] - af - small_rows(k);
@@ -561,6 +578,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                         ++r0c;
                     }
                 } else {
+#pragma unroll 1
                     for (int k = b + h; k < e; k += 2) {
                         if (col_lane) {
                             const double u = col[k] - small_rows(k);
@@ -573,10 +591,11 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                 const double mean = acc * iw[j];
                 if (a.mean_out && h == 0 && c < CP) a.mean_out[static_cast<int64_t>(s0 + j) * CP + c] = mean;
                 double zs = 0.0;
-                if (a.nL == 1) {
+                if (nL == 1) {
                     for (int r = rstart; r < r0c; ++r) {
                         const int q0 = rs0[r], q1 = rs0[r + 1];
                         double racc = 0.0;
+#pragma unroll 1
                         for (int k = q0 + h; k < q1; k += 2) {
                             const double d = col_lane ? col[k] - mean : 0.0;
                             const double z = WEIGHTED ? wv[k] * d : d;
@@ -590,6 +609,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                         }
                     }
                 } else {
+#pragma unroll 1
                     for (int k = b + h; k < e; k += 2) {
                         const double d = col_lane ? col[k] - mean : 0.0;
                         if (col_lane) col[k] = d;
@@ -603,6 +623,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
         for (int j = sa; j < sb; ++j) {
             const int b = sego[j], e = sego[j + 1];
             double acc = 0.0;
+#pragma unroll 1
             for (int k = b + h; k < e; k += 2) {
                 const double v = col_lane ? col[k] : 0.0;
                 acc = WEIGHTED ? fma(wv[k], v, acc) : acc + v;
@@ -615,9 +636,11 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
             double zs = 0.0;
             if (rs0) {
                 // runs of the first large dim: z (kRhs) or d (kFinal) into the stage
+#pragma unroll 1
                 while (rs0[r0c] < e) {
                     const int q0 = rs0[r0c], q1 = rs0[r0c + 1];
                     double racc = 0.0;
+#pragma unroll 1
                     for (int k = q0 + h; k < q1; k += 2) {
                         const double d = col_lane ? col[k] - mean : 0.0;
                         const double z = WEIGHTED ? wv[k] * d : d;
@@ -631,9 +654,11 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                 }
                 if (rs1) {
                     __syncwarp();  // z / d of the other half
+#pragma unroll 1
                     while (rs1[r1c] < e) {
                         const int q0 = rs1[r1c], q1 = rs1[r1c + 1];
                         double racc = 0.0;
+#pragma unroll 1
                         for (int k = q0 + h; k < q1; k += 2) {
                             const double d = col_lane ? col[k] : 0.0;
                             racc += (MODE == kFinal && WEIGHTED) ? wv[k] * d : d;
@@ -644,6 +669,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
                     }
                 }
             } else {
+#pragma unroll 1
                 for (int k = b + h; k < e; k += 2) {
                     const double d = col_lane ? col[k] - mean : 0.0;
                     const double z = WEIGHTED ? wv[k] * d : d;
@@ -700,7 +726,7 @@ stream_pass_kernel(const PassArgs<double> a, const StreamLayout L) {
     asm volatile("bar.sync 1, %0;" ::"r"(kStreamWarps * 32) : "memory");
     const int tid = threadIdx.x;
     const int cta = a.bins_cta0 + blockIdx.x;
-    if (a.nS > 0 && scatter) {
+    if (nS > 0 && scatter) {
         double* dst = a.bins_partial + static_cast<int64_t>(cta) * a.SG * CP;
         for (int idx = tid; idx < a.SG * CP; idx += kStreamWarps * 32) {
             const int row = idx / CP, cc = idx - row * CP;
