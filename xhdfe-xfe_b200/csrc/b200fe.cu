@@ -948,6 +948,8 @@ int prepare_work(b200fe_context* ctx, const std::string& tag, Work<T>& wk) {
     B_CHECK((set_pass_smem<T, CQ, kMatvec>(ctx, wk.tile_smem, wk.long_smem)));
     B_CHECK((set_pass_smem<T, CQ, kRhs>(ctx, wk.tile_smem, wk.long_smem)));
     B_CHECK((set_pass_smem<T, CQ, kFinal>(ctx, wk.tile_smem, wk.long_smem)));
+    // the kernel's launch bounds allow three CTAs an SM; the grid is also the order
+    // in which the bins' partials are summed
     int per_sm = 1;
     B_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_pass_kernel<T, CQ, kMatvec>,
                                                         kTileThreads, wk.tile_smem));
@@ -1073,6 +1075,12 @@ PassArgs<T> make_pass_args(const Structure& st, int cols, int CP, const Work<T>&
     return a;
 }
 
+using StreamKernel = void (*)(const PassArgs<double>, const StreamLayout);
+template <int MODE, int KL, int KS>
+StreamKernel stream_kernel(bool weighted) {
+    return weighted ? stream_pass_kernel<MODE, true, KL, KS> : stream_pass_kernel<MODE, false, KL, KS>;
+}
+
 // Bulk-copy FP64 data pass over the regular tiles (stream_kernels.cuh): one
 // CTA per SM with as many stages as shared memory holds (at least two).
 // *grid = 0 (nothing launched) when it does not apply: the pass is off, the
@@ -1129,13 +1137,15 @@ int launch_stream_pass(b200fe_context* ctx, const PassArgs<double>& a, int* grid
         B_TRY(cudaMemsetAsync(ctx->stream_status, 0, 4 * sizeof(int), ctx->stream));
     }
     L.status = ctx->stream_status;
-    // one large dim with up to one small one (worker, firm and year): the dims
-    // known at compile time
-    const int form = a.nL == 1 && a.nS <= 1 ? a.nS : 2;
-    auto kern = form == 0   ? (weighted ? stream_pass_kernel<MODE, true, 1, 0> : stream_pass_kernel<MODE, false, 1, 0>)
-                : form == 1 ? (weighted ? stream_pass_kernel<MODE, true, 1, 1> : stream_pass_kernel<MODE, false, 1, 1>)
-                            : (weighted ? stream_pass_kernel<MODE, true, -1, -1>
-                                        : stream_pass_kernel<MODE, false, -1, -1>);
+    // one or two large dims with up to one small one (worker, firm, year and
+    // occupation): the dims known at compile time
+    const bool known = (a.nL == 1 || a.nL == 2) && a.nS <= 1;
+    const int form = known ? 1 + 2 * (a.nL - 1) + a.nS : 0;
+    const StreamKernel kern = form == 1   ? stream_kernel<MODE, 1, 0>(weighted)
+                              : form == 2 ? stream_kernel<MODE, 1, 1>(weighted)
+                              : form == 3 ? stream_kernel<MODE, 2, 0>(weighted)
+                              : form == 4 ? stream_kernel<MODE, 2, 1>(weighted)
+                                          : stream_kernel<MODE, -1, -1>(weighted);
     const unsigned bit = 1u << (4 * form + 2 * (MODE == kFinal ? 1 : 0) + (weighted ? 1 : 0));
     if (!(ctx->stream_smem_set & bit)) {
         B_TRY(raise_smem_limit(reinterpret_cast<const void*>(kern), budget));

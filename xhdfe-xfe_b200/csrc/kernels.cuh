@@ -100,6 +100,21 @@ __device__ __forceinline__ void store_quad_stream(double* p, const Acc4& a) {
 }
 
 
+// 2^-896 times a finite value as FP64, exactly (zeros and subnormals too), and
+// the factor that undoes it: an FP32 -> FP64 conversion per gathered element
+// is what the gathers wait for (2-way 50M rows, 16 columns: 189 us an iteration
+// with conversions, 151 with shifts), and the factor goes into the other operand
+// of the product, once for the four columns of a lane.
+__device__ __forceinline__ double scaled64(float x) {
+    const int u = __float_as_int(x);
+    return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
+}
+__device__ __forceinline__ double scaled64(double x) { return x; }
+template <typename T>
+__device__ __forceinline__ double unscale64() {
+    return sizeof(T) == 4 ? 0x1p896 : 1.0;
+}
+
 // ---------------------------------------------------------------------------
 // Primary-segment passes.
 //
@@ -116,7 +131,13 @@ __device__ __forceinline__ void store_quad_stream(double* p, const Acc4& a) {
 //
 // tile_pass_kernel handles tiles of whole segments (<= kTileObs obs): all
 // loads of a tile are issued at once into shared memory, then segment means,
-// runs and bins are reduced from shared memory.  Segments longer than
+// runs and bins are reduced from shared memory.  kMatvec (mixed solves with two
+// large dims) is bound by latency at 16 warps an SM: 394 us a pass over 2M rows,
+// 16 columns with a gather after the other, the offsets read where they are used
+// and a conversion per staged value; 280 us with kTileGather rows in flight,
+// offsets and runs read before the gather, the bins' reads taken four steps at a
+// time and scaled64 for the conversions.  Every rounding and every order of
+// summation is that of the data modes' code.  Segments longer than
 // kLongSeg form their own tiles and go through segment_pass_kernel.
 // ---------------------------------------------------------------------------
 enum PassMode { kMatvec = 0, kRhs = 1, kFinal = 2 };
@@ -160,6 +181,19 @@ struct PassArgs {
     int64_t nlong;
 };
 
+template <typename T>
+__device__ __forceinline__ void load_quad_raw(const T* __restrict__ p, T (&v)[4]);
+template <>
+__device__ __forceinline__ void load_quad_raw<float>(const float* __restrict__ p, float (&v)[4]) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+template <>
+__device__ __forceinline__ void load_quad_raw<double>(const double* __restrict__ p, double (&v)[4]) {
+    const double2 s = __ldg(reinterpret_cast<const double2*>(p)), t = __ldg(reinterpret_cast<const double2*>(p) + 1);
+    v[0] = s.x; v[1] = s.y; v[2] = t.x; v[3] = t.y;
+}
+
 // (D_r x)_k for the 4 columns of lane quad q
 template <typename T>
 __device__ __forceinline__ void gather_u(const PassArgs<T>& a, int64_t k, int q, Acc4& u) {
@@ -192,6 +226,14 @@ __device__ __forceinline__ void smem_load4<double>(const double* p, Acc4& o) {
     const double2 a = reinterpret_cast<const double2*>(p)[0];
     const double2 b = reinterpret_cast<const double2*>(p)[1];
     o.v[0] = a.x; o.v[1] = a.y; o.v[2] = b.x; o.v[3] = b.y;
+}
+__device__ __forceinline__ void smem_load_raw(const float* p, float (&v)[4]) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void smem_load_raw(const double* p, double (&v)[4]) {
+    const double2 s = reinterpret_cast<const double2*>(p)[0], t = reinterpret_cast<const double2*>(p)[1];
+    v[0] = s.x; v[1] = s.y; v[2] = t.x; v[3] = t.y;
 }
 template <typename T>
 __device__ __forceinline__ void smem_store4(T* p, const Acc4& o);
@@ -229,6 +271,13 @@ struct Stage {
             for (int j = 0; j < 4; ++j) o.v[j] = static_cast<double>(u[(4 * q + j) * LD + kl]);
         }
     }
+    // kMatvec: the four values times 1 / unscale64<T>()
+    __device__ static __forceinline__ void load4_scaled(const T* u, int kl, int q, Acc4& o) {
+        T v[4];
+        smem_load_raw(u + kl * CP + 4 * q, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o.v[j] = scaled64(v[j]);
+    }
     __device__ static __forceinline__ void store4(T* u, int kl, int q, const Acc4& o) {
         if (MODE == kMatvec) {
             smem_store4<T>(u + kl * CP + 4 * q, o);
@@ -242,8 +291,12 @@ struct Stage {
     }
 };
 
+constexpr int kTileGather = 2;  // kMatvec: observations a group has in flight
+constexpr int kBinSteps = 4;    // kMatvec: steps of the bin update read together
+constexpr int kTileAhead = 2;   // kMatvec: runs of a group whose offsets are read ahead
+
 template <typename T, int CQ, int MODE>
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads, MODE == kMatvec ? 3 : 1)
 tile_pass_kernel(const PassArgs<T> a) {
     constexpr int CP = 4 * CQ;
     using St = Stage<T, CP, MODE>;
@@ -265,18 +318,89 @@ tile_pass_kernel(const PassArgs<T> a) {
     for (int i = tid; i < (kTileThreads / 32) * a.SG * BROW; i += kTileThreads) bins[i] = 0.0;
     double colsq[4] = {0.0, 0.0, 0.0, 0.0};
 
+    // kMatvec keeps the tile's packed small ids where the data modes reduce colsq
+    uint32_t* sbuf = reinterpret_cast<uint32_t*>(red);
     for (int64_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
         if (a.tile_long[t]) continue;
         const int32_t s0 = a.tile_seg[t], s1 = a.tile_seg[t + 1];
         const int64_t k0 = a.seg_off[s0];
         const int nk = static_cast<int>(a.seg_off[s1] - k0);
+        // this group's first segment and first runs, on their way before phase A
+        int32_t rb[kMaxLarge], re[kMaxLarge];
+        int pb = 0, pe = 0;
+        uint32_t rpo[kMaxLarge][kTileAhead];  // run offsets, two 16-bit halves
+        int32_t rpd[kMaxLarge][kTileAhead];
+        double piw = 0.0;
+        if (MODE == kMatvec) {
+            if (s0 + g < s1) {
+                pb = static_cast<int>(a.seg_off[s0 + g] - k0);
+                pe = static_cast<int>(a.seg_off[s0 + g + 1] - k0);
+                piw = a.inv_wp[s0 + g];
+            }
+#pragma unroll
+            for (int l = 0; l < kMaxLarge; ++l) {
+                if (l >= a.nL) continue;
+                rb[l] = a.run_base[l][s0];
+                re[l] = a.run_base[l][s1];
+#pragma unroll
+                for (int i = 0; i < kTileAhead; ++i) {
+                    const int32_t m = rb[l] + g + i * GPB;
+                    if (m < re[l]) {
+                        rpo[l][i] = static_cast<uint32_t>(a.run_start[l][m] - k0) |
+                                    static_cast<uint32_t>(a.run_start[l][m + 1] - k0) << 16;
+                        rpd[l][i] = a.run_dest[l][m];
+                    }
+                }
+            }
+        }
         __syncthreads();  // previous tile fully consumed
         // ---- phase A: stage values and weights --------------------------
         if (MODE == kMatvec) {
-            for (int kl = g; kl < nk; kl += GPB) {
-                Acc4 u;
-                gather_u(a, k0 + kl, q, u);
-                St::store4(ubuf, kl, q, u);
+            for (int kl0 = g; kl0 < nk; kl0 += kTileGather * GPB) {
+                int32_t id[kMaxLarge][kTileGather];
+                uint32_t packed[kTileGather];
+                Acc4 u[kTileGather];
+#pragma unroll
+                for (int i = 0; i < kTileGather; ++i) {
+                    const int kl = kl0 + i * GPB;
+                    acc_zero(u[i]);
+#pragma unroll
+                    for (int l = 0; l < kMaxLarge; ++l)
+                        id[l][i] = (l < a.nL && kl < nk) ? __ldg(a.rid[l] + k0 + kl) : -1;
+                    packed[i] = (a.nS > 0 && kl < nk) ? __ldg(a.sid + k0 + kl) : 0u;
+                }
+                T x[kMaxLarge][kTileGather][4];
+#pragma unroll
+                for (int l = 0; l < kMaxLarge; ++l)
+#pragma unroll
+                    for (int i = 0; i < kTileGather; ++i)
+                        if (id[l][i] >= 0) load_quad_raw(a.x + (a.lbase[l] + id[l][i]) * CP + 4 * q, x[l][i]);
+#pragma unroll
+                for (int l = 0; l < kMaxLarge; ++l)
+#pragma unroll
+                    for (int i = 0; i < kTileGather; ++i)
+                        if (id[l][i] >= 0)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) u[i].v[j] += scaled64(x[l][i][j]);
+                for (int s = 0; s < a.nS; ++s)
+#pragma unroll
+                    for (int i = 0; i < kTileGather; ++i)
+                        if (kl0 + i * GPB < nk) {
+                            T y[4];
+                            load_quad_raw(a.x + (a.sbase[s] + ((packed[i] >> (8 * s)) & 0xffu)) * CP + 4 * q, y);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) u[i].v[j] += scaled64(y[j]);
+                        }
+#pragma unroll
+                for (int i = 0; i < kTileGather; ++i) {
+                    const int kl = kl0 + i * GPB;
+                    if (kl < nk) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) u[i].v[j] = __dmul_rn(u[i].v[j], unscale64<T>());
+                        St::store4(ubuf, kl, q, u[i]);
+                        if (q == 0) sbuf[kl] = packed[i];
+                    }
+                }
             }
         } else {
             const int total = CP * nk;
@@ -308,10 +432,20 @@ tile_pass_kernel(const PassArgs<T> a) {
         __syncthreads();
         // ---- phase B: segment means; ubuf <- z (kMatvec/kRhs) or d (kFinal)
         for (int32_t s = s0 + g; s < s1; s += GPB) {
-            const int b = static_cast<int>(a.seg_off[s] - k0);
-            const int e = static_cast<int>(a.seg_off[s + 1] - k0);
+            const bool ahead = MODE == kMatvec && s == s0 + g;
+            const int b = ahead ? pb : static_cast<int>(a.seg_off[s] - k0);
+            const int e = ahead ? pe : static_cast<int>(a.seg_off[s + 1] - k0);
             Acc4 acc;
             acc_zero(acc);
+            if (MODE == kMatvec)
+                for (int kl = b; kl < e; ++kl) {
+                    Acc4 val;
+                    St::load4_scaled(ubuf, kl, q, val);
+                    const double w = __dmul_rn(static_cast<double>(wbuf[kl]), unscale64<T>());
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc.v[j] = fma(w, val.v[j], acc.v[j]);
+                }
+            else
             for (int kl = b; kl < e; ++kl) {
                 Acc4 val;
                 St::load4(ubuf, kl, q, val);
@@ -322,9 +456,20 @@ tile_pass_kernel(const PassArgs<T> a) {
                     if (MODE == kRhs) colsq[j] = fma(val.v[j], val.v[j], colsq[j]);
                 }
             }
-            const double iw = a.inv_wp[s];
+            const double iw = ahead ? piw : a.inv_wp[s];
             Acc4 zs;
             acc_zero(zs);
+            if (MODE == kMatvec)
+                for (int kl = b; kl < e; ++kl) {
+                    Acc4 val;
+                    St::load4_scaled(ubuf, kl, q, val);
+                    const double w = static_cast<double>(wbuf[kl]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        val.v[j] = w * __dsub_rn(__dmul_rn(val.v[j], unscale64<T>()), __dmul_rn(acc.v[j], iw));
+                    St::store4(ubuf, kl, q, val);
+                }
+            else
             for (int kl = b; kl < e; ++kl) {
                 Acc4 val;
                 St::load4(ubuf, kl, q, val);
@@ -348,12 +493,17 @@ tile_pass_kernel(const PassArgs<T> a) {
 #pragma unroll
             for (int l = 0; l < kMaxLarge; ++l) {
                 if (l >= a.nL) continue;
-                const int32_t rb = a.run_base[l][s0], re = a.run_base[l][s1];
-                for (int32_t m = rb + g; m < re; m += GPB) {
-                    const int b = static_cast<int>(a.run_start[l][m] - k0);
-                    const int e = static_cast<int>(a.run_start[l][m + 1] - k0);
+                auto sum_run = [&](int b, int e, int32_t dest) {
                     Acc4 acc;
                     acc_zero(acc);
+                    if (MODE == kMatvec)
+                        for (int kl = b; kl < e; ++kl) {
+                            Acc4 z;
+                            St::load4_scaled(ubuf, kl, q, z);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) acc.v[j] = fma(unscale64<T>(), z.v[j], acc.v[j]);
+                        }
+                    else
                     for (int kl = b; kl < e; ++kl) {
                         Acc4 z;
                         St::load4(ubuf, kl, q, z);
@@ -361,9 +511,21 @@ tile_pass_kernel(const PassArgs<T> a) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) acc.v[j] = fma(w, z.v[j], acc.v[j]);
                     }
-                    store_quad_stream(a.R[l] + static_cast<int64_t>(a.run_dest[l][m]) * CP + 4 * q,
-                                      acc);
+                    store_quad_stream(a.R[l] + static_cast<int64_t>(dest) * CP + 4 * q, acc);
+                };
+                if (MODE != kMatvec) {
+                    rb[l] = a.run_base[l][s0];
+                    re[l] = a.run_base[l][s1];
                 }
+                int32_t m = rb[l] + g;
+                if (MODE == kMatvec)
+#pragma unroll
+                    for (int i = 0; i < kTileAhead; ++i, m += GPB)
+                        if (m < re[l])
+                            sum_run(static_cast<int>(rpo[l][i] & 0xffffu), static_cast<int>(rpo[l][i] >> 16), rpd[l][i]);
+                for (; m < re[l]; m += GPB)
+                    sum_run(static_cast<int>(a.run_start[l][m] - k0), static_cast<int>(a.run_start[l][m + 1] - k0),
+                            a.run_dest[l][m]);
             }
             // ---- phase C': small-dim bins, warp-private, fixed order ------
             // A warp step covers 32/CP consecutive observations, one per
@@ -377,10 +539,41 @@ tile_pass_kernel(const PassArgs<T> a) {
                 const int per_warp = (nk + (kTileThreads / 32) - 1) / (kTileThreads / 32);
                 const int wb = warp * per_warp;
                 const int we = min(nk, wb + per_warp);
+                if (MODE == kMatvec && G <= 2) {
+                    // one or two groups: four steps' reads together, the pair's
+                    // keys compared by a shuffle
+                    for (int base = wb; base < we; base += kBinSteps * G) {
+                        uint32_t packed[kBinSteps];
+                        double z[kBinSteps];
+#pragma unroll
+                        for (int i = 0; i < kBinSteps; ++i) {
+                            const int kl = base + i * G + gi;
+                            packed[i] = kl < we ? sbuf[kl] : 0u;
+                            z[i] = kl < we ? scaled64(St::at(ubuf, kl, c)) : 0.0;
+                        }
+#pragma unroll
+                        for (int i = 0; i < kBinSteps; ++i) {
+                            if (base + i * G >= we) break;
+                            const bool valid = base + i * G + gi < we;
+                            const double zo = G == 2 ? __shfl_xor_sync(0xffffffffu, z[i], 16) : 0.0;
+                            const uint32_t po = G == 2 ? __shfl_xor_sync(0xffffffffu, packed[i], 16) : 0u;
+                            const bool pair = G == 2 && base + i * G + 1 < we;
+                            for (int s = 0; s < a.nS; ++s) {
+                                const uint32_t key = (packed[i] >> (8 * s)) & 0xffu;
+                                const bool same = pair && key == ((po >> (8 * s)) & 0xffu);
+                                if (valid && !(same && gi == 1)) {
+                                    double& bin = my_bins[(a.sgoff[s] + static_cast<int>(key)) * BROW + c];
+                                    bin = fma(unscale64<T>(), same ? z[i] + zo : z[i], bin);
+                                }
+                                __syncwarp();
+                            }
+                        }
+                    }
+                } else
                 for (int base = wb; base < we; base += G) {
                     const int kl = base + gi;
                     const bool valid = kl < we;
-                    const uint32_t packed = valid ? __ldg(a.sid + k0 + kl) : 0u;
+                    const uint32_t packed = valid ? (MODE == kMatvec ? sbuf[kl] : __ldg(a.sid + k0 + kl)) : 0u;
                     for (int s = 0; s < a.nS; ++s) {
                         const uint32_t key = valid ? ((packed >> (8 * s)) & 0xffu) : 0x100u + gi;
                         const unsigned int match = __match_any_sync(0xffffffffu, key);

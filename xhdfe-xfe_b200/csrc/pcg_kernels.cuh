@@ -172,20 +172,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// 2^-896 times a finite value as FP64, exactly (zeros and subnormals too), and
-// the factor that undoes it: an FP32 -> FP64 conversion per gathered element
-// is what the gathers wait for (2-way 50M rows, 16 columns: 189 us an iteration
-// with conversions, 151 with shifts), and the factor goes into the other operand
-// of the product, once for the four columns of a lane.
-__device__ __forceinline__ double scaled64(float x) {
-    const int u = __float_as_int(x);
-    return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
-}
-__device__ __forceinline__ double scaled64(double x) { return x; }
-template <typename T>
-__device__ __forceinline__ double unscale64() {
-    return sizeof(T) == 4 ? 0x1p896 : 1.0;
-}
 // z = M^-1 r: the FP32 product rounded once, as the exact FP64 product would be
 __device__ __forceinline__ float precond(float d, float r) { return __fmul_rn(d, r); }
 __device__ __forceinline__ double precond(double d, double r) { return __dmul_rn(d, r); }
