@@ -636,8 +636,8 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     // run rows): its setup also yields the exact small-dim diagonal
     // With two large dims the explicit block replaces the pass over the
     // observations in solves that run in FP64 throughout, wherever its
-    // contributions fit (2M rows, worker/firm/year/occupation, 9 columns: an
-    // iteration of 560 us becomes one of 83).  The FP32 inner solves of the
+    // contributions fit (2M rows, worker/firm/year/occupation, 9 columns: 7.2 ms
+    // for 31.1).  The FP32 inner solves of the
     // mixed scheme keep the pass: their answers carry its roundings (R in FP32
     // per run), up to 1e-7 of a column in badly identified rows.  The pairs are
     // counted here, since the small dim's diagonal then comes from the coupling.
