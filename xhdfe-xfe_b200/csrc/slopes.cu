@@ -440,8 +440,15 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             }
         }
     }
-    // coefficient form: the runs in both orders and their chunks in L's order
-    if (sf.on) {
+    // coefficient form: its buffers, the runs in both orders and their chunks in
+    // L's order
+    const int gD = sf.on ? static_cast<int>(std::max<int64_t>(
+                               1, std::min<int64_t>((sf.NL + 63) / 64, 2 * static_cast<int64_t>(ctx->num_sms))))
+                         : 0;
+    SlopeStepArgs sa{};
+    double *space_Sly = nullptr, *space_one = nullptr, *space_sc = nullptr, *space_dot = nullptr, *space_py = nullptr;
+    int* space_act = nullptr;
+    auto space_setup = [&]() -> int {
         const SlopeDim &P = dims[p], &L = dims[sf.L];
         sf.kp = P.nb;
         sf.kd = L.nb;
@@ -539,6 +546,26 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             sf.dn.part = X.part;
             sf.dn.big = X.big;
             sf.dn.t = sf.t;
+            const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
+            B_CHECK(get_buf(ctx, "sl_xly", std::max<size_t>(sly, 1), &space_Sly));
+            B_CHECK(get_buf(ctx, "sl_xyy", std::max(1, sf.Y * sf.Y), &sf.Syy));
+            B_CHECK(get_buf(ctx, "sl_xone", C, &space_one));
+            B_CHECK(get_buf(ctx, "sl_xsc", static_cast<size_t>(4) * C, &space_sc));
+            B_CHECK(get_buf(ctx, "sl_xact", static_cast<size_t>(2) * C, &space_act));
+            B_CHECK(get_buf(ctx, "sl_xdot", static_cast<size_t>(gD) * C, &space_dot));
+            B_CHECK(get_buf(ctx, "sl_xpy", std::max<size_t>(static_cast<size_t>(gD) * sf.Y * C, 1), &space_py));
+            sa.grid = grid_for(ctx, (row + RB - 1) / RB, 1, 2);
+            B_CHECK(get_buf(ctx, "sl_xpg", static_cast<size_t>(sa.grid) * C, &sa.part_g));
+        }
+        return B200FE_OK;
+    };
+    if (sf.on) {
+        const int rc = space_setup();
+        if (rc != B200FE_OK) {
+            // no room for it on the device: the observation passes, as without it
+            if (ctx->err.rfind("cudaMalloc(", 0) != 0) return rc;
+            ctx->err.clear();
+            sf.on = false;
         }
     }
     // ---- input norms and stop thresholds
@@ -776,12 +803,8 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
 
     // ---- coefficient form: S_Ly and S_yy, its vectors and its steps
     SchurGatherArgs sgx = sga;  // the image of the coefficients x
-    SlopeStepArgs sa{};
     SlopeScalars scal[2] = {};
     double* ones = nullptr;
-    const int gD = sf.on ? static_cast<int>(std::max<int64_t>(
-                               1, std::min<int64_t>((sf.NL + 63) / 64, 2 * static_cast<int64_t>(ctx->num_sms))))
-                         : 0;
     auto chunk_sums = [&](int d, int cols, int64_t pitch, double* out) -> int {
         const SlopeDim& D = dims[d];
         if (n_big[d] > 0) {
@@ -804,21 +827,13 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         return i;
     };
     if (sf.on) {
-        const int64_t rows = sf.NL + sf.Y;
         for (int i = 0; i < sgx.nd; ++i) sgx.dim[i].p = sf.x + sf.sp.row0[space_dim(cg[i])] * C;
-        double *Sly, *one_buf, *xsc;
-        int* xact;
         const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
-        B_CHECK(get_buf(ctx, "sl_xly", std::max<size_t>(sly, 1), &Sly));
-        B_CHECK(get_buf(ctx, "sl_xyy", std::max(1, sf.Y * sf.Y), &sf.Syy));
-        B_CHECK(get_buf(ctx, "sl_xone", C, &one_buf));
-        B_CHECK(get_buf(ctx, "sl_xsc", static_cast<size_t>(4) * C, &xsc));
-        B_CHECK(get_buf(ctx, "sl_xact", static_cast<size_t>(2) * C, &xact));
         const std::vector<double> h1(C, 1.0);
-        B_TRY(cudaMemcpyAsync(one_buf, h1.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
-        ones = one_buf;
-        for (int i = 0; i < 2; ++i) scal[i] = SlopeScalars{xsc + i * C, xsc + (2 + i) * C, xact + i * C};
-        if (sly) B_TRY(cudaMemsetAsync(Sly, 0, sizeof(double) * sly, s));
+        B_TRY(cudaMemcpyAsync(space_one, h1.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
+        ones = space_one;
+        for (int i = 0; i < 2; ++i) scal[i] = SlopeScalars{space_sc + i * C, space_sc + (2 + i) * C, space_act + i * C};
+        if (sly) B_TRY(cudaMemsetAsync(space_Sly, 0, sizeof(double) * sly, s));
         for (int y0 = 0; y0 < sf.Y; y0 += C) {
             const int cols = std::min(C, sf.Y - y0);
             if (y0 == 0) B_TRY(cudaMemsetAsync(sf.x, 0, sizeof(double) * sf.NL * C, s));
@@ -828,29 +843,24 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             B_CHECK(schur_gather(sgx));
             for (int d : cg) {
                 B_CHECK(segment(d, false, Q));
-                if (d == sf.L) B_CHECK(chunk_sums(d, cols, sf.Yp, Sly + y0));
+                if (d == sf.L) B_CHECK(chunk_sums(d, cols, sf.Yp, space_Sly + y0));
                 else B_CHECK(chunk_sums(d, cols, sf.Y, sf.Syy + (sf.sp.row0[space_dim(d)] - sf.NL) * sf.Y + y0));
             }
         }
-        sf.dn.Sly = Sly;
-        double *dot, *py;
-        B_CHECK(get_buf(ctx, "sl_xdot", static_cast<size_t>(gD) * C, &dot));
-        B_CHECK(get_buf(ctx, "sl_xpy", std::max<size_t>(static_cast<size_t>(gD) * sf.Y * C, 1), &py));
-        sf.dn.dot = dot;
-        sf.dn.part_y = py;
+        sf.dn.Sly = space_Sly;
+        sf.dn.dot = space_dot;
+        sf.dn.part_y = space_py;
         sa.sp = sf.sp;
         sa.NL = sf.NL;
         sa.Y = sf.Y;
         sa.thr = d_thr;
-        sa.dot = dot;
+        sa.dot = space_dot;
         sa.ndot = gD;
         sa.p = sf.p;
         sa.x = sf.x;
         sa.s = sf.s;
         sa.t = sf.t;
-        sa.grid = grid_for(ctx, (rows + RB - 1) / RB, 1, 2);
         sa.done = done;
-        B_CHECK(get_buf(ctx, "sl_xpg", static_cast<size_t>(sa.grid) * C, &sa.part_g));
     }
     int side = 0;  // which set of scalars the next step reads
     auto space_step = [&](bool first) -> int {
