@@ -1723,7 +1723,7 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     const bool coupled = st.coupled && st.nS == 1;
     const int SG = coupled ? st.SG : 0;
     const int SGP = coupled ? st.SGP : 0;
-    if (SG > kPcgMaxSG) return B200FE_UNAVAILABLE;
+    if (!pcg_rows_fit(ctx->num_sms, SG)) return B200FE_UNAVAILABLE;
     // two staging buffers of the coupling where they fit beside the rest
     const int cbuf = pcg_smem_bytes<T>(CP, SG, SGP, 2) <= 200 * 1024 ? 2 : 1;
     const size_t smem = pcg_smem_bytes<T>(CP, SG, SGP, cbuf);

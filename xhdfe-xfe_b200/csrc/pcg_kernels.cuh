@@ -61,6 +61,12 @@ constexpr int kPcgRowsPerWarp = 8;   // short rows per warp step
 constexpr int kPcgListsPerSm = 16;   // summation lists of C_fy' p_f per SM: the warps of the FP32 grid's CTA
 constexpr int kPcgMinCtas = 16;      // CTAs of the smallest launch
 constexpr int kPcgOwnRows = (kPcgMaxSG + kPcgMinCtas - 1) / kPcgMinCtas;  // small rows a CTA finishes, at most
+// Whether a launch of `ctas` CTAs can hold SG small rows: CTA b keeps rows b, b + ctas, ...
+// in kPcgOwnRows places.  Always so from kPcgMinCtas CTAs on; a device (or a
+// partition of one) with fewer SMs than that launches fewer.
+__host__ __device__ constexpr bool pcg_rows_fit(int ctas, int SG) {
+    return SG <= kPcgMaxSG && SG <= ctas * kPcgOwnRows;
+}
 // Rows of p gathered per iteration, in bytes, up to which the launch is one
 // cluster of kPcgMinCtas CTAs: there an iteration is a chain of L2 latencies
 // and barriers, and the hardware barrier of 16 CTAs with 16 partials to add is
