@@ -53,7 +53,9 @@ typedef struct b200fe_options {
     int precision;         /* B200FE_PREC_FP64 or B200FE_PREC_MIXED (default MIXED)           */
     int certify;           /* 1: compute abs_residual / abs_residual_rel on the device (1)    */
     int check_interval;    /* PCG iterations between host convergence checks (default 4)      */
-    int reuse_structure;   /* 1: ids and weights equal those of the previous call (0)         */
+    int reuse_structure;   /* 1: ids and weights equal those of the previous call (0); with two
+                              large FE dims beside the largest the structure differs by
+                              precision, and a call of the other one builds its own         */
     double inner_tol;      /* MIXED: relative tolerance of each FP32 inner solve (1e-5)       */
     int tolerance_mode;    /* certificate limit as the reference: 0 xhdfe-fast,
                               1 reghdfe-comparable (tol_eff = min(tol, 1e-9)), 2 strict (1)  */

@@ -410,6 +410,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     st.D = D;
     st.weighted = (w != nullptr);
     for (int d = 0; d < D; ++d) st.G[d] = G[d];
+    st.asked_two = ctx->sparse_two;
     // primary = most levels (first on ties)
     int p = 0;
     for (int d = 1; d < D; ++d)
@@ -1904,11 +1905,8 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
     Work<double> w64{};
     B_CHECK(prepare_work<double, CQ>(ctx, "w64_", w64));
     const bool mixed = (o.precision == B200FE_PREC_MIXED) && GR > 0;
-    // the inner solves of the mixed scheme run in FP32; in FP64 on a reused
-    // structure that holds the explicit block of two large dims
-    const bool inner32 = mixed && !st.two_large;
     Work<float> w32{};
-    if (inner32) B_CHECK(prepare_work<float, CQ>(ctx, "w32_", w32));
+    if (mixed) B_CHECK(prepare_work<float, CQ>(ctx, "w32_", w32));
 
     double *b64, *a64, *r64, *q64, *z64 = nullptr, *p64 = nullptr, *x64 = nullptr,
            *rin64 = nullptr;
@@ -1917,7 +1915,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
     B_CHECK(get_buf(ctx, "r64", GR * CP, &r64));
     B_CHECK(get_buf(ctx, "q64", GR * CP, &q64));
     float *x32 = nullptr, *r32 = nullptr, *z32 = nullptr, *p32 = nullptr, *q32 = nullptr;
-    if (inner32) {
+    if (mixed) {
         B_CHECK(get_buf(ctx, "x32", GR * CP, &x32));
         B_CHECK(get_buf(ctx, "r32", GR * CP, &r32));
         B_CHECK(get_buf(ctx, "z32", GR * CP, &z32));
@@ -2099,7 +2097,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
             B_CHECK(small_h2d(ctx, inv_scale_d, inv_scale.data(), sizeof(double) * CP));
             int its = 0;
             const int32_t* ctl = nullptr;  // words of a persistent inner solve
-            if (inner32) {
+            if (mixed) {
                 scale_rows_kernel<float><<<rgrid, kRowThreads, 0, s>>>(GR, CP, r64, inv_scale_d, r32);
                 B_LAUNCHED();
                 int prc = B200FE_UNAVAILABLE;
@@ -2141,7 +2139,7 @@ int solve_block(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
                 rb.add(dot_res, sizeof(double) * CP, rr.data());
                 if (ctl) rb.add(ctl, sizeof(hc), hc);
                 B_CHECK(rb.wait(ctx));
-                if (ctl) B_CHECK(pcg_outcome(ctx, hc, CP, inner32 ? sizeof(float) : sizeof(double), &its));
+                if (ctl) B_CHECK(pcg_outcome(ctx, hc, CP, mixed ? sizeof(float) : sizeof(double), &its));
             }
             total_iters += its;
             if (outer == 0) first_round_its = its;
@@ -2310,6 +2308,23 @@ int solve_all(b200fe_context* ctx, const double* d_v, int cols, double* d_out,
 
 
 
+// The matvec forms that a call's options ask for.
+void ask_forms(b200fe_context* ctx, const b200fe_options& o) {
+    // 3: the run-level matvec of the automatic choice, without the explicit block
+    ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
+    ctx->sparse_schur = o.pass_kernel == 0;
+    ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
+}
+
+// Whether the context's structure is that of this call (after ask_forms).  With
+// two large dims it differs by precision, so a call of the other one builds its
+// own: form and answer of a call do not depend on the calls before it.
+bool can_reuse(const b200fe_context* ctx, const b200fe_options& o, int64_t n, int num_dims, bool weighted) {
+    const Structure& st = ctx->st;
+    return o.reuse_structure && st.valid && st.n == n && st.D == num_dims && st.weighted == weighted &&
+           (st.nL != 2 || st.nS > 1 || st.asked_two == ctx->sparse_two);
+}
+
 int absorb_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int cols, int num_dims,
                        const int32_t* const* d_gids, const int32_t* G, const double* d_w,
                        const b200fe_options& o, double* d_out, b200fe_result* res) {
@@ -2327,13 +2342,9 @@ int absorb_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int co
     B_TRY(cudaEventCreate(&e1));
     B_TRY(cudaEventCreate(&e2));
     B_TRY(cudaEventRecord(e0, s));
-    const bool reuse = o.reuse_structure && ctx->st.valid && ctx->st.n == n &&
-                       ctx->st.D == num_dims && ctx->st.weighted == (d_w != nullptr);
+    ask_forms(ctx, o);
+    const bool reuse = can_reuse(ctx, o, n, num_dims, d_w != nullptr);
     ctx->profiling = o.profile != 0;
-    // 3: the run-level matvec of the automatic choice, without the explicit block
-    ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
-    ctx->sparse_schur = o.pass_kernel == 0;
-    ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
     ctx->prof.clear();
     ctx->ev_used = 0;
     if (!reuse) {
@@ -2493,15 +2504,12 @@ int absorb_host_pipelined(b200fe_context* ctx, const double* y, const double* X,
     B_CHECK(arrived(0));
     // the FE structure as soon as the ids are in, while the columns arrive
     int rc = B200FE_OK;
-    if (!(o.reuse_structure && ctx->st.valid && ctx->st.n == n && ctx->st.D == num_dims &&
-          ctx->st.weighted == (dw != nullptr)) && num_dims > 0) {
+    ask_forms(ctx, o);
+    if (num_dims > 0 && !can_reuse(ctx, o, n, num_dims, dw != nullptr)) {
         B_TRY(cudaStreamWaitEvent(s, ev_ids, 0));
         cudaEvent_t e0, e1;
         B_TRY(cudaEventCreate(&e0));
         B_TRY(cudaEventCreate(&e1));
-        ctx->pass_kernel = o.pass_kernel == 3 ? 0 : o.pass_kernel;
-        ctx->sparse_schur = o.pass_kernel == 0;
-        ctx->sparse_two = o.pass_kernel == 0 && o.precision == B200FE_PREC_FP64 && ctx->persistent;
         B_TRY(cudaEventRecord(e0, s));
         rc = build_structure(ctx, n, num_dims, dg, G, dw);
         B_TRY(cudaEventRecord(e1, s));

@@ -124,6 +124,7 @@ struct Structure {
     // rows instead of passing over the runs
     bool sparse = false;
     bool two_large = false;            // ... over two large dims, their rows one after the other
+    bool asked_two = false;            // built by a call that asks for it (FP64 throughout)
     int64_t lrows = 0;                 // rows of the large dims
     int64_t sp_pairs = 0;              // contributions before merging
     int64_t sp_nnz = 0;
