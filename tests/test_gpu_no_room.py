@@ -1,0 +1,59 @@
+"""No room on the device for a faster form's workspace: the call takes the form that
+needs less and gives the same answer.  B200FE_REFUSE at context creation refuses
+the named workspace as a full device would.
+
+Both forms stop at 1e-11 of ||b||; on these panels an error of the FE
+coefficients shows up in the within transform less than a hundredfold, so 1e-9
+of the column norm bounds the distance of either from the projection.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(pkg, monkeypatch, refuse, calls):
+    """What each call gives with and without the refused workspace; the refusing context serves all calls."""
+    monkeypatch.delenv("B200FE_REFUSE", raising=False)
+    free = pkg.Absorber(0)
+    monkeypatch.setenv("B200FE_REFUSE", refuse)
+    tight = pkg.Absorber(0)
+    monkeypatch.delenv("B200FE_REFUSE")
+    out = [(c(free), c(tight)) for c in calls]
+    free.close()
+    tight.close()
+    return out
+
+
+def _same(a, b, y, X):
+    assert a.converged and b.converged
+    assert a.kernel_launches != b.kernel_launches  # another form
+    for u, v, x in [(a.y_tilde, b.y_tilde, y[:, None])] + [(a.X_tilde, b.X_tilde, X)]:
+        u, v = u.reshape(x.shape), v.reshape(x.shape)
+        assert np.all(np.linalg.norm(u - v, axis=0) <= 1e-9 * np.linalg.norm(x, axis=0))
+
+
+@pytest.mark.parametrize("refuse", ["pc_tile_val", "pc_key,pc32_,pc64_", "pc32_ctl,pc64_ctl"])
+@pytest.mark.parametrize("years", [True, False])
+def test_persistent_pcg(pkg, panels, monkeypatch, refuse, years):
+    p = panels.akm_two_way(20_000, n_firms=600, n_years=12, seed=7, three_way=years)
+    X = np.column_stack([p.X, np.random.default_rng(0).standard_normal((p.n, 4))])
+    calls = [lambda a, k=k, c=c: a.absorb(p.y, X[:, :c], p.fes, p.levels, None, pkg.make_options(tol=1e-11, precision=k))
+             for k in ("mixed", "fp64") for c in (2, 6)]
+    for (a, b), c in zip(_pair(pkg, monkeypatch, refuse, calls), (2, 6, 2, 6)):
+        _same(a, b, p.y, X[:, :c])
+
+
+def test_tiles_of_both_precisions(pkg, panels):
+    """The tiles of a reused structure are built for the second precision when it comes."""
+    p = panels.akm_two_way(20_000, n_firms=600, n_years=12, seed=8, three_way=True)
+    run = lambda a, k, reuse: a.absorb(p.y, p.X, p.fes, p.levels, None, pkg.make_options(  # noqa: E731
+        tol=1e-9, precision=k, reuse_structure=reuse))
+    both = pkg.Absorber(0)
+    for i, k in enumerate(("mixed", "fp64", "mixed")):
+        one = pkg.Absorber(0)
+        a, b = run(one, k, False), run(both, k, i > 0)
+        assert np.array_equal(a.y_tilde, b.y_tilde) and np.array_equal(a.X_tilde, b.X_tilde)
+        one.close()
+    both.close()

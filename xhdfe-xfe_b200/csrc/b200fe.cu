@@ -356,8 +356,10 @@ int build_sparse_block(b200fe_context* ctx, int64_t pairs) {
     return B200FE_OK;
 }
 
-// Tiles of the short rows for a column pitch of 4 cq (PcgTiles): without a
-// coupled small dim one order serves every pitch.
+// Tiles of the short rows for a column pitch of 4 cq (PcgTiles) with values in T:
+// without a coupled small dim one order serves every pitch.  The other precision's
+// values come with the same tiles built again (the same bytes).
+template <typename T>
 int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
     Structure& st = ctx->st;
     const cudaStream_t s = ctx->stream;
@@ -365,7 +367,8 @@ int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
     const int slot = !coupled || cq == 1 ? 0 : cq == 2 ? 1 : 2;
     PcgTiles& t = st.pc_tiles[slot];
     *out = &t;
-    if (t.built) return B200FE_OK;
+    constexpr bool f32 = std::is_same<T, float>::value;
+    if (f32 ? t.val32 != nullptr : t.val64 != nullptr) return B200FE_OK;
     const std::string sfx = std::to_string(slot);
     const int sr = coupled ? 32 / cq : kPcgRowsPerWarp;
     const int lists = coupled ? kPcgListsPerSm * ctx->num_sms : 0;
@@ -374,6 +377,7 @@ int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
     const size_t t1 = static_cast<size_t>(t.n) + 1;
     const int64_t cap = st.sp_nnz + 4 * t.n + 4;  // every tile padded to a multiple of four entries
     int32_t *key, *row, *key_s, *row_s, *len, *off;
+    T* val;
     B_CHECK(get_buf(ctx, "pc_key", std::max<int64_t>(npad, 1), &key));
     B_CHECK(get_buf(ctx, "pc_row", std::max<int64_t>(npad, 1), &row));
     B_CHECK(get_buf(ctx, "pc_key_s", std::max<int64_t>(npad, 1), &key_s));
@@ -383,8 +387,7 @@ int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
     B_CHECK(get_buf(ctx, "pc_tile_meta" + sfx, t1, &t.meta));
     B_CHECK(get_buf(ctx, "pc_tile_rows" + sfx, t1 * kPcgRowsPerWarp, &t.rows));
     B_CHECK(get_buf(ctx, "pc_tile_col" + sfx, cap, &t.col));
-    B_CHECK(get_buf(ctx, "pc_tile_val64" + sfx, cap, &t.val64));
-    B_CHECK(get_buf(ctx, "pc_tile_val32" + sfx, cap, &t.val32));
+    B_CHECK(get_buf(ctx, (f32 ? "pc_tile_val32" : "pc_tile_val64") + sfx, cap, &val));
     if (npad > 0) {
         pcg_tile_key_kernel<<<grid_for(ctx, npad, 256), 256, 0, s>>>(st.sp_row_off, st.pc_short_rows, st.pc_nshort,
                                                                      npad, sr, lists, key, row);
@@ -395,10 +398,11 @@ int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
         B_LAUNCHED();
         B_CHECK(cub_exclusive_sum(ctx, len, off, static_cast<int64_t>(t1)));
         pcg_tile_fill_kernel<<<grid_for(ctx, t.n * 32, 256), 256, 0, s>>>(
-            st.sp_row_off, st.sp_col, st.sp_val64, row_s, t.n, off, t.meta, t.rows, t.col, t.val64, t.val32);
+            st.sp_row_off, st.sp_col, st.sp_val64, row_s, t.n, off, t.meta, t.rows, t.col, val);
         B_LAUNCHED();
     }
-    t.built = true;
+    if constexpr (f32) t.val32 = val;
+    else t.val64 = val;
     return B200FE_OK;
 }
 
@@ -1724,7 +1728,7 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     const bool coupled = st.coupled && st.nS == 1;
     const int SG = coupled ? st.SG : 0;
     const int SGP = coupled ? st.SGP : 0;
-    if (!pcg_rows_fit(ctx->num_sms, SG)) return B200FE_UNAVAILABLE;
+    if (st.pc_no_room || !pcg_rows_fit(ctx->num_sms, SG)) return B200FE_UNAVAILABLE;
     // two staging buffers of the coupling where they fit beside the rest
     const int cbuf = pcg_smem_bytes<T>(CP, SG, SGP, 2) <= 200 * 1024 ? 2 : 1;
     const size_t smem = pcg_smem_bytes<T>(CP, SG, SGP, cbuf);
@@ -1753,8 +1757,29 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     a.val = pick_prec<T>(st.sp_val32, st.sp_val64);
     a.nshort = st.pc_nshort;
     a.short_rows = st.pc_short_rows;
-    const PcgTiles* tiles;
-    B_CHECK(build_pcg_tiles(ctx, CQ, &tiles));
+    const PcgTiles* tiles = nullptr;
+    double* thr_d = nullptr;
+    int32_t *iters_d = nullptr, *ctl = nullptr;
+    auto buffers = [&]() -> int {
+        const std::string tag = std::is_same<T, float>::value ? "pc32_" : "pc64_";
+        B_CHECK(build_pcg_tiles<T>(ctx, CQ, &tiles));
+        B_CHECK(get_buf(ctx, tag + "lpart", static_cast<size_t>(std::max<int64_t>(st.pc_nlchunks, 1)) * CP, &a.lpart));
+        B_CHECK(get_buf(ctx, tag + "cta_part", static_cast<size_t>(nb_max) * a.part_stride, &a.cta_part));
+        B_CHECK(get_buf(ctx, tag + "thr", CP, &thr_d));
+        B_CHECK(get_buf(ctx, tag + "rz", CP, &a.rz_out));
+        B_CHECK(get_buf(ctx, tag + "iters", CP, &iters_d));
+        return get_buf(ctx, tag + "ctl", 4, &ctl);  // loops, status, barrier[2]
+    };
+    a.part_stride = CP * (3 + SG);
+    ctx->refused = false;
+    const int rc = buffers();
+    if (no_room(ctx, rc, {"pc_tile", "pc_key", "pc_row", "pc32_", "pc64_"})) {
+        // the multi-kernel PCG reads the block's rows as they are
+        for (PcgTiles& t : ctx->st.pc_tiles) t = PcgTiles{};
+        ctx->st.pc_no_room = true;
+        return B200FE_UNAVAILABLE;
+    }
+    if (rc != B200FE_OK) return rc;
     a.ntiles = tiles->n;
     a.tile_meta = tiles->meta;
     a.tile_rows = tiles->rows;
@@ -1775,17 +1800,7 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     a.r = r;
     a.p = p;
     a.q = q;
-    a.part_stride = CP * (3 + SG);
     a.max_iter = max_iter;
-    const std::string tag = std::is_same<T, float>::value ? "pc32_" : "pc64_";
-    B_CHECK(get_buf(ctx, tag + "lpart", static_cast<size_t>(std::max<int64_t>(st.pc_nlchunks, 1)) * CP, &a.lpart));
-    B_CHECK(get_buf(ctx, tag + "cta_part", static_cast<size_t>(nb_max) * a.part_stride, &a.cta_part));
-    double* thr_d;
-    B_CHECK(get_buf(ctx, tag + "thr", CP, &thr_d));
-    B_CHECK(get_buf(ctx, tag + "rz", CP, &a.rz_out));
-    int32_t *iters_d, *ctl;
-    B_CHECK(get_buf(ctx, tag + "iters", CP, &iters_d));
-    B_CHECK(get_buf(ctx, tag + "ctl", 4, &ctl));  // loops, status, barrier[2]
     a.iters_out = iters_d;
     a.loops_out = ctl;
     a.status = ctl + 1;
@@ -2637,6 +2652,7 @@ int b200fe_context_create(int device, b200fe_context** out) {
     if (const char* g = std::getenv("B200FE_GRAPHS")) ctx->graphs = std::strcmp(g, "0") != 0;
     if (const char* g = std::getenv("B200FE_PERSISTENT")) ctx->persistent = std::strcmp(g, "0") != 0;
     if (const char* g = std::getenv("B200FE_PIPELINE")) ctx->pipeline = std::strcmp(g, "0") != 0;
+    if (const char* g = std::getenv("B200FE_REFUSE")) ctx->refuse = g;
     if (const char* g = std::getenv("B200FE_STREAM")) ctx->stream_pass = std::strcmp(g, "0") != 0;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);

@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
+#include <initializer_list>
 #include <limits>
 #include <map>
 #include <memory>
@@ -57,13 +58,13 @@ struct LargeDim {
 };
 
 // Tiles of short rows of the explicit Schur block (pcg_kernels.cuh), built on
-// first use: with a coupled small dim they depend on the column pitch.
+// first use in the precision that uses them: with a coupled small dim they
+// depend on the column pitch.
 struct PcgTiles {
-    bool built = false;
     int64_t n = 0;
     int2 *meta = nullptr, *rows = nullptr;
     int32_t* col = nullptr;
-    double* val64 = nullptr;
+    double* val64 = nullptr;  // null: not built in this precision
     float* val32 = nullptr;
 };
 
@@ -141,6 +142,7 @@ struct Structure {
     int4* pc_lchunk_meta = nullptr;    // {row, begin, end, first} of the long-row chunks
     int64_t pc_nhuge = 0;
     int32_t* pc_huge_li = nullptr;
+    bool pc_no_room = false;           // the device had no room for the kernel's buffers
     // records of the regular tiles for the bulk-copy data passes
     // (stream_kernels.cuh); stream_ok when every one fits the staged sizes
     bool stream_ok = false;
@@ -173,6 +175,8 @@ struct b200fe_context {
     cudaStream_t stream = nullptr;
     std::string err;
     std::unordered_map<std::string, b200fe_host::Buf> bufs;
+    bool refused = false;  // a workspace allocation failed for lack of device memory (get_buf, no_room)
+    std::string refuse;    // B200FE_REFUSE at context creation (get_buf)
     b200fe_host::Structure st;
     long long launches = 0;
     long long lib_calls = 0;
@@ -273,6 +277,18 @@ inline const char* poison_filter() {
     return f;
 }
 
+// B200FE_REFUSE=<prefix>[,<prefix>] at context creation: new workspace whose name
+// begins with one of them is refused as if the device had no room for it, so that
+// what is done without it can be tested.
+inline bool refuse_buf(const b200fe_context* ctx, const std::string& name) {
+    for (size_t b = 0; b < ctx->refuse.size();) {
+        const size_t e = std::min(ctx->refuse.find(',', b), ctx->refuse.size());
+        if (e > b && name.compare(0, e - b, ctx->refuse, b, e - b) == 0) return true;
+        b = e + 1;
+    }
+    return false;
+}
+
 template <typename T>
 inline int get_buf(b200fe_context* ctx, const std::string& name, size_t count, T** out) {
     size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
@@ -285,9 +301,11 @@ inline int get_buf(b200fe_context* ctx, const std::string& name, size_t count, T
             b.p = nullptr;
             b.bytes = 0;
         }
-        cudaError_t e = cudaMalloc(&b.p, bytes);
+        const cudaError_t e = refuse_buf(ctx, name) ? cudaErrorMemoryAllocation : cudaMalloc(&b.p, bytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
+            b.p = nullptr;
+            ctx->refused = e == cudaErrorMemoryAllocation;
             ctx->err = "cudaMalloc(" + name + ", " + std::to_string(bytes) + " B): " +
                        cudaGetErrorString(e);
             return B200FE_CUDA_ERROR;
@@ -302,6 +320,23 @@ inline int get_buf(b200fe_context* ctx, const std::string& name, size_t count, T
     }
     *out = static_cast<T*>(b.p);
     return B200FE_OK;
+}
+
+// Whether an optional form, tried with ctx->refused cleared, failed (rc) only for
+// lack of device memory.  The workspace whose names begin with one of the prefixes
+// is then given back, for what is done in its place.
+inline bool no_room(b200fe_context* ctx, int rc, std::initializer_list<const char*> prefixes) {
+    if (rc == B200FE_OK || !ctx->refused) return false;
+    ctx->refused = false;
+    ctx->err.clear();
+    cudaStreamSynchronize(ctx->stream);
+    for (auto& [name, b] : ctx->bufs)
+        for (const char* p : prefixes)
+            if (b.p && name.compare(0, std::strlen(p), p) == 0) {
+                cudaFree(b.p);
+                b = Buf{};
+            }
+    return true;
 }
 
 // Raises a kernel's dynamic shared-memory limit to at least `bytes`.  The

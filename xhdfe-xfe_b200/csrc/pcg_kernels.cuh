@@ -1033,12 +1033,12 @@ __global__ void pcg_tile_len_kernel(const int32_t* __restrict__ row_off, const i
     }
 }
 // One warp per tile: lanes take (row, every fourth nonzero).
+template <typename T>
 __global__ void pcg_tile_fill_kernel(const int32_t* __restrict__ row_off, const int32_t* __restrict__ col,
                                      const double* __restrict__ val, const int32_t* __restrict__ srow,
                                      int64_t ntiles, const int32_t* __restrict__ off,
                                      int2* __restrict__ meta, int2* __restrict__ rows,
-                                     int32_t* __restrict__ tcol, double* __restrict__ tval64,
-                                     float* __restrict__ tval32) {
+                                     int32_t* __restrict__ tcol, T* __restrict__ tval) {
     constexpr int RW = kPcgRowsPerWarp;
     const int lane = threadIdx.x & 31, r = lane % RW;
     const int64_t nw = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
@@ -1058,10 +1058,8 @@ __global__ void pcg_tile_fill_kernel(const int32_t* __restrict__ row_off, const 
         if (lane == 0) meta[t] = make_int2(o, total);
         const int64_t d = 4 * static_cast<int64_t>(o) + e0;
         for (int j = lane / RW; j < n; j += 32 / RW) {
-            const double x = val[b + j];
             tcol[d + j] = col[b + j];
-            tval64[d + j] = x;
-            tval32[d + j] = static_cast<float>(x);
+            tval[d + j] = static_cast<T>(val[b + j]);
         }
     }
 }
