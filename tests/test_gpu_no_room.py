@@ -57,3 +57,22 @@ def test_tiles_of_both_precisions(pkg, panels):
         assert np.array_equal(a.y_tilde, b.y_tilde) and np.array_equal(a.X_tilde, b.X_tilde)
         one.close()
     both.close()
+
+
+@pytest.mark.parametrize("refuse", ["sp_count", "sp_kin", "sp_val64", "run_meta1", "cfy32", "chunk_beg_sp"])
+@pytest.mark.parametrize("years", [True, False])
+def test_block_of_two_large_dims(pkg, panels, monkeypatch, refuse, years):
+    if not years and refuse in ("run_meta1", "cfy32"):
+        pytest.skip("no coupled small dim, no such workspace")
+    p = panels.akm_two_way(20_000, n_firms=600, n_years=12, seed=9, three_way=True)
+    rng = np.random.default_rng(9)
+    spell = np.r_[True, (np.diff(p.fes[0]) != 0) | (np.diff(p.fes[1]) != 0)]
+    job = rng.integers(0, 150, int(spell.sum()))[np.cumsum(spell) - 1].astype(np.int32)
+    fes = [p.fes[0], p.fes[1], job] + ([p.fes[2]] if years else [])
+    G = [int(f.max()) + 1 for f in fes]
+    w = rng.lognormal(0.0, 0.5, p.n)
+    calls = [lambda a, r=r: a.absorb(p.y, p.X, fes, G, w, pkg.make_options(tol=1e-11, precision="fp64",
+                                                                       reuse_structure=r)) for r in (False, True)]
+    (a, b), (_, again) = _pair(pkg, monkeypatch, refuse, calls)
+    _same(a, b, p.y, p.X)
+    assert again.setup_ms == 0.0 and np.array_equal(again.y_tilde, b.y_tilde)

@@ -406,8 +406,8 @@ int build_pcg_tiles(b200fe_context* ctx, int cq, const PcgTiles** out) {
     return B200FE_OK;
 }
 
-int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const* gids,
-                    const int32_t* G, const double* w) {
+int build_structure_once(b200fe_context* ctx, int64_t n, int D, const int32_t* const* gids, const int32_t* G,
+                         const double* w) {
     Structure& st = ctx->st;
     st = Structure();
     st.n = n;
@@ -554,10 +554,12 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     st.w_rows = Wall;
     B_CHECK(get_buf(ctx, "diagE", std::max<int64_t>(st.GR, 1), &Eall));
 
+    // the second large dim's runs are kept beside the first's where the coupling reads both
+    auto runs_suffix = [&](int l) -> std::string { return l > 0 && ctx->sparse_two ? std::to_string(l) : ""; };
     // large dims: ids in primary order, runs, sorted run order, chunks, diagonal
     for (int l = 0; l < st.nL; ++l) {
         LargeDim& L = st.L[l];
-        const std::string sfx = std::to_string(l);
+        const std::string sfx = std::to_string(l), own = runs_suffix(l);
         B_CHECK(get_buf(ctx, "rid" + sfx, n, &L.rid));
         gather_kernel<int32_t><<<grid_for(ctx, n, T256), T256, 0, s>>>(gids[L.dim], st.pord, n,
                                                                         L.rid);
@@ -575,7 +577,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         B_CHECK(get_buf(ctx, "run_grp" + sfx, nr, &run_grp));
         L.run_grp = run_grp;
         B_CHECK(get_buf(ctx, "run_start" + sfx, static_cast<size_t>(nr) + 1, &run_start));
-        B_CHECK(get_buf(ctx, "run_seg" + sfx, nr, &run_seg));
+        B_CHECK(get_buf(ctx, "run_seg" + own, nr, &run_seg));
         L.run_start = run_start;
         run_fill_kernel<<<grid_for(ctx, n, T256), T256, 0, s>>>(rflags, run_id, gp, L.rid, n,
                                                                 run_grp, run_start, run_seg);
@@ -588,7 +590,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
         int32_t *riota, *sorted_runs, *sorted_grp;
         B_CHECK(get_buf(ctx, "tmp_n_a", n, &riota));  // flags no longer needed
         B_CHECK(get_buf(ctx, "sorted_runs", nr, &sorted_runs));
-        B_CHECK(get_buf(ctx, "sorted_grp" + sfx, nr, &sorted_grp));
+        B_CHECK(get_buf(ctx, "sorted_grp" + own, nr, &sorted_grp));
         iota_kernel<<<grid_for(ctx, nr, T256), T256, 0, s>>>(riota, nr);
         B_LAUNCHED();
         B_CHECK(cub_sort_pairs(ctx, run_grp, sorted_grp, riota, sorted_runs, nr, L.G));
@@ -739,7 +741,7 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
             }
             for (int l = 0; l < st.nL; ++l) {
                 const LargeDim& L = st.L[l];
-                const std::string sfx = std::to_string(l);
+                const std::string sfx = std::to_string(l), own = runs_suffix(l);
                 double* cfy = st.cfy64 + st.lbase[l] * SGP;
                 int2* seg_meta = st.seg_meta;
                 int4* run_meta = st.run_meta;
@@ -758,10 +760,10 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
                 int32_t *sorted_grp, *run_seg, *grp_off;
                 int4* frec;
                 double* frec_cf;
-                B_CHECK(get_buf(ctx, "sorted_grp" + sfx, L.nruns, &sorted_grp));
+                B_CHECK(get_buf(ctx, "sorted_grp" + own, L.nruns, &sorted_grp));
                 B_CHECK(get_buf(ctx, "fy_rec", L.nruns, &frec));
                 B_CHECK(get_buf(ctx, "fy_rec_cf", L.nruns, &frec_cf));
-                B_CHECK(get_buf(ctx, "run_seg" + sfx, L.nruns, &run_seg));
+                B_CHECK(get_buf(ctx, "run_seg" + own, L.nruns, &run_seg));
                 B_CHECK(get_buf(ctx, "grp_off" + sfx, static_cast<size_t>(L.G) + 1, &grp_off));
                 const int64_t nranges = (L.nruns + kFyRangeRuns - 1) / kFyRangeRuns;
                 double* cpart;
@@ -886,6 +888,25 @@ int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const*
     for (int d = 0; d < D; ++d) st.present[d] = G[d];
     st.valid = true;
     return B200FE_OK;
+}
+
+// The FE structure of a call.  No room for the explicit block of two large dims
+// (up to eight contributions a run, twice for their sort, and the coupling rows):
+// the structure of the observation passes, as without it.
+int build_structure(b200fe_context* ctx, int64_t n, int D, const int32_t* const* gids, const int32_t* G,
+                    const double* w) {
+    ctx->refused = false;
+    int rc = build_structure_once(ctx, n, D, gids, G, w);
+    if (ctx->sparse_two && ctx->st.nL == 2 &&
+        no_room(ctx, rc, {"sp_", "pc_", "cfy", "cyy", "fy_rec", "block_", "seg_meta", "run_meta", "run_w64", "run_w32",
+                          "run_seg1", "sorted_grp1", "chunk_grp_sp", "chunk_beg_sp", "chunk_end_sp", "chunk_whole_sp",
+                          "multi_grp_sp", "multi_c0_sp", "multi_c1_sp", "multi_s0_sp", "multi_s1_sp", "sup_c0_sp",
+                          "sup_c1_sp", "cub_tmp"})) {
+        ctx->sparse_two = false;
+        rc = build_structure_once(ctx, n, D, gids, G, w);
+        ctx->sparse_two = ctx->st.asked_two = true;  // what was asked for: the next such call reuses it
+    }
+    return rc;
 }
 
 // ---------------------------------------------------------------------------
