@@ -76,3 +76,10 @@ def test_block_of_two_large_dims(pkg, panels, monkeypatch, refuse, years):
     (a, b), (_, again) = _pair(pkg, monkeypatch, refuse, calls)
     _same(a, b, p.y, p.X)
     assert again.setup_ms == 0.0 and np.array_equal(again.y_tilde, b.y_tilde)
+
+
+def test_tile_records(pkg, panels, monkeypatch):
+    p = panels.akm_two_way(60_000, n_firms=900, n_years=12, seed=10, three_way=True)
+    call = lambda a: a.absorb(p.y, p.X, p.fes, p.levels, None, pkg.make_options(tol=1e-11))  # noqa: E731
+    (a, b), = _pair(pkg, monkeypatch, "stream_blob", [call])
+    _same(a, b, p.y, p.X)

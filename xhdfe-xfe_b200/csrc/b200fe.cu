@@ -149,11 +149,15 @@ int build_stream_meta(b200fe_context* ctx) {
     B_LAUNCHED();
     B_CHECK(cub_exclusive_sum(ctx, bsize, st.stream_boff, static_cast<int64_t>(nreg) + 1));
     // room for every record without waiting for their sizes (blob_layout: each
-    // of at most ten sections is padded to 16 bytes)
+    // of at most ten sections is padded to 16 bytes); the data passes do without
+    // the records where the device has none
     size_t room = static_cast<size_t>(nreg) * (2 * st.stream_aux_stride + 160 + 8 * st.nL) +
                   static_cast<size_t>(st.G[st.p]) * 10 + static_cast<size_t>(st.n) * 2 * st.nS;
     for (int l = 0; l < st.nL; ++l) room += static_cast<size_t>(st.L[l].nruns) * (l == 0 ? 10 : 6);
-    B_CHECK(get_buf(ctx, "stream_blob", room + 16, &st.stream_blob));
+    ctx->refused = false;
+    const int rc = get_buf(ctx, "stream_blob", room + 16, &st.stream_blob);
+    if (no_room(ctx, rc, {"stream_blob", "stream_meta", "stream_boff"})) return B200FE_OK;
+    if (rc != B200FE_OK) return rc;
     st.stream_flags = flags;  // read with the last wait of the build
     TileBlobArgs x{};
     x.nreg = nreg;
