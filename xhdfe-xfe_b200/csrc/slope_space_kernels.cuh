@@ -32,6 +32,15 @@ namespace b200fe {
 constexpr int kSpaceMaxCols = 32;      // columns of a lock step (a warp's lanes)
 constexpr int kSpaceMaxSmall = 64;     // basis columns of the small dims
 constexpr int kSpaceMaxRuns = 512;     // runs of one primary group (one lane slot walks them)
+// Rounds of C columns for S_Ly up to which the form is set up at once (never for a
+// solve that the start already satisfies).  A solve of one check interval, 4
+// iterations, on 1M rows takes 3.97 ms with the form and 3.95 by observation passes
+// with 3 rounds (13 columns, 36 levels), 4.41 and 4.00 with 4, 3.24 and 2.70 with 6
+// (6 columns), 4.66 and 2.82 with 16 (1 column, 16 levels).  With more rounds a check
+// interval of observation passes comes first, and the form follows when at its rate
+// more iterations than rounds are left: 8.0 ms for a solve of 52 iterations with 16
+// rounds (7.5 with the form at once, 15.4 by observation passes).
+constexpr int kSpaceFreeRounds = 3;
 constexpr int kSpaceRunBatch = 4;      // runs a slot has in flight (8: 76 us for 58 in the large dim's pass)
 constexpr int kSpaceSerialChunks = 4;  // more chunks of a group: a warp sums them first
 constexpr int kSpaceGroupBatch = 4;    // groups a thread of the vector updates has in flight

@@ -43,7 +43,8 @@ struct SpaceForm {
     int64_t NL = 0;    // its basis columns
     int Y = 0, Yp = 0; // the small dims' basis columns, rounded up to 8
     int64_t runs = 0;
-    int32_t* start = nullptr;
+    const int32_t *start = nullptr, *off = nullptr;  // L's runs: first row each, first run of each group
+    const double* mom = nullptr;                     // moments of L's chunks
     SlopeSpace sp{};
     SlopeDim chunks{};  // chunks of runs of L's groups (grp_ch, part, big)
     int32_t* big_list = nullptr;
@@ -57,10 +58,11 @@ struct SpaceForm {
 // Whether the CG dims (all but the primary p) suit the coefficient form: one
 // dimension of any size, the others of at most kSpaceMaxSmall basis columns, and
 // S_Ly no larger than the residual and its image (it is read once an iteration,
-// they four times by the observation passes).  Setting S_Ly up costs Y / C
-// iterations of the observation passes, hence the bound on Y per column: a solve
-// takes 40 to 80.  Lock steps of more columns than a warp's lanes stay with the
-// observation passes.
+// they four times by the observation passes).  S_Ly takes a gather and segment
+// pass over the observations for every C of its Y columns, hence the bound on Y
+// per column; whether a solve is worth that is seen once it runs
+// (kSpaceFreeRounds).  Lock steps of more columns than a warp's lanes stay with
+// the observation passes.
 bool space_applies(const SlopeDim* dims, const std::vector<int>& cg, int C, int64_t n, SpaceForm& f) {
     if (C > kSpaceMaxCols || cg.empty()) return false;
     f.L = cg[0];
@@ -348,10 +350,14 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
     SpaceForm sf;
     sf.on = schur && space_applies(dims, cg, C, n, sf);
     if (schur) {
-        for (int d : cg) {
+        // L last: its runs and moments are still there when the form is set up
+        std::vector<int> pair_order;
+        for (int d : cg)
+            if (!sf.on || d != sf.L) pair_order.push_back(d);
+        if (sf.on) pair_order.push_back(sf.L);
+        for (int d : pair_order) {
             SlopeDim& D = dims[d];
             const std::string sx = std::to_string(d);
-            const bool keep = sf.on && d == sf.L;  // its runs stay for the solve
             int32_t *flag, *pid, *start, *off;
             double* contrib;
             B_CHECK(get_buf(ctx, "sl_pflag", n, &flag));
@@ -361,7 +367,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             B_CHECK(cub_inclusive_sum(ctx, flag, pid, n));
             int np = 0;
             B_CHECK(sync_read_int(ctx, pid + (n - 1), 1, &np));
-            B_CHECK(get_buf(ctx, keep ? "sl_xstart" : "sl_pstart", static_cast<size_t>(np) + 1, &start));
+            B_CHECK(get_buf(ctx, "sl_pstart", static_cast<size_t>(np) + 1, &start));
             pair_start_kernel<<<grid_for(ctx, n + 1, T), T, 0, s>>>(flag, pid, n, start);
             B_LAUNCHED();
             B_CHECK(get_buf(ctx, "sl_contrib", static_cast<size_t>(np) * 3, &contrib));
@@ -372,7 +378,7 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             // per group sums of the pair planes: one block per group, fixed order
             int32_t* poff;
             double* csum;
-            B_CHECK(get_buf(ctx, keep ? "sl_xoff" : "sl_poff", static_cast<size_t>(D.G) + 1, &poff));
+            B_CHECK(get_buf(ctx, "sl_poff", static_cast<size_t>(D.G) + 1, &poff));
             B_CHECK(get_buf(ctx, "sl_csum", static_cast<size_t>(D.G) * 3, &csum));
             pair_offsets_kernel<<<grid_for(ctx, static_cast<int64_t>(D.G) + 1, T), T, 0, s>>>(
                 off, pid, D.G, n, np, poff);
@@ -396,15 +402,11 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
             schur_block_inverse_kernel<<<gb, T, 0, s>>>(D, cm, csum, const_cast<double*>(D.minv),
                                                         pop);
             B_LAUNCHED();
-            if (keep) {
+            if (sf.on && d == sf.L) {
                 sf.runs = np;
                 sf.start = start;
-                sf.fm.ch_beg = poff;  // replaced by the chunks' below
-                double* blk;
-                B_CHECK(get_buf(ctx, "sl_xblk", static_cast<size_t>(sf.NL) * D.nb, &blk));
-                slope_group_block_kernel<<<grid_for(ctx, D.G, T, 4), T, 0, s>>>(D, cm, blk);
-                B_LAUNCHED();
-                sf.dn.blk = blk;
+                sf.off = poff;
+                sf.mom = cm;
             }
         }
     }
@@ -438,134 +440,6 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
                 multi_chunks = list;
                 n_multi_chunks = total;
             }
-        }
-    }
-    // coefficient form: its buffers, the runs in both orders and their chunks in
-    // L's order
-    const int gD = sf.on ? static_cast<int>(std::max<int64_t>(
-                               1, std::min<int64_t>((sf.NL + 63) / 64, 2 * static_cast<int64_t>(ctx->num_sms))))
-                         : 0;
-    SlopeStepArgs sa{};
-    double *space_Sly = nullptr, *space_one = nullptr, *space_sc = nullptr, *space_dot = nullptr, *space_py = nullptr;
-    int* space_act = nullptr;
-    auto space_setup = [&]() -> int {
-        const SlopeDim &P = dims[p], &L = dims[sf.L];
-        sf.kp = P.nb;
-        sf.kd = L.nb;
-        const int K = sf.kp * sf.kd;
-        const int64_t np = sf.runs;
-        const int32_t* poff = sf.fm.ch_beg;
-        double *mom, *mom_p;
-        int32_t *prim, *keys, *ord, *grp, *woff, *most, *nch, *gch;
-        B_CHECK(get_buf(ctx, "sl_xmom", static_cast<size_t>(np) * K, &mom));
-        B_CHECK(get_buf(ctx, "sl_xmomp", static_cast<size_t>(np) * K, &mom_p));
-        B_CHECK(get_buf(ctx, "sl_xprim", np, &prim));
-        B_CHECK(get_buf(ctx, "sl_sorted", n, &keys));
-        B_CHECK(get_buf(ctx, "sl_xord", np, &ord));
-        B_CHECK(get_buf(ctx, "sl_xgrp", np, &grp));
-        B_CHECK(get_buf(ctx, "sl_xwoff", static_cast<size_t>(P.G) + 1, &woff));
-        B_CHECK(get_buf(ctx, "sl_xmost", 1, &most));
-        slope_run_moments_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, P, w, sf.start, np, mom, prim);
-        B_LAUNCHED();
-        B_CHECK(cub_sort_pairs(ctx, prim, keys, iota, ord, np, P.G));
-        segment_offsets_kernel<<<grid_for(ctx, np + 1, T), T, 0, s>>>(keys, np, P.G, woff);
-        B_LAUNCHED();
-        slope_run_order_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, sf.start, ord, np, K, mom, grp, mom_p);
-        B_LAUNCHED();
-        B_TRY(cudaMemsetAsync(most, 0, sizeof(int32_t), s));
-        longest_range_kernel<<<grid_for(ctx, P.G, T, 4), T, 0, s>>>(woff, P.G, most);
-        B_LAUNCHED();
-        B_CHECK(get_buf(ctx, "sl_nch", static_cast<size_t>(L.G) + 1, &nch));
-        B_CHECK(get_buf(ctx, "sl_xgch", static_cast<size_t>(L.G) + 1, &gch));
-        slope_chunk_count_kernel<<<grid_for(ctx, L.G + 1, T), T, 0, s>>>(poff, L.G, nch);
-        B_LAUNCHED();
-        B_CHECK(cub_exclusive_sum(ctx, nch, gch, static_cast<int64_t>(L.G) + 1));
-        int32_t *flag, *idx;
-        B_CHECK(get_buf(ctx, "sl_bflag", L.G, &flag));
-        B_CHECK(get_buf(ctx, "sl_bidx", L.G, &idx));
-        multi_chunk_flags_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(gch, nullptr, L.G, flag, kSpaceSerialChunks);
-        B_LAUNCHED();
-        B_CHECK(cub_exclusive_sum(ctx, flag, idx, L.G));
-        int h_most = 0, h_nch = 0, h_last[2] = {0, 0};
-        ReadBatch rb;
-        rb.add(most, sizeof(int), &h_most);
-        rb.add(gch + L.G, sizeof(int), &h_nch);
-        rb.add(idx + (L.G - 1), sizeof(int), &h_last[0]);
-        rb.add(flag + (L.G - 1), sizeof(int), &h_last[1]);
-        B_CHECK(rb.wait(ctx));
-        sf.on = h_most <= kSpaceMaxRuns;
-        if (sf.on) {
-            SlopeDim& X = sf.chunks;
-            X.G = L.G;
-            X.nb = L.nb;
-            X.has_a = L.has_a;
-            X.has_b = L.has_b;
-            X.grp_ch = gch;
-            X.nch = h_nch;
-            int32_t *cb, *ce;
-            B_CHECK(get_buf(ctx, "sl_xchb", h_nch, &cb));
-            B_CHECK(get_buf(ctx, "sl_xche", h_nch, &ce));
-            slope_chunk_fill_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(poff, L.G, gch, cb, ce, nullptr);
-            B_LAUNCHED();
-            B_CHECK(get_buf(ctx, "sl_xpart", static_cast<size_t>(h_nch) * L.nb * C, &X.part));
-            sf.n_big = h_last[0] + h_last[1];
-            if (sf.n_big > 0) {
-                B_CHECK(get_buf(ctx, "sl_xblist", sf.n_big, &sf.big_list));
-                compact_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(flag, idx, L.G, sf.big_list);
-                B_LAUNCHED();
-                B_CHECK(get_buf(ctx, "sl_xbig", static_cast<size_t>(sf.NL) * C, &X.big));
-            }
-            // the CG dims' coefficients: L's rows, then the small dims'
-            sf.sp.C = C;
-            sf.sp.RB = RB;
-            int64_t row = 0;
-            for (int pass = 0; pass < 2; ++pass)
-                for (int d : cg) {
-                    if ((d == sf.L) != (pass == 0)) continue;
-                    const int i = sf.sp.nd++;
-                    sf.sp.G[i] = dims[d].G;
-                    sf.sp.nb[i] = dims[d].nb;
-                    sf.sp.has_a[i] = dims[d].has_a;
-                    sf.sp.row0[i] = row;
-                    sf.sp.minv[i] = dims[d].minv;
-                    row += static_cast<int64_t>(dims[d].G) * dims[d].nb;
-                }
-            const size_t cw = static_cast<size_t>(row) * C;
-            B_CHECK(get_buf(ctx, "sl_xx", cw, &sf.x));
-            B_CHECK(get_buf(ctx, "sl_xs", cw, &sf.s));
-            B_CHECK(get_buf(ctx, "sl_xt", cw, &sf.t));
-            B_CHECK(get_buf(ctx, "sl_xp", cw, &sf.p));
-            sf.wk = SlopeWorkerArgs{woff, grp, mom_p, P.minv, P.has_a, P.G, C, sf.p, P.zv};
-            sf.fm = SlopeFirmArgs{cb, ce, h_nch, prim, mom, P.zv, C, X.part};
-            sf.dn.NL = sf.NL;
-            sf.dn.Y = sf.Y;
-            sf.dn.Yp = sf.Yp;
-            sf.dn.C = C;
-            sf.dn.p = sf.p;
-            sf.dn.grp_ch = gch;
-            sf.dn.part = X.part;
-            sf.dn.big = X.big;
-            sf.dn.t = sf.t;
-            const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
-            B_CHECK(get_buf(ctx, "sl_xly", std::max<size_t>(sly, 1), &space_Sly));
-            B_CHECK(get_buf(ctx, "sl_xyy", std::max(1, sf.Y * sf.Y), &sf.Syy));
-            B_CHECK(get_buf(ctx, "sl_xone", C, &space_one));
-            B_CHECK(get_buf(ctx, "sl_xsc", static_cast<size_t>(4) * C, &space_sc));
-            B_CHECK(get_buf(ctx, "sl_xact", static_cast<size_t>(2) * C, &space_act));
-            B_CHECK(get_buf(ctx, "sl_xdot", static_cast<size_t>(gD) * C, &space_dot));
-            B_CHECK(get_buf(ctx, "sl_xpy", std::max<size_t>(static_cast<size_t>(gD) * sf.Y * C, 1), &space_py));
-            sa.grid = grid_for(ctx, (row + RB - 1) / RB, 1, 2);
-            B_CHECK(get_buf(ctx, "sl_xpg", static_cast<size_t>(sa.grid) * C, &sa.part_g));
-        }
-        return B200FE_OK;
-    };
-    if (sf.on) {
-        const int rc = space_setup();
-        if (rc != B200FE_OK) {
-            // no room for it on the device: the observation passes, as without it
-            if (ctx->err.rfind("cudaMalloc(", 0) != 0) return rc;
-            ctx->err.clear();
-            sf.on = false;
         }
     }
     // ---- input norms and stop thresholds
@@ -801,7 +675,130 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         return B200FE_OK;
     };
 
-    // ---- coefficient form: S_Ly and S_yy, its vectors and its steps
+    // ---- coefficient form: its buffers, the runs in both orders and their chunks in
+    // L's order
+    const int gD = sf.on ? static_cast<int>(std::max<int64_t>(
+                               1, std::min<int64_t>((sf.NL + 63) / 64, 2 * static_cast<int64_t>(ctx->num_sms))))
+                         : 0;
+    SlopeStepArgs sa{};
+    double *space_Sly = nullptr, *space_one = nullptr, *space_sc = nullptr, *space_dot = nullptr, *space_py = nullptr;
+    int* space_act = nullptr;
+    auto space_setup = [&]() -> int {
+        const SlopeDim &P = dims[p], &L = dims[sf.L];
+        sf.kp = P.nb;
+        sf.kd = L.nb;
+        const int K = sf.kp * sf.kd;
+        const int64_t np = sf.runs;
+        const int32_t* poff = sf.off;
+        double *mom, *mom_p, *blk;
+        int32_t *prim, *keys, *ord, *grp, *woff, *most, *nch, *gch;
+        B_CHECK(get_buf(ctx, "sl_xmom", static_cast<size_t>(np) * K, &mom));
+        B_CHECK(get_buf(ctx, "sl_xblk", static_cast<size_t>(sf.NL) * sf.kd, &blk));
+        slope_group_block_kernel<<<grid_for(ctx, L.G, T, 4), T, 0, s>>>(L, sf.mom, blk);
+        B_LAUNCHED();
+        sf.dn.blk = blk;
+        B_CHECK(get_buf(ctx, "sl_xmomp", static_cast<size_t>(np) * K, &mom_p));
+        B_CHECK(get_buf(ctx, "sl_xprim", np, &prim));
+        B_CHECK(get_buf(ctx, "sl_sorted", n, &keys));
+        B_CHECK(get_buf(ctx, "sl_xord", np, &ord));
+        B_CHECK(get_buf(ctx, "sl_xgrp", np, &grp));
+        B_CHECK(get_buf(ctx, "sl_xwoff", static_cast<size_t>(P.G) + 1, &woff));
+        B_CHECK(get_buf(ctx, "sl_xmost", 1, &most));
+        slope_run_moments_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, P, w, sf.start, np, mom, prim);
+        B_LAUNCHED();
+        B_CHECK(cub_sort_pairs(ctx, prim, keys, iota, ord, np, P.G));
+        segment_offsets_kernel<<<grid_for(ctx, np + 1, T), T, 0, s>>>(keys, np, P.G, woff);
+        B_LAUNCHED();
+        slope_run_order_kernel<<<grid_for(ctx, np, T), T, 0, s>>>(L, sf.start, ord, np, K, mom, grp, mom_p);
+        B_LAUNCHED();
+        B_TRY(cudaMemsetAsync(most, 0, sizeof(int32_t), s));
+        longest_range_kernel<<<grid_for(ctx, P.G, T, 4), T, 0, s>>>(woff, P.G, most);
+        B_LAUNCHED();
+        B_CHECK(get_buf(ctx, "sl_nch", static_cast<size_t>(L.G) + 1, &nch));
+        B_CHECK(get_buf(ctx, "sl_xgch", static_cast<size_t>(L.G) + 1, &gch));
+        slope_chunk_count_kernel<<<grid_for(ctx, L.G + 1, T), T, 0, s>>>(poff, L.G, nch);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, nch, gch, static_cast<int64_t>(L.G) + 1));
+        int32_t *flag, *idx;
+        B_CHECK(get_buf(ctx, "sl_bflag", L.G, &flag));
+        B_CHECK(get_buf(ctx, "sl_bidx", L.G, &idx));
+        multi_chunk_flags_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(gch, nullptr, L.G, flag, kSpaceSerialChunks);
+        B_LAUNCHED();
+        B_CHECK(cub_exclusive_sum(ctx, flag, idx, L.G));
+        int h_most = 0, h_nch = 0, h_last[2] = {0, 0};
+        ReadBatch rb;
+        rb.add(most, sizeof(int), &h_most);
+        rb.add(gch + L.G, sizeof(int), &h_nch);
+        rb.add(idx + (L.G - 1), sizeof(int), &h_last[0]);
+        rb.add(flag + (L.G - 1), sizeof(int), &h_last[1]);
+        B_CHECK(rb.wait(ctx));
+        sf.on = h_most <= kSpaceMaxRuns;
+        if (sf.on) {
+            SlopeDim& X = sf.chunks;
+            X.G = L.G;
+            X.nb = L.nb;
+            X.has_a = L.has_a;
+            X.has_b = L.has_b;
+            X.grp_ch = gch;
+            X.nch = h_nch;
+            int32_t *cb, *ce;
+            B_CHECK(get_buf(ctx, "sl_xchb", h_nch, &cb));
+            B_CHECK(get_buf(ctx, "sl_xche", h_nch, &ce));
+            slope_chunk_fill_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(poff, L.G, gch, cb, ce, nullptr);
+            B_LAUNCHED();
+            B_CHECK(get_buf(ctx, "sl_xpart", static_cast<size_t>(h_nch) * L.nb * C, &X.part));
+            sf.n_big = h_last[0] + h_last[1];
+            if (sf.n_big > 0) {
+                B_CHECK(get_buf(ctx, "sl_xblist", sf.n_big, &sf.big_list));
+                compact_kernel<<<grid_for(ctx, L.G, T), T, 0, s>>>(flag, idx, L.G, sf.big_list);
+                B_LAUNCHED();
+                B_CHECK(get_buf(ctx, "sl_xbig", static_cast<size_t>(sf.NL) * C, &X.big));
+            }
+            // the CG dims' coefficients: L's rows, then the small dims'
+            sf.sp.C = C;
+            sf.sp.RB = RB;
+            int64_t row = 0;
+            for (int pass = 0; pass < 2; ++pass)
+                for (int d : cg) {
+                    if ((d == sf.L) != (pass == 0)) continue;
+                    const int i = sf.sp.nd++;
+                    sf.sp.G[i] = dims[d].G;
+                    sf.sp.nb[i] = dims[d].nb;
+                    sf.sp.has_a[i] = dims[d].has_a;
+                    sf.sp.row0[i] = row;
+                    sf.sp.minv[i] = dims[d].minv;
+                    row += static_cast<int64_t>(dims[d].G) * dims[d].nb;
+                }
+            const size_t cw = static_cast<size_t>(row) * C;
+            B_CHECK(get_buf(ctx, "sl_xx", cw, &sf.x));
+            B_CHECK(get_buf(ctx, "sl_xs", cw, &sf.s));
+            B_CHECK(get_buf(ctx, "sl_xt", cw, &sf.t));
+            B_CHECK(get_buf(ctx, "sl_xp", cw, &sf.p));
+            sf.wk = SlopeWorkerArgs{woff, grp, mom_p, P.minv, P.has_a, P.G, C, sf.p, P.zv};
+            sf.fm = SlopeFirmArgs{cb, ce, h_nch, prim, mom, P.zv, C, X.part};
+            sf.dn.NL = sf.NL;
+            sf.dn.Y = sf.Y;
+            sf.dn.Yp = sf.Yp;
+            sf.dn.C = C;
+            sf.dn.p = sf.p;
+            sf.dn.grp_ch = gch;
+            sf.dn.part = X.part;
+            sf.dn.big = X.big;
+            sf.dn.t = sf.t;
+            const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
+            B_CHECK(get_buf(ctx, "sl_xly", std::max<size_t>(sly, 1), &space_Sly));
+            B_CHECK(get_buf(ctx, "sl_xyy", std::max(1, sf.Y * sf.Y), &sf.Syy));
+            B_CHECK(get_buf(ctx, "sl_xone", C, &space_one));
+            B_CHECK(get_buf(ctx, "sl_xsc", static_cast<size_t>(4) * C, &space_sc));
+            B_CHECK(get_buf(ctx, "sl_xact", static_cast<size_t>(2) * C, &space_act));
+            B_CHECK(get_buf(ctx, "sl_xdot", static_cast<size_t>(gD) * C, &space_dot));
+            B_CHECK(get_buf(ctx, "sl_xpy", std::max<size_t>(static_cast<size_t>(gD) * sf.Y * C, 1), &space_py));
+            sa.grid = grid_for(ctx, (row + RB - 1) / RB, 1, 2);
+            B_CHECK(get_buf(ctx, "sl_xpg", static_cast<size_t>(sa.grid) * C, &sa.part_g));
+        }
+        return B200FE_OK;
+    };
+    // S_Ly and S_yy, its vectors and its steps
     SchurGatherArgs sgx = sga;  // the image of the coefficients x
     SlopeScalars scal[2] = {};
     double* ones = nullptr;
@@ -826,7 +823,21 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         }
         return i;
     };
-    if (sf.on) {
+    // the form from the residual as it is, whose chunk sums the last gradient left
+    auto space_start = [&]() -> int {
+        int rc;
+        {
+            ProfScope ps(ctx, B200FE_PROF_SETUP, 0.0);
+            rc = space_setup();
+        }
+        if (rc != B200FE_OK) {
+            // no room for it on the device: the observation passes, as without it
+            if (ctx->err.rfind("cudaMalloc(", 0) != 0) return rc;
+            ctx->err.clear();
+            sf.on = false;
+        }
+        if (!sf.on) return B200FE_OK;
+        for (int d : cg) B_CHECK(chunk_sums(d, C, C, sf.s + sf.sp.row0[space_dim(d)] * C));
         for (int i = 0; i < sgx.nd; ++i) sgx.dim[i].p = sf.x + sf.sp.row0[space_dim(cg[i])] * C;
         const size_t sly = static_cast<size_t>((sf.NL + 7) / 8 * 8) * sf.Yp;
         const std::vector<double> h1(C, 1.0);
@@ -861,7 +872,8 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         sa.s = sf.s;
         sa.t = sf.t;
         sa.done = done;
-    }
+        return B200FE_OK;
+    };
     int side = 0;  // which set of scalars the next step reads
     auto space_step = [&](bool first) -> int {
         if (!first) {
@@ -912,34 +924,10 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         return B200FE_OK;
     };
 
-    if (schur) B_CHECK(project(R, false));
-    B_CHECK(gradient(false, true));
     const int ci = std::max(1, o.check_interval);
     const int max_it = o.max_iter > 0 ? o.max_iter : 10000;
     int it = 0, hd = 0;
-    B_CHECK(sync_read_int(ctx, done, 1, &hd));
-    // the residual follows the coefficients, and its gradient decides; what two
-    // more starts from it do not settle is left to the observation passes
-    for (int start = 0; sf.on && start < 3 && !hd && it < max_it; ++start) {
-        for (int d : cg) B_CHECK(chunk_sums(d, C, C, sf.s + sf.sp.row0[space_dim(d)] * C));
-        B_CHECK(space_step(true));
-        int stop = 0;
-        while (!stop && it < max_it) {
-            const int steps = std::min(ci, max_it - it);
-            for (int k = 0; k < steps; ++k) B_CHECK(space_step(false));
-            it += steps;
-            B_CHECK(sync_read_int(ctx, done, 1, &stop));
-        }
-        B_CHECK(schur_gather(sgx));
-        {
-            ProfScope ps(ctx, B200FE_PROF_VECTOR, 24.0 * n * C);
-            slope_update_kernel<<<grid_for(ctx, n * C, T), T, 0, s>>>(R, Q, ones, n, C);
-            B_LAUNCHED();
-        }
-        B_CHECK(gradient(false, true));
-        B_CHECK(sync_read_int(ctx, done, 1, &hd));
-    }
-    while (!hd && it < max_it) {
+    auto observation_steps = [&]() -> int {
         const int steps = std::min(ci, max_it - it);
         for (int k = 0; k < steps; ++k) {
             if (schur) {
@@ -962,7 +950,54 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
         }
         it += steps;
         B_CHECK(sync_read_int(ctx, done, 1, &hd));
+        return B200FE_OK;
+    };
+    if (schur) B_CHECK(project(R, false));
+    B_CHECK(gradient(false, true));
+    B_CHECK(sync_read_int(ctx, done, 1, &hd));
+    // The coefficient form only where iterations are left that pay for its set-up
+    // (kSpaceFreeRounds)
+    const int rounds = (sf.Y + C - 1) / C;
+    if (sf.on && rounds > kSpaceFreeRounds) {
+        std::vector<double> before(C), now(C);
+        B_CHECK(sync_read_double(ctx, gamma, C, now.data()));
+        for (double left = 0.0; sf.on && !hd && it < max_it && left <= rounds;) {
+            const int it0 = it;
+            before.swap(now);
+            B_CHECK(observation_steps());
+            B_CHECK(sync_read_double(ctx, gamma, C, now.data()));
+            left = 0.0;  // iterations to the threshold at this block's rate, the slowest column's
+            for (int c = 0; c < C; ++c)
+                if (now[c] > thr[c])
+                    left = now[c] < before[c] ? std::max(left, (it - it0) * std::log(now[c] / thr[c]) /
+                                                                   std::log(before[c] / now[c]))
+                                              : std::numeric_limits<double>::infinity();
+        }
     }
+    if (sf.on && !hd && it < max_it) B_CHECK(space_start());
+    // the residual follows the coefficients, and its gradient decides; what two
+    // more starts from it do not settle is left to the observation passes
+    for (int start = 0; sf.on && start < 3 && !hd && it < max_it; ++start) {
+        if (start > 0)
+            for (int d : cg) B_CHECK(chunk_sums(d, C, C, sf.s + sf.sp.row0[space_dim(d)] * C));
+        B_CHECK(space_step(true));
+        int stop = 0;
+        while (!stop && it < max_it) {
+            const int steps = std::min(ci, max_it - it);
+            for (int k = 0; k < steps; ++k) B_CHECK(space_step(false));
+            it += steps;
+            B_CHECK(sync_read_int(ctx, done, 1, &stop));
+        }
+        B_CHECK(schur_gather(sgx));
+        {
+            ProfScope ps(ctx, B200FE_PROF_VECTOR, 24.0 * n * C);
+            slope_update_kernel<<<grid_for(ctx, n * C, T), T, 0, s>>>(R, Q, ones, n, C);
+            B_LAUNCHED();
+        }
+        B_CHECK(gradient(false, true));
+        B_CHECK(sync_read_int(ctx, done, 1, &hd));
+    }
+    while (!hd && it < max_it) B_CHECK(observation_steps());
     // Schur form: the primary's share of the certificate, ||D_p' W r||^2
     std::vector<double> nu_p(C, 0.0);
     if (schur) {
