@@ -83,3 +83,16 @@ def test_tile_records(pkg, panels, monkeypatch):
     call = lambda a: a.absorb(p.y, p.X, p.fes, p.levels, None, pkg.make_options(tol=1e-11))  # noqa: E731
     (a, b), = _pair(pkg, monkeypatch, "stream_blob", [call])
     _same(a, b, p.y, p.X)
+
+
+@pytest.mark.parametrize("refuse", ["sl_xblk", "sl_xmom", "sl_xprim", "sl_xly", "sl_xpg", "sl_x"])
+@pytest.mark.parametrize("cols", [2, 9])  # the form after a check interval, and at once
+def test_slopes_in_coefficient_space(pkg, panels, monkeypatch, refuse, cols):
+    p = panels.akm_two_way(30_000, n_firms=400, n_years=12, seed=11, three_way=True)
+    rng = np.random.default_rng(11)
+    z, X = rng.standard_normal(p.n), np.column_stack([p.X, rng.standard_normal((p.n, 6))])[:, : cols - 1]
+    call = lambda a: a.absorb(p.y, X, p.fes, p.levels, None, pkg.make_options(tol=1e-11),  # noqa: E731
+                              slopes=[(1, z, True)])
+    (a, b), (_, again) = _pair(pkg, monkeypatch, refuse, [call, call])
+    _same(a, b, p.y, X)
+    assert np.array_equal(again.y_tilde, b.y_tilde) and again.kernel_launches == b.kernel_launches

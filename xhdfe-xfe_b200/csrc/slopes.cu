@@ -826,16 +826,15 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
     // the form from the residual as it is, whose chunk sums the last gradient left
     auto space_start = [&]() -> int {
         int rc;
+        ctx->refused = false;
         {
             ProfScope ps(ctx, B200FE_PROF_SETUP, 0.0);
             rc = space_setup();
         }
-        if (rc != B200FE_OK) {
-            // no room for it on the device: the observation passes, as without it
-            if (ctx->err.rfind("cudaMalloc(", 0) != 0) return rc;
-            ctx->err.clear();
-            sf.on = false;
-        }
+        // no room for it on the device: the observation passes go on, whose own
+        // workspace is all there by now, and the form's is given back
+        if (no_room(ctx, rc, {"sl_x"})) sf.on = false;
+        else if (rc != B200FE_OK) return rc;
         if (!sf.on) return B200FE_OK;
         for (int d : cg) B_CHECK(chunk_sums(d, C, C, sf.s + sf.sp.row0[space_dim(d)] * C));
         for (int i = 0; i < sgx.nd; ++i) sgx.dim[i].p = sf.x + sf.sp.row0[space_dim(cg[i])] * C;
