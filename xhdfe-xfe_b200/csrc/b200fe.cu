@@ -1723,15 +1723,15 @@ int pcg(b200fe_context* ctx, const Work<T>& wk, const T* wp, const T* run_w, con
 
 // Algorithmic bytes of one persistent PCG iteration: the explicit block
 // (column and value per nonzero, row offsets, the p rows gathered and the q
-// rows written once), the coupling rows, and the vector updates (x, r, z, p,
-// q, dinv read; x, r, z written; z, p read and p written for the directions).
+// rows written once), the coupling rows, and the vector updates (r, q, dinv read
+// and r written; then r, p, x, dinv read and x, p written).
 double pcg_iter_bytes(const Structure& st, int CP, size_t tsize) {
     const double tb = static_cast<double>(tsize);
     const double gf = static_cast<double>(st.lrows);
     const double gr = static_cast<double>(st.GR);
     double b = static_cast<double>(st.sp_nnz) * (4.0 + tb) + gf * 4.0 + 2.0 * gf * CP * tb;
     if (st.coupled && st.nS == 1) b += gf * st.SGP * tb;
-    b += gr * CP * tb * 11.0 + gr * tb;
+    b += gr * CP * tb * 8.0 + 2.0 * gr * tb;
     return b;
 }
 
