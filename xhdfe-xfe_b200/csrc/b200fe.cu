@@ -648,9 +648,12 @@ int build_structure_once(b200fe_context* ctx, int64_t n, int D, const int32_t* c
     // With two large dims the explicit block replaces the pass over the
     // observations in solves that run in FP64 throughout, wherever its
     // contributions fit (2M rows, worker/firm/year/occupation, 9 columns: 7.2 ms
-    // for 31.1).  The FP32 inner solves of the
-    // mixed scheme keep the pass: their answers carry its roundings (R in FP32
-    // per run), up to 1e-7 of a column in badly identified rows.  The pairs are
+    // for 31.4 with 52 iterations, 3.1 for 7.5 with 8).  The limit of eight a run
+    // (count_sparse_pairs) lies where it still gains: 1M rows, 9 columns with a move in
+    // 20% of the years 5.5 ms for 15.5, in 30% 6.2 for 14.1; 40% is over it.  The FP32
+    // inner solves of the mixed scheme keep the pass: their answers carry its
+    // roundings (R in FP32 per run), up to 1e-7 of a column in badly identified
+    // rows, and another form would move them by as much.  The pairs are
     // counted here, since the small dim's diagonal then comes from the coupling.
     const bool block_ok = st.GR > 0 && st.nL <= 1 && st.nS <= 1;
     int64_t pairs = -1, coupled_rows = st.lrows * st.SG, run_room = 0;
@@ -1762,7 +1765,13 @@ int pcg_persistent(b200fe_context* ctx, const Work<T>& wk, const T* dinv, T* x, 
     // barrier (kPcgClusterBytes); the others, and all where a cluster of that
     // size cannot be launched: a cooperative launch of one CTA per SM
     const bool cluster = pcg_gather_bytes(st, CP, sizeof(T)) <= kPcgClusterBytes;
-    // levels per lane of the coupling: none, or SG over the 32 / CQ lanes of a column quad
+    // levels per lane of the coupling: none, or SG over the 32 / CQ lanes of a column
+    // quad.  16 columns have two forms: 5 a lane (up to 40 levels) and 8 (all 64), since
+    // the sums of 8 take the registers that the gathers would have in flight: 36
+    // levels, 5M rows 6.05 ms a call with 5 and 6.33 with 8 (1M rows 3.00 and 3.10).
+    // 3 a lane (24 levels) gains nothing for 10 or 20 on the grid (5.70 and 5.70 ms, 5.49
+    // and 5.52), a sixth of the PCG in a cluster (100k rows, 20 levels: 21.6 us an
+    // iteration for 25.9).
     constexpr int KF = 2 * CQ, KS = CQ == 4 ? 5 : KF;
     using Kernel = void (*)(PcgArgs<T>);
     const Kernel kern_cluster = SG == 0             ? pcg_persistent_kernel<T, CQ, 0, true>
@@ -3094,7 +3103,6 @@ void ldlt_solve(const Ldlt& f, std::vector<long double>& b) {
     for (int k = 0; k < p; ++k) b[f.perm[k]] = y[k];
 }
 
-// sum_i f_i a_i b_i over the column pairs, summed over CTAs; out [npairs]
 // 16-byte aligned columns at base + j * ld
 bool vector_columns(const double* base, int64_t ld, int cols) {
     return (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (cols <= 1 || (ld & 1) == 0);

@@ -3,9 +3,9 @@
 //
 // A cudaMemcpyAsync of pageable memory is staged by the driver with one core:
 // 152 MB in took 12 ms and 128 MB out 22 ms of a 50 ms call on 2M rows, 8 columns
-// (three dims), and the calling thread is busy meanwhile.  With 8 workers on 16
-// cores the call takes 12.2 ms (52.5 before; its first, with the pinned slots to
-// get, 47 for 81); the PCIe transfers alone need 5.  Here the arrays
+// (three dims), and the calling thread is busy meanwhile.  With workers on half of
+// 16 cores (kStageWorkers at most) the call takes 12.7 ms (50.8 before; its first,
+// with the pinned slots to get, 47 for 81); the PCIe transfers alone need 5.  Here the arrays
 // are cut into pieces of kStagePiece; a worker copies a piece into its own
 // pinned slot and submits the slot's transfer, or submits a transfer into its
 // slot and copies it out (taking the page faults of the result there).  No piece
@@ -26,7 +26,9 @@ namespace b200fe_host {
 constexpr size_t kStagePiece = size_t(1) << 20;
 constexpr int kStageSlots = 2;          // pinned slots per worker
 constexpr int kStageWorkers = 12;       // at most
-constexpr size_t kStageMinBytes = size_t(8) << 20;  // smaller calls copy directly
+// Calls with fewer bytes of columns copy directly, the threads would cost more: 3
+// columns, 7 MB 3.9 ms staged and 3.1 directly, 14 MB 4.4 and 4.7, 46 MB 7.2 and 12.7.
+constexpr size_t kStageMinBytes = size_t(8) << 20;
 
 // Memory that only a staged copy can move (neither pinned nor registered).
 inline bool pageable(const void* p) {

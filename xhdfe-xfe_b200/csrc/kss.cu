@@ -17,8 +17,9 @@
 //     group of lanes per worker, matches in worker order) and a firm pass
 //     Ap = Df p - B' t over the matches in firm order, cut into chunks of at
 //     most kChunk matches so a firm with a large share of the matches (Zipf
-//     firm sizes) is summed by many groups; chunk partials are combined per
-//     firm in chunk order (fixed order, no atomics);
+//     firm sizes) is summed by many groups; a CTA combines the chunk partials
+//     of such a firm, strided over its groups and then in a tree (fixed order,
+//     no atomics);
 //   * the PCG scalars (alpha, beta, convergence, per-lane iteration counts and
 //     retirement) are computed on the device by the last CTA of each
 //     reduction, so a PCG step has no host round trip; the host reads one
@@ -293,8 +294,9 @@ __device__ void kss_action(KssScalars* sc, int action, int l, double d0, double 
     }
 }
 
-// Block partials of one or two per-lane dots, then the last CTA sums the
-// partials in block order and runs the scalar step.
+// Block partials of one or two per-lane dots, then the last CTA sums them (every
+// thread of a lane a fixed slice of the blocks, the slices in order) and runs the
+// scalar step.
 template <int LW, int NDOT>
 __device__ __forceinline__ void kss_reduce_tail(double s0, double s1, double* __restrict__ part,
                                                 KssScalars* sc, int action) {

@@ -30,8 +30,12 @@
 //
 // Data written by other CTAs during the launch is read with ld.global.cg (L2;
 // L1 is not coherent across CTAs).  Every sum has a fixed order, so results
-// are bitwise reproducible.  The barrier's wait is bounded (kBarrierCycles):
-// on timeout it sets *status and every CTA leaves at its next barrier.
+// are bitwise reproducible on devices of one number of SMs.  The launch is
+// cooperative, one CTA per SM, and its barrier's wait is bounded (kBarrierCycles
+// of clock64: on timeout it sets *status and every CTA leaves at its next
+// barrier); or it is one thread-block cluster (kPcgClusterBytes), whose CTAs the
+// device schedules together and which meet at the hardware's cluster barrier:
+// that wait has no limit of its own, and no CTA leaves before the others.
 //
 // What bounds it: small systems by latency (three barriers and some ten
 // dependent L2 reads an iteration), large ones by the gathers of p from L2,
@@ -41,9 +45,9 @@
 // address (an LDS.128 then takes 2 cycles instead of 4), rows in tiles of
 // equal length (no lane of a warp waits for another row's nonzeros), and FP32
 // -> FP64 by shifts in the gathers.  Per iteration (B200, FP32): 10k rows
-// 2-way, 4 columns 28.0 -> 9.4 us; 300k rows 3-way, 4 columns 47 -> 19; 5M rows
-// 3-way, 16 columns 72 -> 44; 50M rows 366 -> 251; FP64, 1M rows 3-way, 16
-// columns 46 -> 32.
+// 2-way, 4 columns 28.0 -> 9.5 us; 300k rows 3-way, 4 columns 47 -> 19; 5M rows
+// 3-way, 16 columns 72 -> 41 to 44; 50M rows 366 -> 248; FP64, 1M rows 3-way, 16
+// columns 46 -> 30 to 32.
 #pragma once
 
 #include <cstdint>
@@ -70,10 +74,13 @@ __host__ __device__ constexpr bool pcg_rows_fit(int ctas, int SG) {
 // Rows of p gathered per iteration, in bytes, up to which the launch is one
 // cluster of kPcgMinCtas CTAs: there an iteration is a chain of L2 latencies
 // and barriers, and the hardware barrier of 16 CTAs with 16 partials to add is
-// shorter than the grid's; above it 16 SMs are too few.  Per iteration on B200
-// (FP32, 4 columns), cluster against grid: 10k rows 2-way 9.5 / 12.6 us, 100k
-// rows 2-way 10.0 / 12.9, 300k rows 3-way (about 1 MB) 16.6 / 16.6, 1M rows
-// 2-way 19.6 / 13.7.
+// shorter than the grid's; above it 16 SMs are too few.  us an iteration on B200,
+// cluster / grid, at that many MB: 2-way panels of 10k to 1M rows in FP32 with 4
+// columns 0.03: 9.3 / 13.4, 0.25: 9.9 / 13.1, 0.72: 11.8 / 13.3, 2.3: 21.8 / 14.1,
+// with 16 columns 0.32: 11.7 / 16.2, 1.0: 13.4 / 16.4, 2.9: 17.7 / 16.4; in FP64 with
+// 4 columns 0.50: 9.6 / 11.8, 1.4: 13.8 / 12.0, with 16 columns 0.64: 12.4 / 17.3,
+// 2.0: 16.3 / 17.4, 5.8: 30.0 / 17.8.  3-way, 20 levels: FP32 0.72: 19.6 / 20.6; FP64,
+// 16 columns 0.65: 17.0 / 21.6, 2.0: 24.9 / 22.3.
 constexpr double kPcgClusterBytes = 1e6;
 constexpr long long kBarrierCycles = 4000000000LL;  // ~2 s at 1.9 GHz
 
@@ -289,9 +296,10 @@ __device__ __forceinline__ void couple_dot(const T* crow, const T* xs, int SGP, 
 // v, v + lists, ... of 32 / CQ short rows in row order), the lists' sums in
 // FP64; a warp takes whole lists.  C_fy's rows cancel (a balanced row sums to
 // zero over the levels), so the rounding of these FP32 sums shows in badly
-// identified rows of the answer: neither the lists nor the level order of
-// C_fy p_small depend on the launch, and the answer depends on it only through
-// FP64 rounding.
+// identified rows of the answer: the lists follow from the number of SMs
+// (kPcgListsPerSm each), and neither they nor the level order of C_fy p_small
+// depend on whether the launch is a cluster or the grid, so that the answer
+// depends on that only through FP64 rounding.
 template <typename T, int CQ, int KH, bool CLUSTER>
 __global__ void __launch_bounds__(pcg_threads<T>(), 1) pcg_persistent_kernel(const PcgArgs<T> a) {
     constexpr unsigned kFull = 0xffffffffu;

@@ -31,7 +31,11 @@ namespace b200fe {
 
 constexpr int kSpaceMaxCols = 32;      // columns of a lock step (a warp's lanes)
 constexpr int kSpaceMaxSmall = 64;     // basis columns of the small dims
-constexpr int kSpaceMaxRuns = 512;     // runs of one primary group (one lane slot walks them)
+// Runs of one primary group (one lane slot walks them).  A call of 8 iterations, 7
+// columns, every primary group with about 420 runs (1M rows) takes 3.8 ms with the form
+// and 4.7 by observation passes; with 1,250 (4M rows) 11.5 and 10.7, with 2,200
+// (16M rows) 28.9 and 34.8: above the limit it depends on the rows.
+constexpr int kSpaceMaxRuns = 512;
 // Rounds of C columns for S_Ly up to which the form is set up at once (never for a
 // solve that the start already satisfies).  A solve of one check interval, 4
 // iterations, on 1M rows takes 3.97 ms with the form and 3.95 by observation passes
