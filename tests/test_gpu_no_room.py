@@ -86,7 +86,7 @@ def test_tile_records(pkg, panels, monkeypatch):
 
 
 @pytest.mark.parametrize("refuse", ["sl_xblk", "sl_xmom", "sl_xprim", "sl_xly", "sl_xpg", "sl_x"])
-@pytest.mark.parametrize("cols", [2, 9])  # the form after a check interval, and at once
+@pytest.mark.parametrize("cols", [1, 9])  # the form after a check interval, and at once
 def test_slopes_in_coefficient_space(pkg, panels, monkeypatch, refuse, cols):
     p = panels.akm_two_way(30_000, n_firms=400, n_years=12, seed=11, three_way=True)
     rng = np.random.default_rng(11)

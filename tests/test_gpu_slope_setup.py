@@ -38,19 +38,20 @@ def test_start_already_satisfies(absorber, pkg, cols, small):
     assert calls[small] == calls[65]
 
 
-def test_few_iterations_and_a_long_set_up(absorber, pkg):
+@pytest.mark.parametrize("cols,small", [(1, 16), (6, 36)])  # 16 and 6 rounds
+def test_few_iterations_and_a_long_set_up(absorber, pkg, cols, small):
     calls = {}
-    for levels in (16, 65):  # 16 rounds for one column
+    for levels in (small, 65):
         rng, fes, G = _panel(60_000, 900, 10, levels, 2)
         opt = pkg.make_options(tol=1e-3, tolerance_mode=0)
-        _, r = _solve(absorber, rng.standard_normal((1, fes[0].size)), fes, G, rng.standard_normal(fes[0].size), opt)
+        _, r = _solve(absorber, rng.standard_normal((cols, fes[0].size)), fes, G, rng.standard_normal(fes[0].size), opt)
         assert 0 < r.iterations <= 4
         calls[levels] = r.library_calls
-    assert calls[16] == calls[65]
+    assert calls[small] == calls[65]
 
 
-# rounds of the set-up: up to 3 it is made at once, then after a check interval
-@pytest.mark.parametrize("cols,small", [(1, 3), (1, 4), (1, 16), (2, 20), (4, 64), (13, 36)])
+# rounds of the set-up: up to 6 it is made at once here, then after a check interval
+@pytest.mark.parametrize("cols,small", [(1, 3), (1, 4), (1, 16), (2, 20), (4, 64), (6, 36), (7, 50), (13, 36)])
 def test_long_solves_take_the_form(absorber, pkg, panels, cols, small):
     p = panels.akm_two_way(30_000, n_firms=400, n_years=12, seed=cols + small)  # spells at few firms: slow
     calls = {}

@@ -44,7 +44,15 @@ constexpr int kSpaceMaxRuns = 512;
 // interval of observation passes comes first, and the form follows when at its rate
 // more iterations than rounds are left: 8.0 ms for a solve of 52 iterations with 16
 // rounds (7.5 with the form at once, 15.4 by observation passes).
+// Up to kSpaceSureRounds that interval is left out where it cannot end the solve:
+// where each of its iterations (of 4 at least) would have to lower the gradient by more
+// than kSpaceDecades powers of ten of its square (random designs, the fastest seen, gain
+// 2 to 3).  A solve of two intervals then gains with 6 rounds, 3.5 ms for 4.1 (6
+// columns), and loses with 10, 3.3 for 3.0 (1 column); one of 56 iterations with 6
+// rounds takes 6.8 ms, 7.9 after an interval of observation passes and 23.0 by them.
 constexpr int kSpaceFreeRounds = 3;
+constexpr int kSpaceSureRounds = 6;
+constexpr double kSpaceDecades = 4.0;
 constexpr int kSpaceRunBatch = 4;      // runs a slot has in flight (8: 76 us for 58 in the large dim's pass)
 constexpr int kSpaceSerialChunks = 4;  // more chunks of a group: a warp sums them first
 constexpr int kSpaceGroupBatch = 4;    // groups a thread of the vector updates has in flight

@@ -960,7 +960,12 @@ int slopes_device_impl(b200fe_context* ctx, const double* d_v, int64_t n, int C,
     if (sf.on && rounds > kSpaceFreeRounds) {
         std::vector<double> before(C), now(C);
         B_CHECK(sync_read_double(ctx, gamma, C, now.data()));
-        for (double left = 0.0; sf.on && !hd && it < max_it && left <= rounds;) {
+        double left = 0.0;
+        if (rounds <= kSpaceSureRounds)
+            for (int c = 0; c < C; ++c)
+                if (now[c] > thr[c] && std::log10(now[c] / thr[c]) > kSpaceDecades * std::max(ci, 4))
+                    left = std::numeric_limits<double>::infinity();
+        while (!hd && it < max_it && left <= rounds) {
             const int it0 = it;
             before.swap(now);
             B_CHECK(observation_steps());
